@@ -516,7 +516,7 @@ __device__ __forceinline__ int mc_step(const Topo& T, const Env& env, float* ws,
     const float rx = u01(rng.draw((uint32_t)step, P_METRO).x);
     accepted = false;
     if (opt_steps == 0) {
-        float e = eval_e_grad(T, env, SC, W.F, W.g, VCAP_SEARCH, PENALTY_SLOPE, W.pb);
+        float e = eval_e_f(T, env, SC.x, W.F, VCAP_SEARCH, PENALTY_SLOPE, W.pb);
         ne++;
         if (lane == 0) SC.h[0] = e;
         __syncwarp();
