@@ -34,13 +34,12 @@ constexpr int LS_STEPS = 10;
 // ---------------------------------------------------------------- blob layout
 // Header words; section offsets are word offsets from the blob start.
 enum BlobHdr {
-    H_NATOM = 0, H_NTORS, H_NHEAVY, H_NPAIR, H_NROT, H_NRANGE, H_NBIAS,
+    H_NATOM = 0, H_NTORS, H_NHEAVY, H_NPAIR, H_NRANGE, H_NBIAS,
     H_TYPES,       // natom ints
     H_AXIS,        // 2T ints (from, to)
     H_RANGE_OFF,   // T+1 ints (in ranges)
     H_RANGES,      // 2*nrange floats
-    H_ROT_OFF,     // T+1 ints
-    H_ROT,         // rotated atoms of every torsion
+    H_TMASK,       // natom rows of ceil(T / 32) words: bit k set where torsion k rotates the atom
     H_PAIR_OFF,    // natom+1 ints: per-atom intra adjacency (both directions)
     H_PAIRS,       // packed entries: j | zero<<16 | hydrophobic pair<<17 | hbond pair<<18
     H_BIAS_OFF,    // natom+1 ints (records)
@@ -52,9 +51,9 @@ enum BlobHdr {
     H_RHEAVY,
     H_MAPIDX,      // natom ints: grid map slot of each atom (-1: none), set at upload
     H_NPREC,       // number of heavy scored pairs (a count, not an offset)
-    H_PREC,        // 2 words per pair: i | j<<12 | hydrophobic<<24 | hbond<<25, and R_i + R_j (float)
-    H_GOFF,        // natom+1 ints: per-atom lists of (pair index, partner) for the gather
-    H_GADJ,        // entries: pair index | partner << 16
+    H_PREC,        // 2 words per pair: 16 i | hydrophobic | hbond<<1 | 16 j << 16, and R_i + R_j (float)
+    H_GOFF,        // per 32 atoms: first entry of their gather lists, longest of the 32 lists
+    H_GADJ,        // entry q of the lists of 32 atoms side by side: 4 * pair index | 16 * partner << 16
     H_TOTAL,
     H_STAGE,       // words of the blob prefix the search stages into shared memory
     H_FRAME0,      // 3 words: non-collinear atoms no torsion moves (a rigid frame), or -1
@@ -75,21 +74,22 @@ enum BlobHdr {
 #ifndef UD_LS_ATTR
 #define UD_LS_ATTR __forceinline__
 #endif
-constexpr int PREC_HYD = 1 << 24, PREC_HB = 1 << 25;
+constexpr int PREC_HYD = 1, PREC_HB = 2;
 constexpr int PAIR_ZERO = 1 << 16, PAIR_HYD = 1 << 17, PAIR_HB = 1 << 18;
 
 // Topology view: one base pointer and word offsets (keeps addressing 32-bit).
 struct Topo {
     const int* b;
     int natom, ntors, nheavy, nbias;
-    int o_types, o_axis, o_roff, o_ranges, o_rot_off, o_rot, o_pair_off, o_pairs, o_bias_off, o_bias, o_heavy,
+    int o_types, o_axis, o_roff, o_ranges, o_tmask, o_pair_off, o_pairs, o_bias_off, o_bias, o_heavy,
         o_radii, o_rhoff, o_rheavy, o_mapidx, nprec, o_prec, o_goff, o_gadj;
     __device__ __forceinline__ int type(int i) const { return b[o_types + i]; }
-    __device__ __forceinline__ int axis(int k) const { return b[o_axis + k]; }
+    __device__ __forceinline__ int2 bond(int k) const { return *reinterpret_cast<const int2*>(b + o_axis + 2 * k); }
     __device__ __forceinline__ int range_off(int k) const { return b[o_roff + k]; }
     __device__ __forceinline__ const float* ranges() const { return reinterpret_cast<const float*>(b + o_ranges); }
-    __device__ __forceinline__ int rot_off(int k) const { return b[o_rot_off + k]; }
-    __device__ __forceinline__ int rot(int q) const { return b[o_rot + q]; }
+    __device__ __forceinline__ unsigned tmask(int a, int w) const {
+        return (unsigned)b[o_tmask + a * ((ntors + 31) >> 5) + w];
+    }
     __device__ __forceinline__ int pair_off(int i) const { return b[o_pair_off + i]; }
     __device__ __forceinline__ int pair(int k) const { return b[o_pairs + k]; }
     __device__ __forceinline__ int bias_off(int i) const { return b[o_bias_off + i]; }
@@ -100,8 +100,7 @@ struct Topo {
     __device__ __forceinline__ int rheavy(int q) const { return b[o_rheavy + q]; }
     __device__ __forceinline__ int map_index(int i) const { return b[o_mapidx + i]; }
     __device__ __forceinline__ int2 prec(int p) const { return *reinterpret_cast<const int2*>(b + o_prec + 2 * p); }
-    __device__ __forceinline__ int goff(int i) const { return b[o_goff + i]; }
-    __device__ __forceinline__ int gadj(int k) const { return b[o_gadj + k]; }
+    __device__ __forceinline__ int2 glist(int c) const { return *reinterpret_cast<const int2*>(b + o_goff + 2 * c); }
 };
 
 __device__ __forceinline__ Topo topo_view(const int* b) {
@@ -115,8 +114,7 @@ __device__ __forceinline__ Topo topo_view(const int* b) {
     t.o_axis = b[H_AXIS];
     t.o_roff = b[H_RANGE_OFF];
     t.o_ranges = b[H_RANGES];
-    t.o_rot_off = b[H_ROT_OFF];
-    t.o_rot = b[H_ROT];
+    t.o_tmask = b[H_TMASK];
     t.o_pair_off = b[H_PAIR_OFF];
     t.o_pairs = b[H_PAIRS];
     t.o_bias_off = b[H_BIAS_OFF];
@@ -214,23 +212,42 @@ __device__ __forceinline__ void near_receptor(const Env& env, float px, float py
     }
 }
 
+// The special function unit's 2^x, reciprocal root and quotient with denormals flushed to zero: the
+// values of __expf(x) = 2^(x log2 e), rsqrtf and __fdividef wherever these are normal numbers,
+// without the scaling that covers denormal ones.
+__device__ __forceinline__ float ex2_ftz(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float div_ftz(float a, float b) {
+    float y;
+    asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+    return y;
+}
+
 // Vina pair energy and dE/dd at surface distance d for a heavy pair with the given
-// pair flags (vina.h:292-321).
+// pair flags (vina.h:292-321).  The repulsion and hydrophobic terms are selects, not branches: the
+// pairs of a warp are of mixed kinds and distances, so that nearly every branch is taken by
+// some lane (hydrogen bonds are rare enough for one).
 __device__ __forceinline__ float vina_ef(float d, bool hyd, bool hb, float& f) {
-    float x1 = d * 2.0f;                    // (d - 0) / 0.5
-    float e1 = __expf(-x1 * x1);
-    float x2 = (d - 3.0f) * 0.5f;           // (d - 3) / 2
-    float e2 = __expf(-x2 * x2);
+    // exp(-((d - 0) / 0.5)^2) and exp(-((d - 3) / 2)^2); the powers of two of the arguments and of the
+    // derivatives are gathered in the constants, which rounds as the separate factors do
+    constexpr float LOG2E = 1.4426950408889634f;
+    const float t = d - 3.0f;
+    const float e1 = ex2_ftz(d * d * (-4.f * LOG2E)), e2 = ex2_ftz(t * t * (-0.25f * LOG2E));
     float e = -0.035579f * e1 + -0.005156f * e2;
-    f = -0.035579f * (e1 * 2.f * (0.f - d) * 4.0f) + -0.005156f * (e2 * 2.f * (3.f - d) * 0.25f);
-    if (d < 0.f) {
-        e += 0.840245f * d * d;
-        f += 0.840245f * 2.f * d;
-    }
-    if (hyd) {
-        if (d <= 0.5f) e += -0.035069f;
-        else if (d < 1.5f) { e += -0.035069f * (1.5f - d); f += -0.035069f * -1.0f; }
-    }
+    f = 8.f * 0.035579f * (e1 * d) + 0.5f * 0.005156f * (e2 * t);
+    const float rep = fminf(d, 0.f);
+    e += 0.840245f * rep * rep;
+    f += 0.840245f * 2.f * rep;
+    e += (hyd ? -0.035069f : 0.f) * __saturatef(1.5f - d);
+    f += hyd && d > 0.5f && d < 1.5f ? 0.035069f : 0.f;
     if (hb) {
         if (d <= -0.7f) e += -0.587439f;
         else if (d < 0.f) { e += -0.587439f * (0.f - d) / 0.7f; f += -0.587439f * (1.f / -0.7f); }
@@ -244,21 +261,20 @@ __device__ __forceinline__ float vina_ef(float d, bool hyd, bool hb, float& f) {
 // squared distance, radius sum and Vina terms are symmetric).
 __device__ __forceinline__ float pair_scalar(float dx, float dy, float dz, float rsum, bool hyd, bool hb, float vcap,
                                              float& s_out) {
-    s_out = 0.f;
     const float rr = dx * dx + dy * dy + dz * dz;
-    if (!(rr < 64.f)) return 0.f;
-    const float rsq = rsqrtf(rr);                       // r and 1/r from one reciprocal root;
-    const float rn = rr > 0.f ? rr * rsq : 0.f;         // r is clamped at EPSILON before dividing
+    const float rsq = rsqrt_ftz(rr);                    // r and 1/r from one reciprocal root;
+    const float rn = rr > 1e-36f ? rr * rsq : 0.f;      // r is clamped at EPSILON before dividing
     float fdr;
     float ep = vina_ef(rn - rsum, hyd, hb, fdr);
     fdr *= rn < EPS_F ? (1.f / EPS_F) : rsq;
     if (ep > 0.f) {
-        const float c = __fdividef(vcap, vcap + ep);
+        const float c = div_ftz(vcap, vcap + ep);
         ep *= c;
         fdr *= c * c;
     }
-    s_out = fdr;
-    return ep;
+    const bool in = rr < 64.f;                          // false for NaN
+    s_out = in ? fdr : 0.f;
+    return in ? ep : 0.f;
 }
 
 __device__ __forceinline__ float eval_ef(float d, int t1, int t2, float& f) {
@@ -515,20 +531,49 @@ __device__ __forceinline__ float frob_drdv(const RotGradBasis& B, int ind, float
 }
 
 // ---------------------------------------------------------------- pose slots
-// A pose slot in shared memory: [energy, cx, cy, cz, rx, ry, rz, pad] + coords[3N] + dihe[T]
+// A pose slot in shared memory: [energy, cx, cy, cz, rx, ry, rz, pad] + coords[N] + dihe[T], an
+// atom's coordinates in one 16-byte word group: one load per atom where three were needed, and
+// the evaluation is bound by instruction issue and load latency.
 struct Slot {
     float* h;    // header (8 floats)
-    float* x;    // coords 3N
+    float4* x;   // coordinates (w unused)
     float* d;    // dihedrals T
 };
+__host__ __device__ __forceinline__ int slot_floats(int natom, int ntors) { return (8 + 4 * natom + ntors + 3) & ~3; }
 __device__ __forceinline__ Slot slot_at(float* base, int stride, int idx, int natom) {
     float* p = base + idx * stride;
-    return {p, p + 8, p + 8 + 3 * natom};
+    return {p, reinterpret_cast<float4*>(p + 8), p + 8 + 4 * natom};
 }
 __device__ __forceinline__ void slot_copy(Slot dst, Slot src, int natom, int ntors) {
-    int n = 8 + 3 * natom + ntors;
+    const int lane = lane_id();
+    if (lane < 2) reinterpret_cast<float4*>(dst.h)[lane] = reinterpret_cast<const float4*>(src.h)[lane];
 #pragma unroll 1
-    for (int i = lane_id(); i < n; i += WARP) dst.h[i] = src.h[i];
+    for (int i = lane; i < natom; i += WARP) dst.x[i] = src.x[i];
+#pragma unroll 1
+    for (int i = lane; i < ntors; i += WARP) dst.d[i] = src.d[i];
+    __syncwarp();
+}
+// a slot's words to (or from) a place that holds the same layout; the same lane moves the same words
+// both ways
+__device__ __forceinline__ void slot_words(float4* dst, const float4* src, int stride) {
+#pragma unroll 1
+    for (int i = lane_id(); i < stride / 4; i += WARP) dst[i] = src[i];
+}
+// between a slot and a pose record in global memory (header, coords[3N], dihe[T])
+__device__ __forceinline__ void slot_store(float* rec, Slot P, int natom, int ntors) {
+    const int lane = lane_id();
+    const float* x = reinterpret_cast<const float*>(P.x);
+    if (lane < 8) rec[lane] = P.h[lane];
+    for (int i = lane; i < 3 * natom; i += WARP) rec[8 + i] = x[i + i / 3];
+    for (int i = lane; i < ntors; i += WARP) rec[8 + 3 * natom + i] = P.d[i];
+    __syncwarp();
+}
+__device__ __forceinline__ void slot_load(Slot P, const float* rec, int natom, int ntors) {
+    const int lane = lane_id();
+    float* x = reinterpret_cast<float*>(P.x);
+    if (lane < 8) P.h[lane] = rec[lane];
+    for (int i = lane; i < 3 * natom; i += WARP) x[i + i / 3] = rec[8 + i];
+    for (int i = lane; i < ntors; i += WARP) P.d[i] = rec[8 + 3 * natom + i];
     __syncwarp();
 }
 
@@ -583,67 +628,81 @@ __device__ __forceinline__ float grid_sample(const GridView& g, int map, float x
 // The reference visits every scored pair from both atoms (per-pair curl, energy halved,
 // bfgs.cuh:305-352).  Both visits give the same energy and opposite forces, so each
 // heavy pair is evaluated once here.  The functions return the lane's share of the intra
-// energy and add the intra forces to F (which holds the other forces of the lane's own atoms).  The kernel is issue bound, so both variants evaluate exactly the listed
-// pairs, spread evenly over the lanes.  (A round robin in registers for ligands of up to 32
+// energy and add the intra forces to F (which holds the other forces of the lane's own atoms).
+// The search is bound by instruction issue and instruction fetch, so both variants evaluate
+// exactly the listed pairs, spread evenly over the lanes, an atom is one 16-byte load, and the
+// pair terms are written without branches or scaling instructions: 717 -> 670 ms on the 148-ligand
+// screen batch at 100 MC steps, the same results bit for bit.  (A round robin in registers for ligands of up to 32
 // atoms, one atom per lane and partners fetched by shuffle, visited every atom pair slot and
 // was measured 11 % slower on the plain search of a screen batch, 17 % on the learned one.)
 
 // Pass 1 evaluates every pair once and stores the force scalar of each pair in the warp's
 // pair buffer PB; pass 2 (only where the forces are wanted) gathers F_a += s_p (x_a - x_b) over
 // the atom's pairs in pair-index order
-__device__ __forceinline__ float intra_energy(const Topo& T, const float* X, float vcap, float* PB) {
+__device__ __forceinline__ const float4& atom_at(const float4* X, unsigned off) {   // off: 16 * atom
+    return *reinterpret_cast<const float4*>(reinterpret_cast<const char*>(X) + off);
+}
+__device__ __forceinline__ float intra_energy(const Topo& T, const float4* X, float vcap, float* PB) {
     float e = 0.f;
 #pragma unroll 1
     for (int p = lane_id(); p < T.nprec; p += WARP) {
         const int2 pr = T.prec(p);
-        const int i = pr.x & 0xFFF, j = (pr.x >> 12) & 0xFFF;
+        const float4 a = atom_at(X, pr.x & 0xFFF0), b = atom_at(X, (unsigned)pr.x >> 16);
         float sc;
-        e += pair_scalar(X[3 * j] - X[3 * i], X[3 * j + 1] - X[3 * i + 1], X[3 * j + 2] - X[3 * i + 2],
-                         __int_as_float(pr.y), pr.x & PREC_HYD, pr.x & PREC_HB, vcap, sc);
+        e += pair_scalar(b.x - a.x, b.y - a.y, b.z - a.z, __int_as_float(pr.y), pr.x & PREC_HYD, pr.x & PREC_HB, vcap, sc);
         PB[p] = sc;
     }
     return e;
 }
-__device__ __forceinline__ void intra_gather(const Topo& T, const float* X, float* F, const float* PB) {
+// The lists of 32 atoms lie side by side and are as long as their longest: every lane runs the
+// same loop over consecutive words.  A list's padding names the atom itself (difference zero).
+__device__ __forceinline__ void intra_gather(const Topo& T, const float4* X, float4* F, const float* PB) {
+    const int lane = lane_id();
 #pragma unroll 1
-    for (int a = lane_id(); a < T.natom; a += WARP) {
-        const float xa = X[3 * a], ya = X[3 * a + 1], za = X[3 * a + 2];
+    for (int c = 0; 32 * c < T.natom; c++) {
+        const int a = 32 * c + lane;
+        const int2 l = T.glist(c);                        // (first entry, entries per atom)
+        if (a >= T.natom) break;
+        const int cnt = min(T.natom - 32 * c, WARP);
+        const int* ent = T.b + T.o_gadj + l.x + lane;
+        const float4 xa = X[a];
         float fx = 0.f, fy = 0.f, fz = 0.f;
-        const int k1 = T.goff(a + 1);
-#pragma unroll 1
-        for (int k = T.goff(a); k < k1; k++) {
-            const int ent = T.gadj(k);
-            const float sc = PB[ent & 0xFFFF];
-            const int b = ent >> 16;
-            fx += sc * (xa - X[3 * b]);
-            fy += sc * (ya - X[3 * b + 1]);
-            fz += sc * (za - X[3 * b + 2]);
+#pragma unroll 2
+        for (int q = 0; q < l.y; q++, ent += cnt) {
+            const unsigned v = (unsigned)*ent;
+            const float sc = *reinterpret_cast<const float*>(reinterpret_cast<const char*>(PB) + (v & 0xFFFFu));
+            const float4 xb = atom_at(X, v >> 16);
+            fx += sc * (xa.x - xb.x);
+            fy += sc * (xa.y - xb.y);
+            fz += sc * (xa.z - xb.z);
         }
-        F[3 * a] += fx; F[3 * a + 1] += fy; F[3 * a + 2] += fz;
+        float4 f = F[a];
+        f.x += fx; f.y += fy; f.z += fz;
+        F[a] = f;
     }
 }
 
 // ligands whose pair list does not fit the pair buffer: pairs spread over the lanes,
 // forces accumulated with shared-memory atomic adds
-__device__ __forceinline__ float intra_atomic(const Topo& T, const float* X, float* F, float vcap) {
+__device__ __forceinline__ float intra_atomic(const Topo& T, const float4* X, float4* F, float vcap) {
     float e = 0.f;
 #pragma unroll 1
     for (int p = lane_id(); p < T.nprec; p += WARP) {
         const int2 pr = T.prec(p);
-        const int i = pr.x & 0xFFF, j = (pr.x >> 12) & 0xFFF;
-        const float dx = X[3 * j] - X[3 * i], dy = X[3 * j + 1] - X[3 * i + 1], dz = X[3 * j + 2] - X[3 * i + 2];
+        const int i = (pr.x & 0xFFF0) >> 4, j = (unsigned)pr.x >> 20;
+        const float dx = X[j].x - X[i].x, dy = X[j].y - X[i].y, dz = X[j].z - X[i].z;
         float sc;
         e += pair_scalar(dx, dy, dz, __int_as_float(pr.y), pr.x & PREC_HYD, pr.x & PREC_HB, vcap, sc);
         if (sc != 0.f) {
-            atomicAdd(F + 3 * i, -sc * dx); atomicAdd(F + 3 * i + 1, -sc * dy); atomicAdd(F + 3 * i + 2, -sc * dz);
-            atomicAdd(F + 3 * j, sc * dx); atomicAdd(F + 3 * j + 1, sc * dy); atomicAdd(F + 3 * j + 2, sc * dz);
+            atomicAdd(&F[i].x, -sc * dx); atomicAdd(&F[i].y, -sc * dy); atomicAdd(&F[i].z, -sc * dz);
+            atomicAdd(&F[j].x, sc * dx); atomicAdd(&F[j].y, sc * dy); atomicAdd(&F[j].z, sc * dz);
         }
     }
     return e;
 }
 
 // ---------------------------------------------------------------- energy + force
-// Returns the warp-summed energy (bfgs.cuh:221-394) and leaves in F (3N) and PB what
+// Returns the warp-summed energy (bfgs.cuh:221-394) and leaves in F (per atom) and PB what
 // add_intra_forces needs to complete dE/dx per atom: a line-search trial that is rejected, and a
 // plain Metropolis move, need the energy alone (58 % of the search's evaluations are rejected
 // trials; see line_search).
@@ -657,7 +716,7 @@ __device__ __forceinline__ float intra_atomic(const Topo& T, const float* X, flo
 // otherwise over every kept receptor atom (the search kernels, whose default scoring is the
 // grid, keep the lighter loop and their register budget).
 template <bool CELLS = false>
-__device__ __forceinline__ float eval_e_f(const Topo& T, const Env& env, const float* X, float* F, float vcap,
+__device__ __forceinline__ float eval_e_f(const Topo& T, const Env& env, const float4* X, float4* F, float vcap,
                                           float slope, float* PB) {
     const int lane = lane_id();
     float energy = 0.f;
@@ -667,9 +726,10 @@ __device__ __forceinline__ float eval_e_f(const Topo& T, const Env& env, const f
     for (int i = lane; i < T.natom; i += WARP) {
         const int ti = T.type(i);
         float fx = 0.f, fy = 0.f, fz = 0.f;
-        bad |= !(isfinite(X[3 * i]) && isfinite(X[3 * i + 1]) && isfinite(X[3 * i + 2]));
+        const float4 xi = X[i];
+        const float px = xi.x, py = xi.y, pz = xi.z;
+        bad |= !(isfinite(px) && isfinite(py) && isfinite(pz));
         if (ti != VN_H) {
-            const float px = X[3 * i], py = X[3 * i + 1], pz = X[3 * i + 2];
             float e_atom = 0.f;
             if (env.mode == 1) {
                 const int m = T.map_index(i);
@@ -710,7 +770,7 @@ __device__ __forceinline__ float eval_e_f(const Topo& T, const Env& env, const f
             if (pz > env.box_hi[2]) { pen += pz - env.box_hi[2]; fz += slope; }
             energy += e_atom + pen * slope;
         }
-        F[3 * i] = fx; F[3 * i + 1] = fy; F[3 * i + 2] = fz;
+        F[i] = make_float4(fx, fy, fz, 0.f);
     }
     __syncwarp();
     if (PB) energy += intra_energy(T, X, vcap, PB);
@@ -723,7 +783,7 @@ __device__ __forceinline__ float eval_e_f(const Topo& T, const Env& env, const f
             const int b0 = T.bias_off(i), b1 = T.bias_off(i + 1);
             if (b0 < b1) {
                 float fb0 = 0.f, fb1 = 0.f, fb2 = 0.f;
-                const float px = X[3 * i], py = X[3 * i + 1], pz = X[3 * i + 2];
+                const float px = X[i].x, py = X[i].y, pz = X[i].z;
 #pragma unroll 1
                 for (int b = b0; b < b1; b++) {
                     const float* bp = T.bias() + 5 * b;
@@ -745,7 +805,7 @@ __device__ __forceinline__ float eval_e_f(const Topo& T, const Env& env, const f
                         energy += eb;
                     }
                 }
-                F[3 * i] += fb0; F[3 * i + 1] += fb1; F[3 * i + 2] += fb2;
+                F[i].x += fb0; F[i].y += fb1; F[i].z += fb2;
             }
         }
     }
@@ -755,32 +815,34 @@ __device__ __forceinline__ float eval_e_f(const Topo& T, const Env& env, const f
 }
 
 // The forces of the pose that eval_e_f has just evaluated: F becomes dE/dx per atom.
-__device__ __forceinline__ void add_intra_forces(const Topo& T, const float* X, float* F, const float* PB) {
+__device__ __forceinline__ void add_intra_forces(const Topo& T, const float4* X, float4* F, const float* PB) {
     if (!PB) return;                                 // intra_atomic has added them
     intra_gather(T, X, F, PB);
     __syncwarp();
 }
 
 // Generalised gradient from per-atom dE/dx (bfgs.cuh:69-193).  G has 6+ntors entries.
-__device__ __forceinline__ void grad_from_forces(const Topo& T, const Env& env, Slot P, const float* F, float* G) {
+__device__ __forceinline__ void grad_from_forces(const Topo& T, const Env& env, Slot P, const float4* F, float* G) {
     const int lane = lane_id();
-    const float* X = P.x;
+    const float4* X = P.x;
 #pragma unroll 1
     for (int k = lane; k < T.ntors; k += WARP) {
-        const int from = T.axis(2 * k), to = T.axis(2 * k + 1);
-        const float xt = X[3 * to], yt = X[3 * to + 1], zt = X[3 * to + 2];
+        const int2 ft = T.bond(k);
+        const float4 xto = X[ft.y], xfrom = X[ft.x];
+        const float xt = xto.x, yt = xto.y, zt = xto.z;
         float s0 = 0.f, s1 = 0.f, s2 = 0.f;
         const int q1 = T.rh_off(k + 1);
 #pragma unroll 1
         for (int q = T.rh_off(k); q < q1; q++) {       // heavy rotated atoms, in order
             const int a = T.rheavy(q);
-            const float t0 = X[3 * a] - xt, t1 = X[3 * a + 1] - yt, t2 = X[3 * a + 2] - zt;
-            const float f0 = F[3 * a], f1 = F[3 * a + 1], f2 = F[3 * a + 2];
+            const float4 xa = X[a], fa = F[a];
+            const float t0 = xa.x - xt, t1 = xa.y - yt, t2 = xa.z - zt;
+            const float f0 = fa.x, f1 = fa.y, f2 = fa.z;
             s0 += t1 * f2 - t2 * f1;
             s1 += t2 * f0 - t0 * f2;
             s2 += t0 * f1 - t1 * f0;
         }
-        const float a0 = xt - X[3 * from], a1 = yt - X[3 * from + 1], a2 = zt - X[3 * from + 2];
+        const float a0 = xt - xfrom.x, a1 = yt - xfrom.y, a2 = zt - xfrom.z;
         G[6 + k] = (s0 * a0 + s1 * a1 + s2 * a2) / sqrtf(a0 * a0 + a1 * a1 + a2 * a2);
     }
     if (env.constraint) {
@@ -798,9 +860,10 @@ __device__ __forceinline__ void grad_from_forces(const Topo& T, const Env& env, 
 #pragma unroll 1
     for (int h = lane; h < T.nheavy; h += WARP) {
         const int i = T.heavy(h);
-        float t0 = X[3 * i] - cx, t1 = X[3 * i + 1] - cy, t2 = X[3 * i + 2] - cz;
+        const float4 xi = X[i], fi = F[i];
+        float t0 = xi.x - cx, t1 = xi.y - cy, t2 = xi.z - cz;
         quat_rotate(q0, q1, q2, q3, t0, t1, t2);
-        const float f0 = F[3 * i], f1 = F[3 * i + 1], f2 = F[3 * i + 2];
+        const float f0 = fi.x, f1 = fi.y, f2 = fi.z;
         a[0] += f0; a[1] += f1; a[2] += f2;
         a[3] += f0 * t0; a[4] += f0 * t1; a[5] += f0 * t2;
         a[6] += f1 * t0; a[7] += f1 * t1; a[8] += f1 * t2;
@@ -820,7 +883,7 @@ __device__ __forceinline__ void grad_from_forces(const Topo& T, const Env& env, 
 }
 
 template <bool CELLS = false>
-__device__ UD_EVAL_ATTR float eval_e_grad(const Topo& T, const Env& env, Slot P, float* F, float* G,
+__device__ UD_EVAL_ATTR float eval_e_grad(const Topo& T, const Env& env, Slot P, float4* F, float* G,
                                              float vcap, float slope, float* PB) {
     float e = eval_e_f<CELLS>(T, env, P.x, F, vcap, slope, PB);
     add_intra_forces(T, P.x, F, PB);
@@ -829,111 +892,113 @@ __device__ UD_EVAL_ATTR float eval_e_grad(const Topo& T, const Env& env, Slot P,
 }
 
 // ---------------------------------------------------------------- kinematics
-__device__ __forceinline__ void refresh_center(const Topo& T, Slot P) {
+// centre of the pose's atoms, in every lane; also written to the header
+__device__ __forceinline__ void refresh_center(const Topo& T, Slot P, float& cx, float& cy, float& cz) {
     const int lane = lane_id();
     float s0 = 0.f, s1 = 0.f, s2 = 0.f;
 #pragma unroll 1
-    for (int i = lane; i < T.natom; i += WARP) { s0 += P.x[3 * i]; s1 += P.x[3 * i + 1]; s2 += P.x[3 * i + 2]; }
+    for (int i = lane; i < T.natom; i += WARP) { const float4 x = P.x[i]; s0 += x.x; s1 += x.y; s2 += x.z; }
     warp_sum3(s0, s1, s2);
-    __syncwarp();
-    if (lane == 0) {
-        const float n = (float)T.natom;
-        P.h[1] = __fdividef(s0, n); P.h[2] = __fdividef(s1, n); P.h[3] = __fdividef(s2, n);
-    }
+    const float n = (float)T.natom;
+    cx = __fdividef(s0, n); cy = __fdividef(s1, n); cz = __fdividef(s2, n);
+    if (lane == 0) { P.h[1] = cx; P.h[2] = cy; P.h[3] = cz; }
     __syncwarp();
 }
 
 // New value of dihedral k after an increment (bfgs.cuh:455-471): returns the applied
-// increment and stores the clamped dihedral.
-__device__ __forceinline__ float dihedral_step(const Topo& T, Slot P, int k, float incr_raw) {
+// increment and the clamped dihedral.
+__device__ __forceinline__ float dihedral_step(const Topo& T, float old, int k, float incr_raw, float& dn) {
     const float inc = normalize_angle(incr_raw);
     const int r0 = T.range_off(k), nr = T.range_off(k + 1) - r0;
-    const float t = normalize_angle(P.d[k] + inc);
-    const float dn = clamp_by_ranges(t, T.ranges() + 2 * r0, nr);
-    const float applied = dn - P.d[k];
-    P.d[k] = dn;
-    return applied;
+    const float t = normalize_angle(old + inc);
+    dn = clamp_by_ranges(t, T.ranges() + 2 * r0, nr);
+    return dn - old;
 }
 
 // Rotate the atoms of torsion k by the angle with sine s and cosine c about the axis
-// from->to through `to` (bfgs.cuh:477-527); all lanes read the axis atoms directly.
+// from->to through `to` (bfgs.cuh:477-527); all lanes read the axis atoms directly, every lane
+// moves those of its own atoms that the torsion's mask names.
 __device__ __forceinline__ void rotate_torsion(const Topo& T, Slot P, int k, float s, float c) {
-    const int lane = lane_id();
-    const int from = T.axis(2 * k), to = T.axis(2 * k + 1);
-    const float tx = P.x[3 * to], ty = P.x[3 * to + 1], tz = P.x[3 * to + 2];
-    float ax = tx - P.x[3 * from], ay = ty - P.x[3 * from + 1], az = tz - P.x[3 * from + 2];
+    const int2 ft = T.bond(k);
+    const float4 t = P.x[ft.y], f = P.x[ft.x];
+    float ax = t.x - f.x, ay = t.y - f.y, az = t.z - f.z;
     const float l2 = ax * ax + ay * ay + az * az;
     if (!(l2 > EPS_F * EPS_F)) { ax = 1.f; ay = 0.f; az = 0.f; }
-    else { const float il = rsqrtf(l2); ax *= il; ay *= il; az *= il; }
+    else { const float il = rsqrt_ftz(l2); ax *= il; ay *= il; az *= il; }
     __syncwarp();
-    const int q1 = T.rot_off(k + 1);
 #pragma unroll 1
-    for (int q = T.rot_off(k) + lane; q < q1; q += WARP) {
-        const int a = T.rot(q);
-        const float v0 = P.x[3 * a] - tx, v1 = P.x[3 * a + 1] - ty, v2 = P.x[3 * a + 2] - tz;
+    for (int a = lane_id(); a < T.natom; a += WARP) {
+        if (!(T.tmask(a, k >> 5) >> (k & 31) & 1u)) continue;
+        const float4 x = P.x[a];
+        const float v0 = x.x - t.x, v1 = x.y - t.y, v2 = x.z - t.z;
         const float m = (1.f - c) * (ax * v0 + ay * v1 + az * v2);
         const float c0 = ay * v2 - az * v1, c1 = az * v0 - ax * v2, c2 = ax * v1 - ay * v0;
-        P.x[3 * a] = c * v0 + m * ax + s * c0 + tx;
-        P.x[3 * a + 1] = c * v1 + m * ay + s * c1 + ty;
-        P.x[3 * a + 2] = c * v2 + m * az + s * c2 + tz;
+        P.x[a] = make_float4(c * v0 + m * ax + s * c0 + t.x, c * v1 + m * ay + s * c1 + t.y,
+                             c * v2 + m * az + s * c2 + t.z, 0.f);
     }
     __syncwarp();
 }
 
 // One torsion increment as the reference applies it (dihedral, rotation, centre).
 __device__ __forceinline__ void apply_dihe(const Topo& T, Slot P, int k, float incr_raw) {
-    float applied = 0.f;
-    if (lane_id() == 0) applied = dihedral_step(T, P, k, incr_raw);
-    applied = __shfl_sync(FULL, applied, 0);
+    float dn;
+    const float applied = dihedral_step(T, P.d[k], k, incr_raw, dn);
     __syncwarp();
+    if (lane_id() == 0) P.d[k] = dn;
     float s, c;
     __sincosf(applied, &s, &c);
     rotate_torsion(T, P, k, s, c);
-    refresh_center(T, P);
+    refresh_center(T, P, s, c, dn);
 }
 
-// pose += alpha * g: torsions in index order, then rotation about the old centre and
+// Pn = P + alpha * g (Pn may be P): torsions in index order, then rotation about the old centre and
 // translation (bfgs.cuh:560-618).  SC holds 2 floats per torsion of scratch.  The
 // dihedral updates are independent of the coordinates, so they run lane-parallel first;
 // the rotations then follow sequentially in index order as in the reference.
-__device__ UD_KIN_ATTR void apply_update(const Topo& T, const Env& env, Slot P, const float* G, float alpha,
+__device__ UD_KIN_ATTR void apply_update(const Topo& T, const Env& env, Slot P, Slot Pn, const float* G, float alpha,
                                              float* SC) {
     const int lane = lane_id();
+    float c0x = P.h[1], c0y = P.h[2], c0z = P.h[3];
 #pragma unroll 1
     for (int k = lane; k < T.ntors; k += WARP) {
-        const float applied = dihedral_step(T, P, k, G[6 + k] * alpha);
-        float s, c;
+        float s, c, dn;
+        const float applied = dihedral_step(T, P.d[k], k, G[6 + k] * alpha, dn);
         __sincosf(applied, &s, &c);       // |applied| <= 2 pi: hardware sine/cosine (~1e-6 abs)
-        SC[2 * k] = s;
-        SC[2 * k + 1] = c;
+        Pn.d[k] = dn;
+        *reinterpret_cast<float2*>(SC + 2 * k) = make_float2(s, c);
     }
+#pragma unroll 1
+    for (int i = lane; i < T.natom; i += WARP) Pn.x[i] = P.x[i];
+    if (lane < 2) reinterpret_cast<float4*>(Pn.h)[lane] = reinterpret_cast<const float4*>(P.h)[lane];
     __syncwarp();
 #pragma unroll 1
-    for (int k = 0; k < T.ntors; k++) rotate_torsion(T, P, k, SC[2 * k], SC[2 * k + 1]);
-    if (T.ntors > 0) refresh_center(T, P);
+    for (int k = 0; k < T.ntors; k++) {
+        const float2 sc = *reinterpret_cast<const float2*>(SC + 2 * k);
+        rotate_torsion(T, Pn, k, sc.x, sc.y);
+    }
+    if (T.ntors > 0) refresh_center(T, Pn, c0x, c0y, c0z);
     if (env.constraint) return;
-    const float c0x = P.h[1], c0y = P.h[2], c0z = P.h[3];
     const float ncx = c0x + alpha * G[0], ncy = c0y + alpha * G[1], ncz = c0z + alpha * G[2];
     const float rx = G[3] * alpha, ry = G[4] * alpha, rz = G[5] * alpha;
     float q0, q1, q2, q3;
     rotvec_to_quat(rx, ry, rz, q0, q1, q2, q3);
-    __syncwarp();
     if (lane == 0) {
-        P.h[1] = ncx; P.h[2] = ncy; P.h[3] = ncz;
-        P.h[4] = rx; P.h[5] = ry; P.h[6] = rz;
+        Pn.h[1] = ncx; Pn.h[2] = ncy; Pn.h[3] = ncz;
+        Pn.h[4] = rx; Pn.h[5] = ry; Pn.h[6] = rz;
     }
 #pragma unroll 1
     for (int i = lane; i < T.natom; i += WARP) {
-        float v0 = P.x[3 * i] - c0x, v1 = P.x[3 * i + 1] - c0y, v2 = P.x[3 * i + 2] - c0z;
+        const float4 x = Pn.x[i];
+        float v0 = x.x - c0x, v1 = x.y - c0y, v2 = x.z - c0z;
         quat_rotate(q0, q1, q2, q3, v0, v1, v2);
-        P.x[3 * i] = v0 + ncx; P.x[3 * i + 1] = v1 + ncy; P.x[3 * i + 2] = v2 + ncz;
+        Pn.x[i] = make_float4(v0 + ncx, v1 + ncy, v2 + ncz, 0.f);
     }
     __syncwarp();
 }
 
 // ---------------------------------------------------------------- optimiser
 struct Work {        // per-warp scratch in shared memory
-    float* F;        // 3N
+    float4* F;       // dE/dx per atom
     float* g;        // D
     float* gn;       // D
     float* p;        // D
@@ -982,10 +1047,7 @@ __device__ UD_LS_ATTR float line_search(const Topo& T, const Env& env, Slot Px, 
     const float pg = start ? 0.f : gdot(W.p, W.g, dim);
 #pragma unroll 1
     for (int trial = 0; trial < LS_STEPS; trial++) {
-        if (mode != LS_INIT) {
-            slot_copy(Pn, Px, T.natom, T.ntors);
-            apply_update(T, env, Pn, W.p, alpha, W.sc);
-        }
+        if (mode != LS_INIT) apply_update(T, env, Px, Pn, W.p, alpha, W.sc);
         const Slot Q = mode == LS_INIT ? Px : Pn;
         e_new = eval_e_f<CELLS>(T, env, Q.x, W.F, vcap, slope, W.pb);
         n_eval++;
@@ -1002,15 +1064,16 @@ __device__ UD_LS_ATTR float line_search(const Topo& T, const Env& env, Slot Px, 
     return e_new;
 }
 
-// BFGS on the pose in slot ix (bfgs.cuh:729-829).  Uses slots ix / ialt / iori; returns
-// the slot index holding the result, whose header[0] is the final energy.
+// BFGS on the pose in slot ix (bfgs.cuh:729-829).  Uses slots ix and ialt, and keeps the start pose in
+// `ori` (a slot's words), to return to where the run has not improved on it: written once per run
+// and rarely read, so the search keeps it in global memory (L2), where it costs no residency.
+// Returns the slot index holding the result, whose header[0] is the final energy.
 template <bool CELLS = false>
 __device__ __forceinline__ int bfgs(const Topo& T, const Env& env, float* slots, int stride, int ix, int ialt,
-                                    int iori, const Work& W, int max_steps, float vcap, float slope, int& n_eval,
+                                    float4* ori, const Work& W, int max_steps, float vcap, float slope, int& n_eval,
                                     int move_from = -1) {
     const int lane = lane_id();
     const int dim = 6 + T.ntors;
-    const Slot X = slot_at(slots, stride, ix, T.natom);
     float E_ori = 0.f, E = 0.f;
     const int ntri = dim * (dim + 1) / 2;
     int cur = ix, alt = ialt;
@@ -1031,7 +1094,7 @@ __device__ __forceinline__ int bfgs(const Topo& T, const Env& env, float* slots,
             __syncwarp();
 #pragma unroll 1
             for (int i = lane; i < dim; i += WARP) W.H[i + i * (i + 1) / 2] = 1.0;
-            slot_copy(slot_at(slots, stride, iori, T.natom), X, T.natom, T.ntors);
+            slot_words(ori, reinterpret_cast<const float4*>(slots + ix * stride), stride);
             continue;
         }
         // y = g_new - g with g.g (the reference tests the old gradient), y.p and y.y in one
@@ -1078,7 +1141,8 @@ __device__ __forceinline__ int bfgs(const Topo& T, const Env& env, float* slots,
     const Slot R = slot_at(slots, stride, cur, T.natom);
     if (E > E_ori) {
         E = E_ori;
-        slot_copy(R, slot_at(slots, stride, iori, T.natom), T.natom, T.ntors);
+        slot_words(reinterpret_cast<float4*>(R.h), ori, stride);
+        __syncwarp();
     }
     if (lane == 0) R.h[0] = E;
     __syncwarp();
@@ -1092,7 +1156,7 @@ __device__ __forceinline__ float gyration_radius(const Topo& T, Slot P) {
 #pragma unroll 1
     for (int h = lane; h < T.nheavy; h += WARP) {
         const int i = T.heavy(h);
-        const float d0 = P.x[3 * i] - P.h[1], d1 = P.x[3 * i + 1] - P.h[2], d2 = P.x[3 * i + 2] - P.h[3];
+        const float d0 = P.x[i].x - P.h[1], d1 = P.x[i].y - P.h[2], d2 = P.x[i].z - P.h[3];
         s += d0 * d0 + d1 * d1 + d2 * d2;
     }
     s = warp_sum(s);
@@ -1133,7 +1197,8 @@ __device__ __forceinline__ void mutate(const Topo& T, const Env& env, const Rng&
         if (lane == 0) { P.h[1] = c0 + d0; P.h[2] = c1 + d1; P.h[3] = c2 + d2; }
 #pragma unroll 1
         for (int i = lane; i < T.natom; i += WARP) {
-            P.x[3 * i] += d0; P.x[3 * i + 1] += d1; P.x[3 * i + 2] += d2;
+            const float4 x = P.x[i];
+            P.x[i] = make_float4(x.x + d0, x.y + d1, x.z + d2, 0.f);
         }
         __syncwarp();
     } else if (which == 1) {
@@ -1148,9 +1213,10 @@ __device__ __forceinline__ void mutate(const Topo& T, const Env& env, const Rng&
         if (lane == 0) { P.h[4] = rv0; P.h[5] = rv1; P.h[6] = rv2; }
 #pragma unroll 1
         for (int i = lane; i < T.natom; i += WARP) {
-            float t0 = P.x[3 * i] - cx, t1 = P.x[3 * i + 1] - cy, t2 = P.x[3 * i + 2] - cz;
+            const float4 x = P.x[i];
+            float t0 = x.x - cx, t1 = x.y - cy, t2 = x.z - cz;
             quat_rotate(q0, q1, q2, q3, t0, t1, t2);
-            P.x[3 * i] = t0 + cx; P.x[3 * i + 1] = t1 + cy; P.x[3 * i + 2] = t2 + cz;
+            P.x[i] = make_float4(t0 + cx, t1 + cy, t2 + cz, 0.f);
         }
         __syncwarp();
     } else if (which - 2 < T.ntors) {
@@ -1198,7 +1264,7 @@ __device__ __forceinline__ void randomize(const Topo& T, const Env& env, const R
         G[6 + k] = lo + (hi - lo) * u01(u.y) - P.d[k];
     }
     __syncwarp();
-    apply_update(T, env, P, G, 1.f, SC);
+    apply_update(T, env, P, P, G, 1.f, SC);
 }
 
 }  // namespace ud

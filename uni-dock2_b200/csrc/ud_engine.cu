@@ -51,7 +51,7 @@ __host__ __device__ inline int pb_floats(int npair) {
 }
 __host__ __device__ inline int ws_floats(int n, int t, int npair) {
     int d = 6 + t;
-    return 4 * rec_floats(n, t) + r4(3 * n) + 5 * r4(d) + r4(2 * t) + r4(d * (d + 1)) + pb_floats(npair);
+    return 3 * slot_floats(n, t) + 4 * n + 5 * r4(d) + r4(2 * t) + r4(d * (d + 1)) + pb_floats(npair);
 }
 
 struct LigDev {
@@ -68,8 +68,9 @@ struct LigDev {
 __device__ __forceinline__ Work work_at(float* ws, const Topo& T) {
     const int natom = T.natom, ntors = T.ntors, d = 6 + ntors;
     Work W;
-    W.F = ws + 4 * rec_floats(natom, ntors);
-    W.g = W.F + r4(3 * natom);
+    float* f = ws + 3 * slot_floats(natom, ntors);
+    W.F = reinterpret_cast<float4*>(f);
+    W.g = f + 4 * natom;
     W.gn = W.g + r4(d);
     W.p = W.gn + r4(d);
     W.y = W.p + r4(d);
@@ -80,10 +81,8 @@ __device__ __forceinline__ Work work_at(float* ws, const Topo& T) {
     return W;
 }
 
-__device__ __forceinline__ void copy_words(float* dst, const float* src, int n) {
-    for (int i = lane_id(); i < n; i += WARP) dst[i] = src[i];
-    __syncwarp();
-}
+// a warp's three slots in turn
+__device__ __forceinline__ int slot_next(int s) { return s == 2 ? 0 : s + 1; }
 
 // initial pose from the blob: input coordinates, dihedrals, centre = mean, rot_vec = 0,
 // energy 999 (src/cuda/task.cu:87-105)
@@ -97,7 +96,7 @@ __device__ void load_initial(const int* blob, Slot P, int natom, int ntors) {
         P.h[1] = c0[0]; P.h[2] = c0[1]; P.h[3] = c0[2];
         P.h[4] = P.h[5] = P.h[6] = P.h[7] = 0.f;
     }
-    for (int i = lane; i < 3 * natom; i += WARP) P.x[i] = x0[i];
+    for (int i = lane; i < natom; i += WARP) P.x[i] = make_float4(x0[3 * i], x0[3 * i + 1], x0[3 * i + 2], 0.f);
     for (int i = lane; i < ntors; i += WARP) P.d[i] = d0[i];
     __syncwarp();
 }
@@ -181,10 +180,10 @@ __global__ void k_score(const int* __restrict__ blobs, const LigDev* __restrict_
     const LigDev L = ligs[io.lig[pose]];
     const int* blob = blobs + L.blob_off;
     Topo T = topo_view(blob);
-    Slot P = slot_at(ws, L.stride, 0, T.natom);
+    Slot P = slot_at(ws, 0, 0, T.natom);
     Work W = work_at(ws, T);
     const float* x = io.xyz + io.xoff[pose];
-    for (int i = lane; i < 3 * T.natom; i += WARP) P.x[i] = x[i];
+    for (int i = lane; i < 3 * T.natom; i += WARP) reinterpret_cast<float*>(P.x)[i + i / 3] = x[i];
     if (lane < 3) { P.h[1 + lane] = io.centers[3 * pose + lane]; P.h[4 + lane] = io.rotvecs[3 * pose + lane]; }
     __syncwarp();
     float e = eval_e_grad<CELLS>(T, env, P, W.F, W.g, vcap, slope, W.pb);
@@ -375,17 +374,16 @@ __global__ void k_bfgs(const int* __restrict__ blobs, const LigDev* __restrict__
     Topo T = topo_view(blobs + L.blob_off);
     Work W = work_at(ws, T);
     float* rec = recs + item_off[item];
-    int nrec = 8 + 3 * T.natom + T.ntors;
-    copy_words(ws, rec, nrec);
+    const int stride = slot_floats(T.natom, T.ntors);
+    slot_load(slot_at(ws, stride, 0, T.natom), rec, T.natom, T.ntors);
     int cur = 0, ne = 0;
     float slope = slope0;
     for (int r = 0; r < rounds; r++) {
-        int others[3], k = 0;
-        for (int s = 0; s < 4; s++) if (s != cur) others[k++] = s;
-        cur = bfgs<CELLS>(T, env, ws, L.stride, cur, others[0], others[1], W, max_steps, vcap, slope, ne);
+        const int alt = slot_next(cur);
+        cur = bfgs<CELLS>(T, env, ws, stride, cur, alt, reinterpret_cast<float4*>(ws + slot_next(alt) * stride), W, max_steps, vcap, slope, ne);
         if (ramp) slope = fminf(slope * 100.f, PENALTY_SLOPE);
     }
-    copy_words(rec, ws + (size_t)cur * L.stride, nrec);
+    slot_store(rec, slot_at(ws, stride, cur, T.natom), T.natom, T.ntors);
     if (nevals && lane == 0) nevals[item] = ne;
 }
 
@@ -396,6 +394,8 @@ struct SearchP {
     int retain;        // poses kept per chain (1..4)
     int ws_max;        // floats per warp
     int blob_max;      // words reserved for the blob
+    float4* ori;       // a slot per warp of the grid: start poses of the BFGS runs
+    int ori_stride;    // float4 per slot
 };
 
 __device__ __forceinline__ bool metropolis(float e_old, float e_new, float temp, float rx) {  // mc.h:12-18
@@ -403,12 +403,10 @@ __device__ __forceinline__ bool metropolis(float e_old, float e_new, float temp,
     return rx < expf((e_old - e_new) / temp);
 }
 
-__device__ __forceinline__ void store_record(float* dst, Slot P, int nrec) { copy_words(dst, P.h, nrec); }
-
 // a chain's best record before its first improvement: the start pose, energy 1e9 (the
 // bound every chain's first accepted pose is compared against)
-__device__ __forceinline__ void init_best(float* out, Slot P, int nrec) {
-    copy_words(out, P.h, nrec);
+__device__ __forceinline__ void init_best(float* out, Slot P, const Topo& T) {
+    slot_store(out, P, T.natom, T.ntors);
     if (lane_id() == 0) out[0] = 1e9f;
     __syncwarp();
 }
@@ -442,15 +440,15 @@ struct Retained {
         if (R > 3) m = fmaxf(m, e3);
         return m;
     }
-    __device__ __forceinline__ void store(Slot P, int nrec, float energy) {
+    __device__ __forceinline__ void store(Slot P, const Topo& T, float energy) {
         if constexpr (RMAX == 1) {
-            copy_words(out, P.h, nrec);
+            slot_store(out, P, T.natom, T.ntors);
             e0 = energy;
         } else {
             const float t = worst();
             int r = 0;                               // the first record holding the highest energy
             if (!(e0 == t)) r = (R > 1 && e1 == t) ? 1 : ((R > 2 && e2 == t) ? 2 : 3);
-            copy_words(out + (long long)r * stride, P.h, nrec);
+            slot_store(out + (long long)r * stride, P, T.natom, T.ntors);
             if (r == 0) e0 = energy; else if (r == 1) e1 = energy; else if (r == 2) e2 = energy; else e3 = energy;
         }
     }
@@ -463,16 +461,17 @@ struct Proposal {
     float p_learned;
 };
 
-// One MC step of a chain (mc.cu:323-393): the candidate (slot A+1) is the accepted pose
+// One MC step of a chain (mc.cu:323-393): the candidate (the slot after A) is the accepted pose
 // with one move applied (a random move, or a sample of the learned proposal), optimised by
 // BFGS with curl 10; Metropolis at T = 1.2 (step 0 always accepts); an accepted new best is
 // optimised again with curl 1000 and recorded.  Returns the accepted slot; sets *accepted.
 template <class Keep>
-__device__ __forceinline__ int mc_step(const Topo& T, const Env& env, float* ws, int stride, int A, const Work& W,
-                                       const Rng& rng, int step, int opt_steps, int nrec, Keep& keep,
+__device__ __forceinline__ int mc_step(const Topo& T, const Env& env, float* ws, int stride, int A, float4* ori,
+                                       const Work& W,
+                                       const Rng& rng, int step, int opt_steps, Keep& keep,
                                        int& ne, const Proposal& prop, bool& accepted) {
     const int lane = lane_id();
-    const int C = (A + 1) & 3;
+    const int C = slot_next(A);
     Slot SC = slot_at(ws, stride, C, T.natom);
     slot_copy(SC, slot_at(ws, stride, A, T.natom), T.natom, T.ntors);
     bool learned = false;
@@ -508,7 +507,7 @@ __device__ __forceinline__ int mc_step(const Topo& T, const Env& env, float* ws,
         }
         __syncwarp();
         // with BFGS the move is applied by its first line-search call (LS_MOVE)
-        if (opt_steps == 0) apply_update(T, env, SC, W.p, 1.f, W.sc);
+        if (opt_steps == 0) apply_update(T, env, SC, SC, W.p, 1.f, W.sc);
     } else {
         mutate(T, env, rng, (uint32_t)step, SC);
     }
@@ -523,16 +522,16 @@ __device__ __forceinline__ int mc_step(const Topo& T, const Env& env, float* ws,
         if (step == 0 || metropolis(e_acc, e, 1.2f, rx)) {
             A = C;
             accepted = true;
-            if (e < keep.best()) keep.store(SC, nrec, e);
+            if (e < keep.best()) keep.store(SC, T, e);
         }
         return A;
     }
-    // slots: A holds the accepted pose; the other three serve the candidate and the
+    // slots: A holds the accepted pose; the other two, and `ori`, serve the candidate and the
     // optimiser.  Both BFGS runs of a step (candidate with curl 10, accepted new best with
     // curl 1000) go through one call site (phase 0 / 1).
     for (int phase = 0; phase < 2; phase++) {
-        const int X = (A + 1 - phase) & 3;
-        const int R = bfgs(T, env, ws, stride, X, (X + 1) & 3, (X + 2) & 3, W, opt_steps,
+        const int X = phase ? A : C;
+        const int R = bfgs(T, env, ws, stride, X, slot_next(X), ori, W, opt_steps,
                            phase ? VCAP_AUTH : VCAP_SEARCH, PENALTY_SLOPE, ne, (phase == 0 && learned) ? A : -1);
         const float e_new = ws[R * stride];
         if (phase == 0) {
@@ -542,7 +541,7 @@ __device__ __forceinline__ int mc_step(const Topo& T, const Env& env, float* ws,
             if (!(e_new < keep.best())) break;
         } else {
             A = R;
-            if (e_new < keep.best()) keep.store(slot_at(ws, stride, A, T.natom), nrec, e_new);
+            if (e_new < keep.best()) keep.store(slot_at(ws, stride, A, T.natom), T, e_new);
         }
     }
     return A;
@@ -567,6 +566,7 @@ __global__ void __launch_bounds__(NT, MINB) k_search(const int* __restrict__ blo
     float* wsbase = smem + sp.blob_max;
     const int warp = threadIdx.x >> 5, lane = lane_id();
     float* ws = wsbase + (size_t)warp * sp.ws_max;
+    float4* const ori = sp.ori + (size_t)(blockIdx.x * (blockDim.x >> 5) + warp) * sp.ori_stride;
     unsigned long long my_evals = 0, my_heavy = 0;
     __shared__ __align__(8) uint64_t s_bar;
     __shared__ int s_flag;
@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(NT, MINB) k_search(const int* __restrict__ blo
         __syncthreads();
         if (threadIdx.x == 0) s_lig = item.x;
         const Topo T = topo_view(sblob);
-        const int nrec = 8 + 3 * T.natom + T.ntors;
+        const int stride = slot_floats(T.natom, T.ntors);
         const Work W = work_at(ws, T);
         while (true) {
             int ci = 0;
@@ -597,10 +597,10 @@ __global__ void __launch_bounds__(NT, MINB) k_search(const int* __restrict__ blo
             float* out = best + L.best_off + (long long)c * sp.retain * L.stride;
             Rng rng{sp.k0, sp.k1, (uint32_t)c, (uint32_t)L.lig_uid};
             int A = 0;
-            Slot SA = slot_at(ws, L.stride, A, T.natom);
+            Slot SA = slot_at(ws, stride, A, T.natom);
             load_initial(sblob, SA, T.natom, T.ntors);
             if (sp.randomize) randomize(T, env, rng, c, sp.nchain, SA, W.g, W.sc);
-            for (int r = 0; r < sp.retain; r++) init_best(out + (long long)r * L.stride, SA, nrec);
+            for (int r = 0; r < sp.retain; r++) init_best(out + (long long)r * L.stride, SA, T);
             Retained<RMAX> keep{out, L.stride, sp.retain, 1e9f, 1e9f, 1e9f, 1e9f};
             int ne = 0;
             if (sp.mc_steps == 0) {
@@ -608,12 +608,12 @@ __global__ void __launch_bounds__(NT, MINB) k_search(const int* __restrict__ blo
                 ne++;
                 if (lane == 0) SA.h[0] = e;
                 __syncwarp();
-                store_record(out, SA, nrec);
+                slot_store(out, SA, T.natom, T.ntors);
             } else {
                 const Proposal none{nullptr, 0.f};
                 bool acc;
                 for (int step = 0; step < sp.mc_steps; step++)
-                    A = mc_step(T, env, ws, L.stride, A, W, rng, step, sp.opt_steps, nrec, keep, ne, none, acc);
+                    A = mc_step(T, env, ws, stride, A, ori, W, rng, step, sp.opt_steps, keep, ne, none, acc);
             }
             my_evals += ne;
             my_heavy += (unsigned long long)ne * T.nheavy;
@@ -641,6 +641,8 @@ struct LearnP {
     int nchain, opt_steps, randomize;
     int retain;               // poses kept per chain (1..4)
     int ws_max, blob_max;
+    float4* ori;              // as in SearchP
+    int ori_stride;
     float p_learned;          // q: probability of a learned move at a block's first step
     int nfeat_maps;           // grid maps used as features (<= 8)
     int block;                // K: MC steps per launch
@@ -745,11 +747,13 @@ __device__ void frame_rotvec_pts(const float* po, const float* pn, float* rv) {
     rv[0] = k * a0; rv[1] = k * a1; rv[2] = k * a2;
     if (!(rv[0] == rv[0] && rv[1] == rv[1] && rv[2] == rv[2])) rv[0] = rv[1] = rv[2] = 0.f;
 }
-__device__ void frame_rotvec(const float* xo, const float* xn, int f0, int f1, int f2, float* rv) {
+__device__ void frame_rotvec(const float* xo, const float4* xn, int f0, int f1, int f2, float* rv) {
     float po[9], pn[9];
     const int f[3] = {f0, f1, f2};
-    for (int j = 0; j < 3; j++)
-        for (int i = 0; i < 3; i++) { po[3 * j + i] = xo[3 * f[j] + i]; pn[3 * j + i] = xn[3 * f[j] + i]; }
+    for (int j = 0; j < 3; j++) {
+        for (int i = 0; i < 3; i++) po[3 * j + i] = xo[3 * f[j] + i];
+        pn[3 * j] = xn[f[j]].x; pn[3 * j + 1] = xn[f[j]].y; pn[3 * j + 2] = xn[f[j]].z;
+    }
     frame_rotvec_pts(po, pn, rv);
 }
 
@@ -939,6 +943,7 @@ __global__ void __launch_bounds__(NT, MINB) k_learn_step(const int* __restrict__
     float* wsbase = smem + sp.blob_max;
     const int warp = threadIdx.x >> 5, lane = lane_id();
     float* ws = wsbase + (size_t)warp * sp.ws_max;
+    float4* const ori = sp.ori + (size_t)(blockIdx.x * (blockDim.x >> 5) + warp) * sp.ori_stride;
     const int step0 = *step_p;
     const int nsteps = min(sp.block, sp.mc_steps - step0);
     unsigned long long my_evals = 0, my_heavy = 0;
@@ -960,7 +965,7 @@ __global__ void __launch_bounds__(NT, MINB) k_learn_step(const int* __restrict__
         __syncthreads();
         if (threadIdx.x == 0) s_lig = item.x;
         const Topo T = topo_view(sblob);
-        const int nrec = 8 + 3 * T.natom + T.ntors;
+        const int stride = slot_floats(T.natom, T.ntors);
         const Work W = work_at(ws, T);
         while (true) {
             int ci = 0;
@@ -972,14 +977,14 @@ __global__ void __launch_bounds__(NT, MINB) k_learn_step(const int* __restrict__
             float* out = best + L.best_off + (long long)c * sp.retain * L.stride;
             float* accp = acc + L.best_off + (long long)c * L.stride;
             const Rng rng{sp.k0, sp.k1, (uint32_t)c, (uint32_t)L.lig_uid};
-            Slot SA = slot_at(ws, L.stride, 0, T.natom);
+            Slot SA = slot_at(ws, stride, 0, T.natom);
             Retained<RMAX> keep{out, L.stride, sp.retain, 1e9f, 1e9f, 1e9f, 1e9f};
             if (step0 == 0) {
                 load_initial(sblob, SA, T.natom, T.ntors);
                 if (sp.randomize) randomize(T, env, rng, c, sp.nchain, SA, W.g, W.sc);
-                for (int r = 0; r < sp.retain; r++) init_best(out + (long long)r * L.stride, SA, nrec);
+                for (int r = 0; r < sp.retain; r++) init_best(out + (long long)r * L.stride, SA, T);
             } else {
-                copy_words(SA.h, accp, nrec);
+                slot_load(SA, accp, T.natom, T.ntors);
                 keep.e0 = out[0];
                 if (sp.retain > 1) keep.e1 = out[L.stride];
                 if (sp.retain > 2) keep.e2 = out[2LL * L.stride];
@@ -992,13 +997,13 @@ __global__ void __launch_bounds__(NT, MINB) k_learn_step(const int* __restrict__
                 const Proposal prop{(prop_out && step > 0 && s == 0) ? prop_out + g * mlp::OUT : nullptr,
                                     sp.p_learned};
                 bool accepted;
-                A = mc_step(T, env, ws, L.stride, A, W, rng, step, sp.opt_steps, nrec, keep, ne, prop, accepted);
+                A = mc_step(T, env, ws, stride, A, ori, W, rng, step, sp.opt_steps, keep, ne, prop, accepted);
                 // moves are recorded with blocks of one step (the features are the block's first pose)
                 if (rec_set.count && step > 0)
-                    record_move(T, env, accp, slot_at(ws, L.stride, A, T.natom), accepted, rec_set, g);
+                    record_move(T, env, accp, slot_at(ws, stride, A, T.natom), accepted, rec_set, g);
             }
             __syncwarp();
-            copy_words(accp, slot_at(ws, L.stride, A, T.natom).h, nrec);
+            slot_store(accp, slot_at(ws, stride, A, T.natom), T.natom, T.ntors);
             my_evals += ne;
             my_heavy += (unsigned long long)ne * T.nheavy;
         }
@@ -1210,6 +1215,7 @@ struct ud_ctx {
     DBuf<float> d_best;
     DBuf<int> d_order, d_counter, d_leaders, d_counts, d_sel, d_selcnt;
     DBuf<int4> d_items;
+    DBuf<float4> d_ori;                 // start poses of the search's BFGS runs, a slot per resident warp
     DBuf<unsigned long long> d_nevals;
     // results
     int num_pose = 0;
@@ -1386,7 +1392,7 @@ int ud_destroy(ud_ctx* c) {
     c->d_maps32.release(); c->d_maps16.release();
     c->d_blobs.release(); c->d_ligs.release(); c->d_best.release();
     c->d_order.release(); c->d_items.release(); c->d_counter.release(); c->d_leaders.release(); c->d_counts.release();
-    c->d_sel.release(); c->d_selcnt.release(); c->d_nevals.release();
+    c->d_sel.release(); c->d_selcnt.release(); c->d_ori.release(); c->d_nevals.release();
     c->d_out.release(); c->d_terms.release(); c->d_decomp.release();
     c->d_item_lig.release(); c->d_item_off.release(); c->d_item_off2.release();
     for (auto& e : c->ev) if (e) cudaEventDestroy(e);
@@ -1544,7 +1550,7 @@ int ud_add_ligands(ud_ctx* c, int nlig, const int* atom_off, const float* xyz, c
                 return blob[hdr];
             };
             blob[H_NATOM] = n; blob[H_NTORS] = T; blob[H_NHEAVY] = nheavy; blob[H_NPAIR] = np;
-            blob[H_NROT] = nrot; blob[H_NRANGE] = nrange; blob[H_NBIAS] = nb;
+            blob[H_NRANGE] = nrange; blob[H_NBIAS] = nb;
             int o;
             o = put(H_TYPES, n);
             for (int i = 0; i < n; i++) blob[o + i] = types[a0 + i];
@@ -1560,13 +1566,15 @@ int ud_add_ligands(ud_ctx* c, int nlig, const int* atom_off, const float* xyz, c
                 if (range_off[t0 + k + 1] - range_off[t0 + k] <= 0) throw Fail(UD_EINVAL, "torsion without range");
             o = put(H_RANGES, 2 * nrange);
             memcpy(&blob[o], ranges + 2 * (size_t)g0, sizeof(float) * 2 * nrange);
-            o = put(H_ROT_OFF, T + 1);
-            for (int k = 0; k <= T; k++) blob[o + k] = rot_off[t0 + k] - r0;
-            o = put(H_ROT, nrot);
-            for (int k = 0; k < nrot; k++) {
-                int v = rot_atoms[r0 + k];
-                if (v < 0 || v >= n) throw Fail(UD_EINVAL, "rotated atom out of range");
-                blob[o + k] = v;
+            {   // torsions that rotate an atom, as bit masks
+                const int tw = (T + 31) / 32;
+                o = put(H_TMASK, n * tw);
+                for (int k = 0; k < T; k++)
+                    for (int q = rot_off[t0 + k]; q < rot_off[t0 + k + 1]; q++) {
+                        const int v = rot_atoms[q];
+                        if (v < 0 || v >= n) throw Fail(UD_EINVAL, "rotated atom out of range");
+                        blob[o + v * tw + (k >> 5)] |= (int)(1u << (k & 31));
+                    }
             }
             o = put(H_BIAS_OFF, n + 1);
             for (int i = 0; i <= n; i++) blob[o + i] = bias_off ? bias_off[a0 + i] - b0 : 0;
@@ -1626,7 +1634,7 @@ int ud_add_ligands(ud_ctx* c, int nlig, const int* atom_off, const float* xyz, c
                         const int ti = types[a0 + i], tj = types[a0 + j];
                         if (ti == VN_H || tj == VN_H) continue;
                         const unsigned b1 = 1u << ti, b2 = 1u << tj;
-                        int w0 = i | (j << 12);
+                        int w0 = 16 * i | (int)((unsigned)(16 * j) << 16);
                         if ((b1 & HYD_MASK) && (b2 & HYD_MASK)) w0 |= PREC_HYD;
                         if (((b1 & ACC_MASK) && (b2 & DON_MASK)) || ((b1 & DON_MASK) && (b2 & ACC_MASK))) w0 |= PREC_HB;
                         const float rs = kVdwHost[ti] + kVdwHost[tj];
@@ -1642,20 +1650,36 @@ int ud_add_ligands(ud_ctx* c, int nlig, const int* atom_off, const float* xyz, c
                 // the adjacency only the final scoring reads (not staged)
                 o = put(H_PREC, (int)rec.size());
                 for (size_t q = 0; q < rec.size(); q++) blob[o + q] = rec[q];
-                // gather lists: for each atom, (pair index, partner) in pair-index order
+                // gather lists: for each atom, (pair index, partner) in pair-index order; the
+                // lists of 32 atoms side by side, padded to the longest with the atom itself
+                // (used only while the pairs fit the pair buffer)
                 std::vector<std::vector<int>> g(n);
-                for (int p = 0; p < np2; p++) {
-                    const int i = rec[2 * p] & 0xFFF, j = (rec[2 * p] >> 12) & 0xFFF;
-                    g[i].push_back(p | (j << 16));
-                    g[j].push_back(p | (i << 16));
+                for (int p = 0; p < np2 && np2 <= PB_MAX; p++) {
+                    const int i = (rec[2 * p] & 0xFFF0) >> 4, j = (int)((unsigned)rec[2 * p] >> 20);
+                    g[i].push_back(4 * p | (int)((unsigned)(16 * j) << 16));
+                    g[j].push_back(4 * p | (int)((unsigned)(16 * i) << 16));
                 }
-                o = put(H_GOFF, n + 1);
+                const int nc = (n + 31) / 32;
+                o = put(H_GOFF, 2 * nc);
                 int acc = 0;
-                for (int i = 0; i < n; i++) { blob[o + i] = acc; acc += (int)g[i].size(); }
-                blob[o + n] = acc;
+                for (int c = 0; c < nc; c++) {
+                    size_t len = 0;
+                    for (int a = 32 * c; a < std::min(n, 32 * c + 32); a++) len = std::max(len, g[a].size());
+                    blob[o + 2 * c] = acc;
+                    blob[o + 2 * c + 1] = (int)len;
+                    acc += std::min(n - 32 * c, 32) * (int)len;
+                }
+                const int og = o;
                 o = put(H_GADJ, acc);
-                for (int i = 0, k = 0; i < n; i++)
-                    for (int v : g[i]) blob[o + k++] = v;
+                for (int c = 0; c < nc; c++) {
+                    const int cnt = std::min(n - 32 * c, 32);
+                    for (int q = 0; q < blob[og + 2 * c + 1]; q++)
+                        for (int l = 0; l < cnt; l++) {
+                            const int a = 32 * c + l;
+                            blob[o + blob[og + 2 * c] + cnt * q + l] =
+                                q < (int)g[a].size() ? g[a][q] : (int)((unsigned)(16 * a) << 16);
+                        }
+                }
                 blob[H_STAGE] = (int)blob.size();
             }
             o = put(H_PAIR_OFF, n + 1);
@@ -1993,6 +2017,7 @@ int ud_bfgs_batch(ud_ctx* c, int n, const int* pose_lig, float* records, int max
 // count) in descending ligand cost, uploaded with the work counter cleared.
 struct SearchPlan {
     int W = 0, grid = 0, nitems = 0, wsm = 0, blob_max = 0;
+    int slot = 0;          // floats of the largest slot
     int minb = 3;          // instantiation: 3 or 4 (256-thread bound), 2 (384-thread bound)
     size_t smem = 0;
     long long tot = 0;
@@ -2010,6 +2035,7 @@ static SearchPlan plan_search(ud_ctx* c, int nchain, K k3, K k4, K k12, int want
         c->h_ligdev[l].best_off = P.tot;
         P.tot += (long long)nchain * c->retain * h.stride;
         P.wsm = std::max(P.wsm, lig_ws(h));
+        P.slot = std::max(P.slot, slot_floats(h.natom, h.ntors));
         order[l] = l;
         // evaluation cost ~ intra pairs + grid atoms + kinematics, times BFGS length
         const double np = (double)(c->h_blobs[h.blob_off + H_NPAIR]);
@@ -2065,6 +2091,7 @@ static SearchPlan plan_search(ud_ctx* c, int nchain, K k3, K k4, K k12, int want
     P.nitems = (int)items.size();
     P.grid = (int)std::min((long long)P.nitems, resident);
     c->shape[0] = P.W; c->shape[1] = per_sm; c->shape[2] = P.minb; c->shape[3] = k;
+    c->d_ori.ensure((size_t)P.grid * P.W * (P.slot / 4));
     c->d_counter.ensure(1);
     c->d_nevals.ensure(3);          // evaluations, heavy-atom evaluations, staging timeouts
     ck(cudaMemsetAsync(c->d_counter.p, 0, sizeof(int), c->stream), "memset");
@@ -2098,6 +2125,8 @@ static void run_search_plan(ud_ctx* c, const SearchPlan& P, const Env& env, uint
     sp.retain = c->retain;
     sp.ws_max = P.wsm;
     sp.blob_max = P.blob_max;
+    sp.ori = c->d_ori.p;
+    sp.ori_stride = P.slot / 4;
     if (P.grid > 0) {
         const SearchKernel kern = search_kernel(P.minb, c->retain);
         kern<<<P.grid, 32 * P.W, P.smem, c->stream>>>(c->d_blobs.p, c->d_ligs.p, c->d_items.p, P.nitems, env, sp,
@@ -2219,6 +2248,8 @@ static void launch_learned(ud_ctx* c, uint64_t seed, int nchain, int mc_steps, i
     sp.randomize = randomize;
     sp.ws_max = P.wsm;
     sp.blob_max = P.blob_max;
+    sp.ori = c->d_ori.p;
+    sp.ori_stride = P.slot / 4;
     sp.p_learned = p_learned;
     sp.retain = c->retain;
     sp.nfeat_maps = std::min(c->nmaps, mlp::NMAP);

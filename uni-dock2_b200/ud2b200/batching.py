@@ -73,8 +73,8 @@ def predict_dock_bytes(natom, ntors, npairs, nrot, nrange, nbias, nchain: int, r
     t = np.asarray(ntors, np.int64)
     p = np.asarray(npairs, np.int64)
     stride = record_floats(n, t)
-    blob = 4 * (64 + 96 + 13 * n + 7 * t + 2 * np.asarray(nrange, np.int64) + 2 * np.asarray(nrot, np.int64)
-                + 5 * np.asarray(nbias, np.int64) + 3 * p)
+    blob = 4 * (64 + 96 + 13 * n + 7 * t + 2 * np.asarray(nrange, np.int64) + np.asarray(nrot, np.int64)
+                + n * ((t + 31) // 32) + 5 * np.asarray(nbias, np.int64) + 2 * p + n * np.minimum(n, p))
     chains = nchain * retain
     rec = 4 * chains * stride
     b = blob + rec + 4 * chains + 64 + 16 * nchain                      # records, leaders, ligand entry, items
