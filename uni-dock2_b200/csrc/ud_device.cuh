@@ -255,6 +255,26 @@ __device__ __forceinline__ float vina_ef(float d, bool hyd, bool hb, float& f) {
     return e;
 }
 
+// The energy of vina_ef in two parts: what depends on the distance alone, and that plus the pair's
+// hydrophobic and hydrogen-bond terms (the same operations in the same order).
+__device__ __forceinline__ float vina_base(float d) {
+    constexpr float LOG2E = 1.4426950408889634f;
+    const float t = d - 3.0f;
+    const float e1 = ex2_ftz(d * d * (-4.f * LOG2E)), e2 = ex2_ftz(t * t * (-0.25f * LOG2E));
+    float e = -0.035579f * e1 + -0.005156f * e2;
+    const float rep = fminf(d, 0.f);
+    e += 0.840245f * rep * rep;
+    return e;
+}
+__device__ __forceinline__ float vina_flags(float e, float d, bool hyd, bool hb) {
+    e += (hyd ? -0.035069f : 0.f) * __saturatef(1.5f - d);
+    if (hb) {
+        if (d <= -0.7f) e += -0.587439f;
+        else if (d < 0.f) e += -0.587439f * (0.f - d) / 0.7f;
+    }
+    return e;
+}
+
 // Intra pair term seen from atom a of the pair (a, b), d = x_b - x_a: returns the pair
 // energy after the per-pair curl and the scalar s with force on a = -s d.  The reaction
 // on b is the negation, bit for bit what the reference computes from b's side (the

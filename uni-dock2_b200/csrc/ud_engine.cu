@@ -1,7 +1,8 @@
 // ud_engine.cu -- kernels and C ABI of the B200 docking engine (libudock_b200.so).
 //
 // Kernels (all sm_100a, one warp per pose unless noted):
-//   k_grid_build   thread per grid point: per-type Vina maps (new; no reference counterpart)
+//   k_grid_build   thread per grid point, brick of points per block: per-type Vina maps (new; no
+//                  reference counterpart)
 //   k_score        E + generalised gradient of a pose batch   (src/cuda/bfgs_wrapper.cu:51-98)
 //   k_terms        final score terms, no curl                 (src/score/score.cpp:12-147)
 //   k_bfgs         BFGS / refinement rounds on pose records   (src/cuda/optimize.cu:14-77)
@@ -108,49 +109,92 @@ __device__ __forceinline__ float eval_e(float d, int t1, int t2) {
 }
 
 constexpr int MAX_MAPS = 20;   // every non-hydrogen XS type
-struct MapTypes { int n; int t[MAX_MAPS]; };
+// map types by radius; slot: the map's place in the output; fresh: first of its radius
+struct MapTypes { int n; int t[MAX_MAPS]; int slot[MAX_MAPS]; int fresh[MAX_MAPS]; };
 
-__global__ void __launch_bounds__(256) k_grid_build(const float4* __restrict__ rec, int nrec, MapTypes mt,
-                                                    float ox, float oy, float oz, float s, int gx, int gy, int gz,
-                                                    float* __restrict__ out32, __half* __restrict__ out16) {
-    __shared__ float4 tile[256];
-    long long npt = (long long)gx * gy * gz;
-    long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    int ix = (int)(idx % gx), iy = (int)((idx / gx) % gy), iz = (int)(idx / ((long long)gx * gy));
+// A block builds a brick of 8 x 8 x 4 grid points.  It first lists the receptor atoms within the 8 A
+// cutoff of the brick, then every thread sums its point's pairs over that list, which keeps the
+// receptor's order: the sums are those over all atoms, term by term.  (Every point against every atom,
+// 1.5e9 FP64 distance tests at 81^3 points and 2760 atoms: a new receptor's five maps and 512 scores on
+// them took 3.43 ms where they now take 1.86.)
+// Atoms are tested in FP32 first, the exact FP64 test decides; the part of the pair term that
+// depends on the radius alone is shared by the maps of one radius.
+constexpr int BX = 8, BY = 8, BZ = 4, BRICK = BX * BY * BZ;
+__global__ void __launch_bounds__(BRICK) k_grid_build(const float4* __restrict__ rec, int nrec,
+                                                      const __grid_constant__ MapTypes mt, float ox, float oy, float oz,
+                                                      float s, int gx, int gy, int gz, float* __restrict__ out32,
+                                                      __half* __restrict__ out16) {
+    constexpr int CAP = 1024;
+    __shared__ float4 list[CAP];
+    __shared__ int wcount[BRICK / WARP];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = lane_id();
+    const int nbx = (gx + BX - 1) / BX, nby = (gy + BY - 1) / BY;
+    const int x0 = blockIdx.x % nbx * BX, y0 = blockIdx.x / nbx % nby * BY, z0 = blockIdx.x / nbx / nby * BZ;
+    const int ix = x0 + tid % BX, iy = y0 + tid / BX % BY, iz = z0 + tid / (BX * BY);
     // grid point in float via one rounded fma; the cutoff test below is done in FP64
     // from the float inputs, so it is bit-identical to the oracle's
-    float px = __fmaf_rn((float)ix, s, ox), py = __fmaf_rn((float)iy, s, oy), pz = __fmaf_rn((float)iz, s, oz);
+    const float px = __fmaf_rn((float)ix, s, ox), py = __fmaf_rn((float)iy, s, oy), pz = __fmaf_rn((float)iz, s, oz);
+    const bool mine = ix < gx && iy < gy && iz < gz;
+    const float lx = __fmaf_rn((float)x0, s, ox), hx = lx + (BX - 1) * s;
+    const float ly = __fmaf_rn((float)y0, s, oy), hy = ly + (BY - 1) * s;
+    const float lz = __fmaf_rn((float)z0, s, oz), hz = lz + (BZ - 1) * s;
     float acc[MAX_MAPS];
-    float rm[MAX_MAPS];
 #pragma unroll
-    for (int m = 0; m < MAX_MAPS; m++) { acc[m] = 0.f; rm[m] = m < mt.n ? vdw(mt.t[m]) : 0.f; }
-    for (int base = 0; base < nrec; base += 256) {
-        int j = base + threadIdx.x;
-        if (j < nrec) tile[threadIdx.x] = rec[j];
+    for (int m = 0; m < MAX_MAPS; m++) acc[m] = 0.f;
+    int count = 0;                                     // atoms in the list (the same in every thread)
+    for (int base = 0; base < nrec; base += BRICK) {
+        // 256 atoms: those near the brick to the list, in order
+        const int j = base + tid;
+        float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+        bool near = false;
+        if (j < nrec) {
+            r = rec[j];
+            const float ax = fmaxf(fmaxf(lx - r.x, r.x - hx), 0.f), ay = fmaxf(fmaxf(ly - r.y, r.y - hy), 0.f),
+                        az = fmaxf(fmaxf(lz - r.z, r.z - hz), 0.f);
+            near = ax * ax + ay * ay + az * az < 64.1f;       // with room for the rounding of the bounds
+        }
+        const unsigned b = __ballot_sync(FULL, near);
+        if (lane == 0) wcount[warp] = __popc(b);
         __syncthreads();
-        int nt = min(256, nrec - base);
-        if (idx < npt) {
-            for (int k = 0; k < nt; k++) {
-                float4 r = tile[k];
-                double rr = cutoff_r2(r.x, r.y, r.z, px, py, pz);
-                if (rr < 64.0) {
-                    float rn = sqrtf((float)rr);
-                    int tj = (int)r.w;
-                    float rj = vdw(tj);
+        int at = count + __popc(b & ((1u << lane) - 1));
+        for (int w = 0; w < BRICK / WARP; w++) {
+            at += w < warp ? wcount[w] : 0;
+            count += wcount[w];
+        }
+        if (near) list[at] = r;
+        __syncthreads();
+        if (count <= CAP - BRICK && base + BRICK < nrec) continue;
+        if (mine) {
+            for (int k = 0; k < count; k++) {
+                const float4 q = list[k];
+                const float dx = q.x - px, dy = q.y - py, dz = q.z - pz;
+                if (dx * dx + dy * dy + dz * dz > 64.01f) continue;
+                const double rr = cutoff_r2(q.x, q.y, q.z, px, py, pz);
+                if (!(rr < 64.0)) continue;
+                const float rn = sqrtf((float)rr);
+                const int tj = (int)q.w;
+                const float rj = vdw(tj);
+                float d = 0.f, e0 = 0.f;
 #pragma unroll
-                    for (int m = 0; m < MAX_MAPS; m++)
-                        if (m < mt.n) acc[m] += eval_e(rn - (rm[m] + rj), mt.t[m], tj);
-                }
+                for (int m = 0; m < MAX_MAPS; m++)
+                    if (m < mt.n) {
+                        const int t = mt.t[m];
+                        if (mt.fresh[m]) { d = rn - (vdw(t) + rj); e0 = vina_base(d); }
+                        acc[m] += vina_flags(e0, d, hyd_pair(t, tj), hb_pair(t, tj));
+                    }
             }
         }
+        count = 0;
         __syncthreads();
     }
-    if (idx < npt) {
+    if (mine) {
+        const long long npt = (long long)gx * gy * gz, idx = ((long long)iz * gy + iy) * gx + ix;
 #pragma unroll
         for (int m = 0; m < MAX_MAPS; m++) {
             if (m < mt.n) {
-                out32[(long long)m * npt + idx] = acc[m];
-                if (out16) out16[(long long)m * npt + idx] = __float2half_rn(acc[m]);
+                const long long o = mt.slot[m] * npt + idx;
+                out32[o] = acc[m];
+                if (out16) out16[o] = __float2half_rn(acc[m]);
             }
         }
     }
@@ -1469,8 +1513,16 @@ int ud_build_grid(ud_ctx* c, float spacing, int nmaps, const int* map_types, int
         for (int i = 0; i < NT + 3; i++) c->map_of_type[i] = -1;
         for (int m = 0; m < nmaps; m++) {
             if (map_types[m] <= 0 || map_types[m] >= NT) throw Fail(UD_EINVAL, "map type out of range");
-            mt.t[m] = map_types[m];
             c->map_of_type[map_types[m]] = (signed char)m;
+        }
+        std::vector<int> by_radius(nmaps);
+        for (int m = 0; m < nmaps; m++) by_radius[m] = m;
+        std::stable_sort(by_radius.begin(), by_radius.end(),
+                         [&](int a, int b) { return kVdwHost[map_types[a]] < kVdwHost[map_types[b]]; });
+        for (int q = 0; q < nmaps; q++) {
+            mt.slot[q] = by_radius[q];
+            mt.t[q] = map_types[by_radius[q]];
+            mt.fresh[q] = q == 0 || kVdwHost[mt.t[q]] != kVdwHost[mt.t[q - 1]];
         }
         for (int a = 0; a < 3; a++) {
             c->origin[a] = c->box_lo[a];
@@ -1485,11 +1537,11 @@ int ud_build_grid(ud_ctx* c, float spacing, int nmaps, const int* map_types, int
             throw Fail(UD_EINVAL, "grid too large: the maps must hold fewer than 2^31 values (larger spacing or box)");
         c->d_maps32.ensure((size_t)npt * nmaps);
         c->d_maps16.ensure((size_t)npt * nmaps);
-        int threads = 256;
-        long long blocks = (npt + threads - 1) / threads;
-        k_grid_build<<<(unsigned)blocks, threads, 0, c->stream>>>(c->d_rec.p, (int)c->h_rec.size(), mt, c->origin[0],
-                                                                  c->origin[1], c->origin[2], spacing, c->gdim[0],
-                                                                  c->gdim[1], c->gdim[2], c->d_maps32.p, c->d_maps16.p);
+        const long long bricks = (long long)((c->gdim[0] + BX - 1) / BX) * ((c->gdim[1] + BY - 1) / BY) *
+                                 ((c->gdim[2] + BZ - 1) / BZ);
+        k_grid_build<<<(unsigned)bricks, BRICK, 0, c->stream>>>(c->d_rec.p, (int)c->h_rec.size(), mt, c->origin[0], c->origin[1],
+                                                      c->origin[2], spacing, c->gdim[0], c->gdim[1], c->gdim[2],
+                                                      c->d_maps32.p, c->d_maps16.p);
         ck(cudaGetLastError(), "k_grid_build launch");
         ck(cudaStreamSynchronize(c->stream), "k_grid_build");
         c->grid_prec = precision == UD_GRID_F16 ? UD_GRID_F16 : UD_GRID_F32;
