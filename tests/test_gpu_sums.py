@@ -1,9 +1,10 @@
-"""GPU parity of the map build where its loops change: bricks of grid points with remainders, receptors
-that overflow a brick's atom list."""
+"""GPU parity of the map build and of the search's sums where their loops change: bricks of grid points
+with remainders, receptors that overflow a brick's atom list, direct sums over neighbour lists,
+and evaluations that leave the forces out."""
 import numpy as np
 import pytest
 
-from gpu_helpers import MAP_TYPES_ALL
+from gpu_helpers import MAP_TYPES_ALL, engine_for, rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -32,3 +33,56 @@ def test_grid_bricks_match_oracle(oracle64, size, spacing, natom):
     want = oracle64.grid_build(rec, MAP_TYPES_ALL, org.astype(np.float64), spacing, gd)
     assert list(gd) == [max(2, int(np.ceil(s / spacing - 1e-4)) + 1) for s in size]
     assert np.all(np.abs(maps - want) <= TOL * np.maximum(1.0, np.abs(want)))
+
+
+@pytest.fixture(scope="module")
+def sums_sys(small_system):
+    from ud2b200 import synth
+    from ud2b200.model import parse_ligands
+    ligs = parse_ligands({f"s{i}": synth.make_ligand(n, t, seed=700 + i, center=small_system["center"])
+                          for i, (n, t) in enumerate([(8, 0), (31, 5), (33, 6), (65, 12)])})
+    sysd = dict(small_system, ligs=ligs)
+    eng, _ = engine_for(sysd)
+    yield dict(sysd, eng=eng)
+    eng.close()
+
+
+@pytest.mark.parametrize("mode", ["grid", "direct"])
+@pytest.mark.parametrize("opt_steps", [0, 3])
+def test_search_energies_are_those_of_the_scoring(sums_sys, mode, opt_steps):
+    """Every chain's best energy (neighbour-list sums or maps; with and without forces) is the batch
+    scoring's energy (cell rows or maps) of its pose; randomised starts (0 MC steps) stick out of
+    the box and of the cells."""
+    from ud2b200 import MODE_DIRECT, MODE_GRID, split_record
+    eng, m = sums_sys["eng"], MODE_GRID if mode == "grid" else MODE_DIRECT
+    for steps in (0, 4):
+        eng.search(seed=5, nchain=24, mc_steps=steps, opt_steps=opt_steps, randomize=True, mode=m)
+        for li, lig in enumerate(sums_sys["ligs"]):
+            recs = [split_record(lig, r) for r in eng.chain_poses(li)]
+            recs = [r for r in recs if r["energy"] < 1e8 and np.isfinite(r["rot_vec"]).all()]
+            assert len(recs) > 12
+            # a refined new best is optimised again with curl 1000
+            vcap = 1000.0 if steps and opt_steps else 10.0
+            e, _ = eng.score_batch([li] * len(recs), [r["coords"] for r in recs], [r["center"] for r in recs],
+                                   [r["rot_vec"] for r in recs], mode=m, vcap=vcap)
+            got = np.array([r["energy"] for r in recs])
+            near = np.abs(got - e) <= TOL * np.maximum(1.0, np.abs(e))
+            assert near.mean() > (0.5 if steps and opt_steps else 0.999), (li, steps, got[~near], e[~near])
+
+
+def test_direct_search_follows_the_receptor(sums_sys, oracle64):
+    """The neighbour lists belong to the current receptor: a direct search after a new receptor scores
+    on that one, also where it is empty."""
+    from ud2b200 import Engine, MODE_DIRECT, split_record
+    box, lig = sums_sys["box"], sums_sys["ligs"][1]
+    rows = np.asarray([r[:4] for r in sums_sys["rows"]])
+    eng = Engine(box)
+    eng.add_ligands([lig])
+    for keep in (len(rows), len(rows) // 2, 0):
+        eng.set_receptor(rows[:keep, :3].astype(np.float32), rows[:keep, 3].astype(np.int32))
+        eng.search(seed=9, nchain=8, mc_steps=0, opt_steps=0, mode=MODE_DIRECT)
+        recs = [split_record(lig, r) for r in eng.chain_poses(0)]
+        e, _ = eng.score_batch([0] * 8, [r["coords"] for r in recs], [r["center"] for r in recs],
+                               [r["rot_vec"] for r in recs], mode=MODE_DIRECT, vcap=10.0)
+        assert rel_err([r["energy"] for r in recs], e) <= TOL
+    eng.close()

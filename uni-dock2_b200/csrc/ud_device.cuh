@@ -146,15 +146,17 @@ struct Env {
     int constraint;
     int bias_type;            // 0 none, 1 pos, 2 align
     float bias_k;
-    const float4* rec;        // x y z type(as float)
-    int nrec;
     GridView grid;
-    // the receptor atoms again, sorted into cubic cells of CELL_A (x fastest), for the direct
+    // the receptor atoms (x y z type), sorted into cubic cells of CELL_A (x fastest), for the direct
     // sums: cell_start[c] .. cell_start[c + 1] are cell c's atoms, in receptor order
     const float4* rec_cells;
     const int* cell_start;
     float cell_o[3];
     int cdim[3];
+    // and once more, for every cell (and one beyond on each side) the atoms of the 27 cells around it
+    // in receptor order: the direct sums of the search
+    const float4* list_atoms;
+    const int* list_start;
 };
 
 // Cell edge of the receptor cell list: a little above the 8 A cutoff, so that two points
@@ -189,16 +191,54 @@ __device__ __forceinline__ double cutoff_r2(float ax, float ay, float az, float 
     return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
 }
 
-// f(r) for every receptor atom in the 27 cells around (px, py, pz): a superset of the atoms
-// within the 8 A cutoff (callers keep the cutoff test), cell rows in (z, y) order, each row's
-// x cells contiguous in the sorted array, receptor order within a cell.  Nothing for a
-// non-finite point (such a pose scores +inf).
+// The intermolecular term of an evaluation: the grid maps, or direct sums over the receptor atoms
+// near the ligand atom, in the order of the cells' rows (scoring and refinement) or in the
+// receptor's order (the search; the sum over all atoms that it replaces, term by term).
+enum { SUM_GRID = 0, SUM_ROWS = 1, SUM_LIST = 2 };
+
+// f(r) for the atoms of a run that may lie within the 8 A cutoff of (px, py, pz) (callers keep the
+// exact cutoff test).  Every lane has an atom and so a run of its own.  Of 32 atoms each lane
+// first marks those near its atom, and then takes its marked ones: with the distance test and the
+// pair terms in one loop nearly every atom of the run was near some lane's atom, and all lanes
+// waited for its terms, though only one in seven is near a given atom.  Refinement stage of a
+// 148-ligand screen batch 46.5 -> 34.5 ms; direct search of 8 ligands, 64 chains, 3 MC steps,
+// which also visited all 2760 receptor atoms, 598 -> 91 ms; the same results bit for bit.
 template <class F>
+__device__ __forceinline__ void near_run(const float4* __restrict__ atoms, int j, int e, float px, float py, float pz,
+                                         F&& f) {
+#pragma unroll 1
+    for (; j < e; j += 32) {
+        const int n = min(32, e - j);
+        unsigned m = 0;
+#pragma unroll 4
+        for (int t = 0; t < n; t++) {
+            const float4 r = __ldg(atoms + j + t);
+            const float dx = r.x - px, dy = r.y - py, dz = r.z - pz;
+            if (dx * dx + dy * dy + dz * dz < 64.01f) m |= 1u << t;    // with room for rounding
+        }
+#pragma unroll 1
+        for (; m; m &= m - 1) f(__ldg(atoms + j + __ffs(m) - 1));
+    }
+}
+// f(r) for the receptor atoms near (px, py, pz): a superset of those within the cutoff.  SUM_ROWS: of
+// the 27 cells around the point, cell rows in (z, y) order, each row's x cells contiguous in the
+// sorted array, receptor order within a cell; SUM_LIST: the list of the point's cell, which holds
+// the atoms of its 27 cells in receptor order.  Nothing for a non-finite point (such a pose scores
+// +inf).
+template <int SUM, class F>
 __device__ __forceinline__ void near_receptor(const Env& env, float px, float py, float pz, F&& f) {
-    if (!env.cell_start || !(isfinite(px) && isfinite(py) && isfinite(pz))) return;
+    if (!(SUM == SUM_ROWS ? env.cell_start : env.list_start) || !(isfinite(px) && isfinite(py) && isfinite(pz))) return;
     const int cx = (int)fminf(fmaxf(floorf((px - env.cell_o[0]) * (1.f / CELL_A)), -2.f), (float)env.cdim[0] + 1.f);
     const int cy = (int)fminf(fmaxf(floorf((py - env.cell_o[1]) * (1.f / CELL_A)), -2.f), (float)env.cdim[1] + 1.f);
     const int cz = (int)fminf(fmaxf(floorf((pz - env.cell_o[2]) * (1.f / CELL_A)), -2.f), (float)env.cdim[2] + 1.f);
+    if constexpr (SUM == SUM_LIST) {                      // lists of the cells -1 .. cdim along each axis
+        const int nx = env.cdim[0] + 2, ny = env.cdim[1] + 2, nz = env.cdim[2] + 2;
+        if ((unsigned)(cx + 1) >= (unsigned)nx || (unsigned)(cy + 1) >= (unsigned)ny || (unsigned)(cz + 1) >= (unsigned)nz)
+            return;
+        const int* s = env.list_start + ((cz + 1) * ny + cy + 1) * nx + cx + 1;
+        near_run(env.list_atoms, __ldg(s), __ldg(s + 1), px, py, pz, f);
+        return;
+    }
     const int x0 = max(cx - 1, 0), x1 = min(cx + 1, env.cdim[0] - 1);
     if (x0 > x1) return;
 #pragma unroll 1
@@ -206,9 +246,7 @@ __device__ __forceinline__ void near_receptor(const Env& env, float px, float py
         const int y = cy - 1 + q % 3, z = cz - 1 + q / 3;
         if ((unsigned)y >= (unsigned)env.cdim[1] || (unsigned)z >= (unsigned)env.cdim[2]) continue;
         const int row = (z * env.cdim[1] + y) * env.cdim[0];
-        const int e = __ldg(env.cell_start + row + x1 + 1);
-#pragma unroll 1
-        for (int j = __ldg(env.cell_start + row + x0); j < e; j++) f(__ldg(env.rec_cells + j));
+        near_run(env.rec_cells, __ldg(env.cell_start + row + x0), __ldg(env.cell_start + row + x1 + 1), px, py, pz, f);
     }
 }
 
@@ -732,10 +770,8 @@ __device__ __forceinline__ float intra_atomic(const Topo& T, const float4* X, fl
 // escapes every cutoff and box test and gets a finite energy, so Metropolis and the best
 // records could take it; +inf makes the line search, the BFGS revert, Metropolis and the
 // best records all reject it, and changes nothing for finite poses.
-// CELLS: direct sums over the receptor cell list (the refinement and the scoring kernels);
-// otherwise over every kept receptor atom (the search kernels, whose default scoring is the
-// grid, keep the lighter loop and their register budget).
-template <bool CELLS = false>
+// SUM: the intermolecular term, SUM_GRID (trilinear on the maps) or one of the direct sums.
+template <int SUM>
 __device__ __forceinline__ float eval_e_f(const Topo& T, const Env& env, const float4* X, float4* F, float vcap,
                                           float slope, float* PB) {
     const int lane = lane_id();
@@ -751,12 +787,12 @@ __device__ __forceinline__ float eval_e_f(const Topo& T, const Env& env, const f
         bad |= !(isfinite(px) && isfinite(py) && isfinite(pz));
         if (ti != VN_H) {
             float e_atom = 0.f;
-            if (env.mode == 1) {
+            if constexpr (SUM == SUM_GRID) {
                 const int m = T.map_index(i);
                 if (m >= 0) e_atom = grid_sample(env.grid, m, px, py, pz, fx, fy, fz);
             } else {
                 const float r1 = T.radius(i);
-                auto pair = [&](const float4 r) {
+                near_receptor<SUM>(env, px, py, pz, [&](const float4 r) {
                     const float rv0 = r.x - px, rv1 = r.y - py, rv2 = r.z - pz;
                     const double rr = cutoff_r2(r.x, r.y, r.z, px, py, pz);
                     if (rr < 64.0) {
@@ -767,12 +803,7 @@ __device__ __forceinline__ float eval_e_f(const Topo& T, const Env& env, const f
                         fdr /= rn;
                         fx -= fdr * rv0; fy -= fdr * rv1; fz -= fdr * rv2;
                     }
-                };
-                if constexpr (CELLS) {
-                    near_receptor(env, px, py, pz, pair);
-                } else {
-                    for (int j = 0; j < env.nrec; j++) pair(__ldg(env.rec + j));
-                }
+                });
             }
             if (e_atom > 0.f) {
                 float s = vcap / (vcap + e_atom);
@@ -902,10 +933,10 @@ __device__ __forceinline__ void grad_from_forces(const Topo& T, const Env& env, 
     __syncwarp();
 }
 
-template <bool CELLS = false>
+template <int SUM>
 __device__ UD_EVAL_ATTR float eval_e_grad(const Topo& T, const Env& env, Slot P, float4* F, float* G,
                                              float vcap, float slope, float* PB) {
-    float e = eval_e_f<CELLS>(T, env, P.x, F, vcap, slope, PB);
+    float e = eval_e_f<SUM>(T, env, P.x, F, vcap, slope, PB);
     add_intra_forces(T, P.x, F, PB);
     grad_from_forces(T, env, P, F, G);
     return e;
@@ -1076,7 +1107,7 @@ constexpr int LS_TRIALS = 0, LS_INIT = 1, LS_MOVE = 2;
 // W.g); LS_MOVE sets Pn = Px moved by W.p (a learned MC move) and evaluates Pn likewise.
 // A rejected trial needs its energy only: the gather of the intra forces and the gradient run for
 // the kept trial alone (148-ligand screen batch, 100 MC steps: 840 -> 694 ms).
-template <bool CELLS = false>
+template <int SUM>
 __device__ UD_LS_ATTR float line_search(const Topo& T, const Env& env, Slot Px, Slot Pn, const Work& W,
                                              int dim, float e0, float vcap, float slope, float& alpha_out,
                                              int& n_eval, int mode) {
@@ -1087,7 +1118,7 @@ __device__ UD_LS_ATTR float line_search(const Topo& T, const Env& env, Slot Px, 
     for (int trial = 0; trial < LS_STEPS; trial++) {
         if (mode != LS_INIT) apply_update(T, env, Px, Pn, W.p, alpha, W.sc);
         const Slot Q = mode == LS_INIT ? Px : Pn;
-        e_new = eval_e_f<CELLS>(T, env, Q.x, W.F, vcap, slope, W.pb);
+        e_new = eval_e_f<SUM>(T, env, Q.x, W.F, vcap, slope, W.pb);
         n_eval++;
         // the last trial is kept even where it fails the test, as in the reference
         const bool take = start || e_new - e0 < 1e-4f * alpha * pg;
@@ -1106,7 +1137,7 @@ __device__ UD_LS_ATTR float line_search(const Topo& T, const Env& env, Slot Px, 
 // `ori` (a slot's words), to return to where the run has not improved on it: written once per run
 // and rarely read, so the search keeps it in global memory (L2), where it costs no residency.
 // Returns the slot index holding the result, whose header[0] is the final energy.
-template <bool CELLS = false>
+template <int SUM>
 __device__ __forceinline__ int bfgs(const Topo& T, const Env& env, float* slots, int stride, int ix, int ialt,
                                     float4* ori, const Work& W, int max_steps, float vcap, float slope, int& n_eval,
                                     int move_from = -1) {
@@ -1122,7 +1153,7 @@ __device__ __forceinline__ int bfgs(const Topo& T, const Env& env, float* slots,
         if (step >= 0) minus_hv(W.H, W.g, W.p, dim);          // p = -H g
         float alpha;
         const bool mv = step < 0 && move_from >= 0;
-        const float E1 = line_search<CELLS>(T, env, slot_at(slots, stride, mv ? move_from : cur, T.natom),
+        const float E1 = line_search<SUM>(T, env, slot_at(slots, stride, mv ? move_from : cur, T.natom),
                                      slot_at(slots, stride, mv ? cur : alt, T.natom), W, dim, E, vcap, slope, alpha,
                                      n_eval, step < 0 ? (mv ? LS_MOVE : LS_INIT) : LS_TRIALS);
         if (step < 0) {

@@ -50,9 +50,10 @@ constexpr int PB_MAX = PB_MAX_FLOATS;
 __host__ __device__ inline int pb_floats(int npair) {
     return npair <= PB_MAX ? r4(npair) : 0;
 }
+// floats of a warp's workspace
 __host__ __device__ inline int ws_floats(int n, int t, int npair) {
     int d = 6 + t;
-    return 3 * slot_floats(n, t) + 4 * n + 5 * r4(d) + r4(2 * t) + r4(d * (d + 1)) + pb_floats(npair);
+    return 3 * slot_floats(n, t) + 5 * r4(d) + r4(2 * t) + r4(d * (d + 1)) + 4 * n + pb_floats(npair);
 }
 
 struct LigDev {
@@ -69,16 +70,16 @@ struct LigDev {
 __device__ __forceinline__ Work work_at(float* ws, const Topo& T) {
     const int natom = T.natom, ntors = T.ntors, d = 6 + ntors;
     Work W;
-    float* f = ws + 3 * slot_floats(natom, ntors);
-    W.F = reinterpret_cast<float4*>(f);
-    W.g = f + 4 * natom;
+    W.g = ws + 3 * slot_floats(natom, ntors);
     W.gn = W.g + r4(d);
     W.p = W.gn + r4(d);
     W.y = W.p + r4(d);
     W.mhy = W.y + r4(d);
     W.sc = W.mhy + r4(d);
     W.H = reinterpret_cast<double*>(W.sc + r4(2 * ntors));
-    W.pb = pb_floats(T.nprec) ? reinterpret_cast<float*>(W.H) + r4(d * (d + 1)) : nullptr;
+    float* f = reinterpret_cast<float*>(W.H) + r4(d * (d + 1));
+    W.F = reinterpret_cast<float4*>(f);
+    W.pb = pb_floats(T.nprec) ? f + 4 * natom : nullptr;
     return W;
 }
 
@@ -210,10 +211,9 @@ struct PoseIO {
     const long long* goff;   // per pose: offset of gradient in out_g
 };
 
-// CELLS: the direct sums walk the receptor cell list.  Grid scoring never reaches the direct
-// sums, so its launches take the <false> instance and keep the smaller register budget (the cell
-// walk costs k_score 14 registers, which is one resident CTA per SM fewer).
-template <bool CELLS>
+// SUM: the intermolecular term (SUM_GRID, SUM_ROWS): grid scoring keeps the smaller register budget
+// (the walk over cells costs k_score 14 registers, which is one resident CTA per SM fewer).
+template <int SUM>
 __global__ void k_score(const int* __restrict__ blobs, const LigDev* __restrict__ ligs, int n, PoseIO io, Env env,
                         float vcap, float slope, int ws_max, float* out_e, float* out_g) {
     extern __shared__ __align__(16) float smem[];
@@ -230,7 +230,7 @@ __global__ void k_score(const int* __restrict__ blobs, const LigDev* __restrict_
     for (int i = lane; i < 3 * T.natom; i += WARP) reinterpret_cast<float*>(P.x)[i + i / 3] = x[i];
     if (lane < 3) { P.h[1 + lane] = io.centers[3 * pose + lane]; P.h[4 + lane] = io.rotvecs[3 * pose + lane]; }
     __syncwarp();
-    float e = eval_e_grad<CELLS>(T, env, P, W.F, W.g, vcap, slope, W.pb);
+    float e = eval_e_grad<SUM>(T, env, P, W.F, W.g, vcap, slope, W.pb);
     if (lane == 0) out_e[pose] = e;
     float* g = out_g + io.goff[pose];
     for (int i = lane; i < 6 + T.ntors; i += WARP) g[i] = W.g[i];
@@ -338,7 +338,7 @@ __global__ void k_terms(const int* __restrict__ blobs, const LigDev* __restrict_
             float gx, gy, gz;
             if (m >= 0) e_inter += grid_sample(env.grid, m, xi, yi, zi, gx, gy, gz);
         } else {
-            near_receptor(env, xi, yi, zi, [&](const float4 r) {
+            near_receptor<SUM_ROWS>(env, xi, yi, zi, [&](const float4 r) {
                 double rr = cutoff_r2(r.x, r.y, r.z, xi, yi, zi);
                 if (rr < 64.0) {
                     int tj = (int)r.w;
@@ -404,8 +404,7 @@ __global__ void k_terms(const int* __restrict__ blobs, const LigDev* __restrict_
 }
 
 // ====================================================================== BFGS batch
-// CELLS as in k_score: refinement on the grid maps takes the <false> instance.
-template <bool CELLS>
+template <int SUM>
 __global__ void k_bfgs(const int* __restrict__ blobs, const LigDev* __restrict__ ligs, int n, const int* item_lig,
                        const long long* item_off, float* recs, Env env, int max_steps, int rounds, float vcap,
                        float slope0, int ramp, int ws_max, int* nevals) {
@@ -424,7 +423,7 @@ __global__ void k_bfgs(const int* __restrict__ blobs, const LigDev* __restrict__
     float slope = slope0;
     for (int r = 0; r < rounds; r++) {
         const int alt = slot_next(cur);
-        cur = bfgs<CELLS>(T, env, ws, stride, cur, alt, reinterpret_cast<float4*>(ws + slot_next(alt) * stride), W, max_steps, vcap, slope, ne);
+        cur = bfgs<SUM>(T, env, ws, stride, cur, alt, reinterpret_cast<float4*>(ws + slot_next(alt) * stride), W, max_steps, vcap, slope, ne);
         if (ramp) slope = fminf(slope * 100.f, PENALTY_SLOPE);
     }
     slot_store(rec, slot_at(ws, stride, cur, T.natom), T.natom, T.ntors);
@@ -509,7 +508,7 @@ struct Proposal {
 // with one move applied (a random move, or a sample of the learned proposal), optimised by
 // BFGS with curl 10; Metropolis at T = 1.2 (step 0 always accepts); an accepted new best is
 // optimised again with curl 1000 and recorded.  Returns the accepted slot; sets *accepted.
-template <class Keep>
+template <int SUM, class Keep>
 __device__ __forceinline__ int mc_step(const Topo& T, const Env& env, float* ws, int stride, int A, float4* ori,
                                        const Work& W,
                                        const Rng& rng, int step, int opt_steps, Keep& keep,
@@ -559,7 +558,7 @@ __device__ __forceinline__ int mc_step(const Topo& T, const Env& env, float* ws,
     const float rx = u01(rng.draw((uint32_t)step, P_METRO).x);
     accepted = false;
     if (opt_steps == 0) {
-        float e = eval_e_f(T, env, SC.x, W.F, VCAP_SEARCH, PENALTY_SLOPE, W.pb);
+        float e = eval_e_f<SUM>(T, env, SC.x, W.F, VCAP_SEARCH, PENALTY_SLOPE, W.pb);
         ne++;
         if (lane == 0) SC.h[0] = e;
         __syncwarp();
@@ -575,7 +574,7 @@ __device__ __forceinline__ int mc_step(const Topo& T, const Env& env, float* ws,
     // curl 1000) go through one call site (phase 0 / 1).
     for (int phase = 0; phase < 2; phase++) {
         const int X = phase ? A : C;
-        const int R = bfgs(T, env, ws, stride, X, slot_next(X), ori, W, opt_steps,
+        const int R = bfgs<SUM>(T, env, ws, stride, X, slot_next(X), ori, W, opt_steps,
                            phase ? VCAP_AUTH : VCAP_SEARCH, PENALTY_SLOPE, ne, (phase == 0 && learned) ? A : -1);
         const float e_new = ws[R * stride];
         if (phase == 0) {
@@ -599,7 +598,7 @@ __device__ __forceinline__ int mc_step(const Topo& T, const Env& env, float* ws,
 // threads: 4 CTAs = 64 registers, 3 = 80; 384 threads: 2 CTAs = 80 registers); the host
 // picks the width and instantiation that keep the most warps resident (shared memory
 // holds one topology blob per CTA, so wide CTAs pay when the blob is large).
-template <int MINB, int RMAX, int NT = 256>
+template <int MINB, int RMAX, int SUM, int NT = 256>
 __global__ void __launch_bounds__(NT, MINB) k_search(const int* __restrict__ blobs,
                                                 const LigDev* __restrict__ ligs, const int4* __restrict__ items,
                                                 int nitems, Env env, SearchP sp, float* best, int* work_counter,
@@ -648,7 +647,7 @@ __global__ void __launch_bounds__(NT, MINB) k_search(const int* __restrict__ blo
             Retained<RMAX> keep{out, L.stride, sp.retain, 1e9f, 1e9f, 1e9f, 1e9f};
             int ne = 0;
             if (sp.mc_steps == 0) {
-                float e = eval_e_f(T, env, SA.x, W.F, VCAP_SEARCH, PENALTY_SLOPE, W.pb);
+                float e = eval_e_f<SUM>(T, env, SA.x, W.F, VCAP_SEARCH, PENALTY_SLOPE, W.pb);
                 ne++;
                 if (lane == 0) SA.h[0] = e;
                 __syncwarp();
@@ -657,7 +656,7 @@ __global__ void __launch_bounds__(NT, MINB) k_search(const int* __restrict__ blo
                 const Proposal none{nullptr, 0.f};
                 bool acc;
                 for (int step = 0; step < sp.mc_steps; step++)
-                    A = mc_step(T, env, ws, stride, A, ori, W, rng, step, sp.opt_steps, keep, ne, none, acc);
+                    A = mc_step<SUM>(T, env, ws, stride, A, ori, W, rng, step, sp.opt_steps, keep, ne, none, acc);
             }
             my_evals += ne;
             my_heavy += (unsigned long long)ne * T.nheavy;
@@ -1041,7 +1040,7 @@ __global__ void __launch_bounds__(NT, MINB) k_learn_step(const int* __restrict__
                 const Proposal prop{(prop_out && step > 0 && s == 0) ? prop_out + g * mlp::OUT : nullptr,
                                     sp.p_learned};
                 bool accepted;
-                A = mc_step(T, env, ws, stride, A, ori, W, rng, step, sp.opt_steps, keep, ne, prop, accepted);
+                A = mc_step<SUM_GRID>(T, env, ws, stride, A, ori, W, rng, step, sp.opt_steps, keep, ne, prop, accepted);
                 // moves are recorded with blocks of one step (the features are the block's first pose)
                 if (rec_set.count && step > 0)
                     record_move(T, env, accp, slot_at(ws, stride, A, T.natom), accepted, rec_set, g);
@@ -1236,6 +1235,9 @@ struct ud_ctx {
     std::vector<float4> h_rec;
     DBuf<float4> d_rec_cells;           // receptor atoms sorted into CELL_A cells (direct sums)
     DBuf<int> d_cell_start;
+    DBuf<float4> d_list_atoms;          // per cell the atoms of the 27 around it, in receptor order
+    DBuf<int> d_list_start;             // (built by the first direct search on a receptor)
+    bool lists_built = false;
     float cell_o[3] = {0, 0, 0};
     int cdim[3] = {1, 1, 1};
     DBuf<float4> d_rec;
@@ -1298,6 +1300,41 @@ struct ud_ctx {
 
 namespace {
 
+struct CellPos { int x, y, z; };
+CellPos cell_pos(const ud_ctx* c, const float4& r) {
+    const float p[3] = {r.x, r.y, r.z};
+    int q[3];
+    for (int a = 0; a < 3; a++) {
+        const float f = std::floor((p[a] - c->cell_o[a]) * (1.f / CELL_A));
+        q[a] = std::min(std::max((int)f, 0), c->cdim[a] - 1);
+    }
+    return {q[0], q[1], q[2]};
+}
+
+// The neighbour lists of SUM_LIST (27 entries per receptor atom)
+void build_lists(ud_ctx* c) {
+    if (c->lists_built) return;
+    const int nx = c->cdim[0] + 2, ny = c->cdim[1] + 2, nz = c->cdim[2] + 2;
+    std::vector<int> start((size_t)nx * ny * nz + 1, 0);
+    auto each = [&](auto&& f) {
+        for (const float4& r : c->h_rec) {
+            const CellPos q = cell_pos(c, r);
+            for (int z = q.z; z < q.z + 3; z++)           // cells q - 1 .. q + 1, stored from -1
+                for (int y = q.y; y < q.y + 3; y++)
+                    for (int x = q.x; x < q.x + 3; x++) f(((size_t)z * ny + y) * nx + x, r);
+        }
+    };
+    each([&](size_t k, const float4&) { start[k + 1]++; });
+    for (size_t k = 1; k < start.size(); k++) start[k] += start[k - 1];
+    std::vector<float4> atoms((size_t)start.back());
+    std::vector<int> fill(start.begin(), start.end() - 1);
+    each([&](size_t k, const float4& r) { atoms[fill[k]++] = r; });
+    c->d_list_atoms.upload(atoms.data(), atoms.size(), c->stream);
+    c->d_list_start.upload(start.data(), start.size(), c->stream);
+    ck(cudaStreamSynchronize(c->stream), "neighbour lists");
+    c->lists_built = true;
+}
+
 int fail(const Fail& f) {
     g_err = f.what();
     return f.code;
@@ -1310,11 +1347,11 @@ Env make_env(ud_ctx* c, int mode) {
     e.constraint = c->constraint;
     e.bias_type = c->bias_type;
     e.bias_k = c->bias_k;
-    e.rec = c->d_rec.p;
-    e.nrec = (int)c->h_rec.size();
     e.rec_cells = c->d_rec_cells.p;
     e.cell_start = c->d_cell_start.p;
     for (int a = 0; a < 3; a++) { e.cell_o[a] = c->cell_o[a]; e.cdim[a] = c->cdim[a]; }
+    e.list_atoms = c->d_list_atoms.p;
+    e.list_start = c->lists_built ? c->d_list_start.p : nullptr;
     e.grid.f32 = c->d_maps32.p;
     e.grid.f16 = c->d_maps16.p;
     e.grid.use_f16 = (c->grid_prec == UD_GRID_F16 && c->d_maps16.p) ? 1 : 0;
@@ -1374,8 +1411,8 @@ void set_smem(K kernel, size_t bytes) {
 }
 
 // The scoring and refinement kernels of a scoring mode: only direct sums walk the cell list.
-auto score_kernel(const Env& env) { return env.mode == UD_MODE_GRID ? k_score<false> : k_score<true>; }
-auto bfgs_kernel(const Env& env) { return env.mode == UD_MODE_GRID ? k_bfgs<false> : k_bfgs<true>; }
+auto score_kernel(const Env& env) { return env.mode == UD_MODE_GRID ? k_score<SUM_GRID> : k_score<SUM_ROWS>; }
+auto bfgs_kernel(const Env& env) { return env.mode == UD_MODE_GRID ? k_bfgs<SUM_GRID> : k_bfgs<SUM_ROWS>; }
 
 }  // namespace
 
@@ -1433,6 +1470,7 @@ int ud_destroy(ud_ctx* c) {
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     c->d_rec.release(); c->d_rec_cells.release(); c->d_cell_start.release();
+    c->d_list_atoms.release(); c->d_list_start.release();
     c->d_maps32.release(); c->d_maps16.release();
     c->d_blobs.release(); c->d_ligs.release(); c->d_best.release();
     c->d_order.release(); c->d_items.release(); c->d_counter.release(); c->d_leaders.release(); c->d_counts.release();
@@ -1469,6 +1507,7 @@ int ud_set_receptor(ud_ctx* c, int n, const float* xyz, const int* types) {
                       (c->box_lo[2] - 8.f <= z && z <= c->box_hi[2] + 8.f);
             if (in) c->h_rec.push_back(make_float4(x, y, z, (float)t));
         }
+        c->lists_built = false;
         c->d_rec.upload(c->h_rec.data(), c->h_rec.size(), c->stream);
         // cell list over the kept region (box +- 8 A): counting sort, stable in receptor order
         int ncell = 1;
@@ -1478,13 +1517,8 @@ int ud_set_receptor(ud_ctx* c, int n, const float* xyz, const int* types) {
             ncell *= c->cdim[a];
         }
         auto cell_of = [&](const float4& r) {
-            const float p[3] = {r.x, r.y, r.z};
-            int q[3];
-            for (int a = 0; a < 3; a++) {
-                const float f = std::floor((p[a] - c->cell_o[a]) * (1.f / CELL_A));
-                q[a] = std::min(std::max((int)f, 0), c->cdim[a] - 1);
-            }
-            return (q[2] * c->cdim[1] + q[1]) * c->cdim[0] + q[0];
+            const CellPos q = cell_pos(c, r);
+            return (q.z * c->cdim[1] + q.y) * c->cdim[0] + q.x;
         };
         std::vector<int> start((size_t)ncell + 1, 0);
         for (const float4& r : c->h_rec) start[cell_of(r) + 1]++;
@@ -2156,13 +2190,20 @@ static SearchPlan plan_search(ud_ctx* c, int nchain, K k3, K k4, K k12, int want
 using SearchKernel = void (*)(const int*, const LigDev*, const int4*, int, Env, SearchP, float*, int*,
                               unsigned long long*);
 // the k_search instantiation of a plan (minb 3, 4: 256-thread bound; 2: 384-thread bound)
-static SearchKernel search_kernel(int minb, int rmax) {
-    if (rmax > 1) return minb == 4 ? k_search<4, 4> : (minb == 2 ? k_search<2, 4, 384> : k_search<3, 4>);
-    return minb == 4 ? k_search<4, 1> : (minb == 2 ? k_search<2, 1, 384> : k_search<3, 1>);
+extern "C++" {
+template <int SUM>
+static SearchKernel search_kernel_of(int minb, int rmax) {
+    if (rmax > 1) return minb == 4 ? k_search<4, 4, SUM> : (minb == 2 ? k_search<2, 4, SUM, 384> : k_search<3, 4, SUM>);
+    return minb == 4 ? k_search<4, 1, SUM> : (minb == 2 ? k_search<2, 1, SUM, 384> : k_search<3, 1, SUM>);
 }
-static SearchPlan plan_fused(ud_ctx* c, int nchain, int want_w = 0, int force_k = 0) {
+}  // extern "C++"
+static SearchKernel search_kernel(const Env& env, int minb, int rmax) {
+    return env.mode == UD_MODE_GRID ? search_kernel_of<SUM_GRID>(minb, rmax) : search_kernel_of<SUM_LIST>(minb, rmax);
+}
+static SearchPlan plan_fused(ud_ctx* c, const Env& env, int nchain, int want_w = 0, int force_k = 0) {
     const int r = c->retain;
-    return plan_search(c, nchain, search_kernel(3, r), search_kernel(4, r), search_kernel(2, r), want_w, force_k);
+    return plan_search(c, nchain, search_kernel(env, 3, r), search_kernel(env, 4, r), search_kernel(env, 2, r),
+                       want_w, force_k);
 }
 
 static void run_search_plan(ud_ctx* c, const SearchPlan& P, const Env& env, uint64_t seed, int nchain, int mc_steps,
@@ -2180,7 +2221,7 @@ static void run_search_plan(ud_ctx* c, const SearchPlan& P, const Env& env, uint
     sp.ori = c->d_ori.p;
     sp.ori_stride = P.slot / 4;
     if (P.grid > 0) {
-        const SearchKernel kern = search_kernel(P.minb, c->retain);
+        const SearchKernel kern = search_kernel(env, P.minb, c->retain);
         kern<<<P.grid, 32 * P.W, P.smem, c->stream>>>(c->d_blobs.p, c->d_ligs.p, c->d_items.p, P.nitems, env, sp,
                                                       c->d_best.p, c->d_counter.p, c->d_nevals.p);
         ck(cudaGetLastError(), "k_search launch");
@@ -2203,7 +2244,7 @@ static void autotune_search(ud_ctx* c, const Env& env, uint64_t seed, int nchain
     int best_w = 8, best_k = 0;
     for (int w : {8, 12, 4})
         for (int k : {1, 2, 4}) {
-            const SearchPlan P = plan_fused(c, nchain, w, k);
+            const SearchPlan P = plan_fused(c, env, nchain, w, k);
             c->d_best.ensure((size_t)P.tot);
             ck(cudaEventRecord(e0, c->stream), "event");
             run_search_plan(c, P, env, seed, nchain, 3, opt_steps, randomize);
@@ -2222,12 +2263,13 @@ static void autotune_search(ud_ctx* c, const Env& env, uint64_t seed, int nchain
 
 static void launch_search(ud_ctx* c, uint64_t seed, int nchain, int mc_steps, int opt_steps, int randomize, int mode) {
     sync_ligs(c);
+    if (mode != UD_MODE_GRID) build_lists(c);
     Env env = make_env(c, mode);
     c->nchain = nchain * c->retain;                  // records per ligand
     if (c->autotune && !(c->pack_w || c->pack_k)) autotune_search(c, env, seed, nchain, opt_steps, randomize);
-    const SearchPlan P = (c->pack_w || c->pack_k) ? plan_fused(c, nchain, c->pack_w, c->pack_k)
-                         : c->autotune         ? plan_fused(c, nchain, c->tune_w, c->tune_k)
-                                               : plan_fused(c, nchain);
+    const SearchPlan P = (c->pack_w || c->pack_k) ? plan_fused(c, env, nchain, c->pack_w, c->pack_k)
+                         : c->autotune         ? plan_fused(c, env, nchain, c->tune_w, c->tune_k)
+                                               : plan_fused(c, env, nchain);
     c->best_floats = P.tot;
     c->d_best.ensure((size_t)P.tot);
     run_search_plan(c, P, env, seed, nchain, mc_steps, opt_steps, randomize);
