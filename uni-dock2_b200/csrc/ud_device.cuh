@@ -700,6 +700,7 @@ __device__ __forceinline__ float grid_sample(const GridView& g, int map, float x
 __device__ __forceinline__ const float4& atom_at(const float4* X, unsigned off) {   // off: 16 * atom
     return *reinterpret_cast<const float4*>(reinterpret_cast<const char*>(X) + off);
 }
+template <bool FORCES>
 __device__ __forceinline__ float intra_energy(const Topo& T, const float4* X, float vcap, float* PB) {
     float e = 0.f;
 #pragma unroll 1
@@ -708,7 +709,7 @@ __device__ __forceinline__ float intra_energy(const Topo& T, const float4* X, fl
         const float4 a = atom_at(X, pr.x & 0xFFF0), b = atom_at(X, (unsigned)pr.x >> 16);
         float sc;
         e += pair_scalar(b.x - a.x, b.y - a.y, b.z - a.z, __int_as_float(pr.y), pr.x & PREC_HYD, pr.x & PREC_HB, vcap, sc);
-        PB[p] = sc;
+        if constexpr (FORCES) PB[p] = sc;
     }
     return e;
 }
@@ -771,7 +772,8 @@ __device__ __forceinline__ float intra_atomic(const Topo& T, const float4* X, fl
 // records could take it; +inf makes the line search, the BFGS revert, Metropolis and the
 // best records all reject it, and changes nothing for finite poses.
 // SUM: the intermolecular term, SUM_GRID (trilinear on the maps) or one of the direct sums.
-template <int SUM>
+// FORCES: false for callers that want the energy alone (F and PB unused).
+template <int SUM, bool FORCES = true>
 __device__ __forceinline__ float eval_e_f(const Topo& T, const Env& env, const float4* X, float4* F, float vcap,
                                           float slope, float* PB) {
     const int lane = lane_id();
@@ -821,10 +823,10 @@ __device__ __forceinline__ float eval_e_f(const Topo& T, const Env& env, const f
             if (pz > env.box_hi[2]) { pen += pz - env.box_hi[2]; fz += slope; }
             energy += e_atom + pen * slope;
         }
-        F[i] = make_float4(fx, fy, fz, 0.f);
+        if constexpr (FORCES) F[i] = make_float4(fx, fy, fz, 0.f);
     }
     __syncwarp();
-    if (PB) energy += intra_energy(T, X, vcap, PB);
+    if (!FORCES || PB) energy += intra_energy<FORCES>(T, X, vcap, PB);
     else energy += intra_atomic(T, X, F, vcap);
     // bias (bfgs.cuh:356-388; vina.h:353-400)
     if (env.bias_type != 0 && T.nbias > 0) {
@@ -856,7 +858,7 @@ __device__ __forceinline__ float eval_e_f(const Topo& T, const Env& env, const f
                         energy += eb;
                     }
                 }
-                F[i].x += fb0; F[i].y += fb1; F[i].z += fb2;
+                if constexpr (FORCES) { F[i].x += fb0; F[i].y += fb1; F[i].z += fb2; }
             }
         }
     }

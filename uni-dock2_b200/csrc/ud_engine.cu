@@ -50,10 +50,12 @@ constexpr int PB_MAX = PB_MAX_FLOATS;
 __host__ __device__ inline int pb_floats(int npair) {
     return npair <= PB_MAX ? r4(npair) : 0;
 }
-// floats of a warp's workspace
-__host__ __device__ inline int ws_floats(int n, int t, int npair) {
+// floats of a warp's workspace; energy_only: of a search without BFGS, which has no use for the
+// inverse Hessian, the forces and the pair buffer (a quarter of the size for an 80-atom ligand)
+__host__ __device__ inline int ws_floats(int n, int t, int npair, bool energy_only = false) {
     int d = 6 + t;
-    return 3 * slot_floats(n, t) + 5 * r4(d) + r4(2 * t) + r4(d * (d + 1)) + 4 * n + pb_floats(npair);
+    const int w = 3 * slot_floats(n, t) + 5 * r4(d) + r4(2 * t);
+    return energy_only ? w : w + r4(d * (d + 1)) + 4 * n + pb_floats(npair);
 }
 
 struct LigDev {
@@ -558,7 +560,7 @@ __device__ __forceinline__ int mc_step(const Topo& T, const Env& env, float* ws,
     const float rx = u01(rng.draw((uint32_t)step, P_METRO).x);
     accepted = false;
     if (opt_steps == 0) {
-        float e = eval_e_f<SUM>(T, env, SC.x, W.F, VCAP_SEARCH, PENALTY_SLOPE, W.pb);
+        float e = eval_e_f<SUM, false>(T, env, SC.x, nullptr, VCAP_SEARCH, PENALTY_SLOPE, nullptr);
         ne++;
         if (lane == 0) SC.h[0] = e;
         __syncwarp();
@@ -647,7 +649,7 @@ __global__ void __launch_bounds__(NT, MINB) k_search(const int* __restrict__ blo
             Retained<RMAX> keep{out, L.stride, sp.retain, 1e9f, 1e9f, 1e9f, 1e9f};
             int ne = 0;
             if (sp.mc_steps == 0) {
-                float e = eval_e_f<SUM>(T, env, SA.x, W.F, VCAP_SEARCH, PENALTY_SLOPE, W.pb);
+                float e = eval_e_f<SUM, false>(T, env, SA.x, nullptr, VCAP_SEARCH, PENALTY_SLOPE, nullptr);
                 ne++;
                 if (lane == 0) SA.h[0] = e;
                 __syncwarp();
@@ -2111,7 +2113,7 @@ struct SearchPlan {
 
 extern "C++" {
 template <typename K>
-static SearchPlan plan_search(ud_ctx* c, int nchain, K k3, K k4, K k12, int want_w = 0, int force_k = 0) {
+static SearchPlan plan_search(ud_ctx* c, int nchain, bool energy_only, K k3, K k4, K k12, int want_w = 0, int force_k = 0) {
     SearchPlan P;
     const int nlig = (int)c->h_ligs.size();
     std::vector<int> order(nlig);
@@ -2120,7 +2122,7 @@ static SearchPlan plan_search(ud_ctx* c, int nchain, K k3, K k4, K k12, int want
         const LigHost& h = c->h_ligs[l];
         c->h_ligdev[l].best_off = P.tot;
         P.tot += (long long)nchain * c->retain * h.stride;
-        P.wsm = std::max(P.wsm, lig_ws(h));
+        P.wsm = std::max(P.wsm, ws_floats(h.natom, h.ntors, h.nprec, energy_only));
         P.slot = std::max(P.slot, slot_floats(h.natom, h.ntors));
         order[l] = l;
         // evaluation cost ~ intra pairs + grid atoms + kinematics, times BFGS length
@@ -2200,9 +2202,9 @@ static SearchKernel search_kernel_of(int minb, int rmax) {
 static SearchKernel search_kernel(const Env& env, int minb, int rmax) {
     return env.mode == UD_MODE_GRID ? search_kernel_of<SUM_GRID>(minb, rmax) : search_kernel_of<SUM_LIST>(minb, rmax);
 }
-static SearchPlan plan_fused(ud_ctx* c, const Env& env, int nchain, int want_w = 0, int force_k = 0) {
+static SearchPlan plan_fused(ud_ctx* c, const Env& env, int nchain, bool energy_only, int want_w = 0, int force_k = 0) {
     const int r = c->retain;
-    return plan_search(c, nchain, search_kernel(env, 3, r), search_kernel(env, 4, r), search_kernel(env, 2, r),
+    return plan_search(c, nchain, energy_only, search_kernel(env, 3, r), search_kernel(env, 4, r), search_kernel(env, 2, r),
                        want_w, force_k);
 }
 
@@ -2244,7 +2246,7 @@ static void autotune_search(ud_ctx* c, const Env& env, uint64_t seed, int nchain
     int best_w = 8, best_k = 0;
     for (int w : {8, 12, 4})
         for (int k : {1, 2, 4}) {
-            const SearchPlan P = plan_fused(c, env, nchain, w, k);
+            const SearchPlan P = plan_fused(c, env, nchain, opt_steps == 0, w, k);
             c->d_best.ensure((size_t)P.tot);
             ck(cudaEventRecord(e0, c->stream), "event");
             run_search_plan(c, P, env, seed, nchain, 3, opt_steps, randomize);
@@ -2266,10 +2268,11 @@ static void launch_search(ud_ctx* c, uint64_t seed, int nchain, int mc_steps, in
     if (mode != UD_MODE_GRID) build_lists(c);
     Env env = make_env(c, mode);
     c->nchain = nchain * c->retain;                  // records per ligand
+    const bool energy_only = mc_steps == 0 || opt_steps == 0;
     if (c->autotune && !(c->pack_w || c->pack_k)) autotune_search(c, env, seed, nchain, opt_steps, randomize);
-    const SearchPlan P = (c->pack_w || c->pack_k) ? plan_fused(c, env, nchain, c->pack_w, c->pack_k)
-                         : c->autotune         ? plan_fused(c, env, nchain, c->tune_w, c->tune_k)
-                                               : plan_fused(c, env, nchain);
+    const SearchPlan P = (c->pack_w || c->pack_k) ? plan_fused(c, env, nchain, energy_only, c->pack_w, c->pack_k)
+                         : c->autotune         ? plan_fused(c, env, nchain, energy_only, c->tune_w, c->tune_k)
+                                               : plan_fused(c, env, nchain, energy_only);
     c->best_floats = P.tot;
     c->d_best.ensure((size_t)P.tot);
     run_search_plan(c, P, env, seed, nchain, mc_steps, opt_steps, randomize);
@@ -2298,9 +2301,9 @@ static void launch_learned(ud_ctx* c, uint64_t seed, int nchain, int mc_steps, i
     // p_learned 0.25, blocks of 4 steps: 1683 ms at k = 2, 1718 at 1, 1808 at 4)
     const int lk = c->pack_k ? c->pack_k : 2;
     const SearchPlan P = c->retain > 1
-                             ? plan_search(c, nchain, k_learn_step<3, 4>, k_learn_step<4, 4>, k_learn_step<2, 4, 384>,
+                             ? plan_search(c, nchain, opt_steps == 0, k_learn_step<3, 4>, k_learn_step<4, 4>, k_learn_step<2, 4, 384>,
                                            c->pack_w, lk)
-                             : plan_search(c, nchain, k_learn_step<3, 1>, k_learn_step<4, 1>, k_learn_step<2, 1, 384>,
+                             : plan_search(c, nchain, opt_steps == 0, k_learn_step<3, 1>, k_learn_step<4, 1>, k_learn_step<2, 1, 384>,
                                            c->pack_w, lk);
     c->best_floats = P.tot;
     c->d_best.ensure((size_t)P.tot);
