@@ -445,7 +445,7 @@ __device__ __forceinline__ int rs16_lane(int v) {
 // Salmon, Moraes, Dror, Shaw, "Parallel random numbers: as easy as 1, 2, 3", SC'11.
 // Stream: key = (seed lo, seed hi ^ 0x5DEECE66), counter = (chain, ligand, step, purpose).
 struct U4 { uint32_t x, y, z, w; };
-__device__ __forceinline__ U4 philox(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, uint32_t k0, uint32_t k1) {
+__device__ __noinline__ U4 philox(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, uint32_t k0, uint32_t k1) {
 #pragma unroll
     for (int r = 0; r < 10; r++) {
         uint32_t lo0 = 0xD2511F53u * c0, hi0 = __umulhi(0xD2511F53u, c0);
@@ -469,6 +469,17 @@ struct Rng {
 };
 
 // ---------------------------------------------------------------- small math
+// What is rarely or never reached inside the search's loop is not inlined there: the loop's warps
+// run at different points of it and share the instruction cache, and fmodf, the range reduction of
+// sincosf and the like are long (574 -> 538 ms on the 148-ligand screen batch at 100 MC steps; 2 %
+// slower for the 64 chains of a single constrained ligand).
+__device__ __noinline__ float fmod_2pi_far(float x) { return fmodf(x, 2.f * PI_F); }
+__device__ __noinline__ float2 sincos_far(float x) {
+    float s, c;
+    sincosf(x, &s, &c);
+    return make_float2(s, c);
+}
+
 // fmodf(x, 2 PI) with exact shortcuts for the common magnitudes: |x| < 2 PI is returned
 // unchanged and 2 PI <= |x| < 4 PI loses one period, both exactly what fmodf returns
 // (the subtraction is exact by Sterbenz's lemma)
@@ -476,7 +487,7 @@ __device__ __forceinline__ float fmod_2pi(float x) {
     const float p = 2.f * PI_F, ax = fabsf(x);
     if (ax < p) return x;
     if (ax < 2.f * p) return x > 0.f ? x - p : x + p;
-    return fmodf(x, p);
+    return fmod_2pi_far(x);
 }
 __device__ __forceinline__ float normalize_angle(float x) {   // mymath.h:38-47
     x = fmod_2pi(x);
@@ -509,7 +520,7 @@ __device__ __forceinline__ void rotvec_to_quat(float vx, float vy, float vz, flo
         float s, c;
         const float h = th * 0.5f;
         if (h <= PI_F) __sincosf(h, &s, &c);     // hardware sine/cosine on [0, pi]
-        else sincosf(h, &s, &c);
+        else { const float2 sc = sincos_far(h); s = sc.x; c = sc.y; }
         const float k = __fdividef(s, th);
         q0 = c;
         q1 = k * vx;
@@ -622,7 +633,9 @@ __device__ __forceinline__ void slot_store(float* rec, Slot P, int natom, int nt
     const int lane = lane_id();
     const float* x = reinterpret_cast<const float*>(P.x);
     if (lane < 8) rec[lane] = P.h[lane];
+#pragma unroll 1
     for (int i = lane; i < 3 * natom; i += WARP) rec[8 + i] = x[i + i / 3];
+#pragma unroll 1
     for (int i = lane; i < ntors; i += WARP) rec[8 + 3 * natom + i] = P.d[i];
     __syncwarp();
 }
@@ -630,7 +643,9 @@ __device__ __forceinline__ void slot_load(Slot P, const float* rec, int natom, i
     const int lane = lane_id();
     float* x = reinterpret_cast<float*>(P.x);
     if (lane < 8) P.h[lane] = rec[lane];
+#pragma unroll 1
     for (int i = lane; i < 3 * natom; i += WARP) x[i + i / 3] = rec[8 + i];
+#pragma unroll 1
     for (int i = lane; i < ntors; i += WARP) P.d[i] = rec[8 + 3 * natom + i];
     __syncwarp();
 }
@@ -743,24 +758,52 @@ __device__ __forceinline__ void intra_gather(const Topo& T, const float4* X, flo
 
 // ligands whose pair list does not fit the pair buffer: pairs spread over the lanes,
 // forces accumulated with shared-memory atomic adds
-__device__ __forceinline__ float intra_atomic(const Topo& T, const float4* X, float4* F, float vcap) {
+__device__ __noinline__ float intra_atomic(const int2* prec, int n, const float4* X, float4* F, float vcap) {
     float e = 0.f;
 #pragma unroll 1
-    for (int p = lane_id(); p < T.nprec; p += WARP) {
-        const int2 pr = T.prec(p);
+    for (int p = lane_id(); p < n; p += WARP) {
+        const int2 pr = prec[p];
         const int i = (pr.x & 0xFFF0) >> 4, j = (unsigned)pr.x >> 20;
-        const float dx = X[j].x - X[i].x, dy = X[j].y - X[i].y, dz = X[j].z - X[i].z;
+        const float d[3] = {X[j].x - X[i].x, X[j].y - X[i].y, X[j].z - X[i].z};
         float sc;
-        e += pair_scalar(dx, dy, dz, __int_as_float(pr.y), pr.x & PREC_HYD, pr.x & PREC_HB, vcap, sc);
+        e += pair_scalar(d[0], d[1], d[2], __int_as_float(pr.y), pr.x & PREC_HYD, pr.x & PREC_HB, vcap, sc);
         if (sc != 0.f) {
-            atomicAdd(&F[i].x, -sc * dx); atomicAdd(&F[i].y, -sc * dy); atomicAdd(&F[i].z, -sc * dz);
-            atomicAdd(&F[j].x, sc * dx); atomicAdd(&F[j].y, sc * dy); atomicAdd(&F[j].z, sc * dz);
+            atomicAdd(&F[i].x, -sc * d[0]); atomicAdd(&F[i].y, -sc * d[1]); atomicAdd(&F[i].z, -sc * d[2]);
+            atomicAdd(&F[j].x, sc * d[0]); atomicAdd(&F[j].y, sc * d[1]); atomicAdd(&F[j].z, sc * d[2]);
         }
     }
     return e;
 }
 
 // ---------------------------------------------------------------- energy + force
+// Bias of one atom (bfgs.cuh:356-388; vina.h:353-400) from its n records: the force, and in w the
+// energy so far plus the records' terms.
+__device__ __noinline__ float4 bias_atom(const float* bp, int n, float4 x, int type, float bias_k, bool hydrogen,
+                                         float energy) {
+    float fb0 = 0.f, fb1 = 0.f, fb2 = 0.f;
+#pragma unroll 1
+    for (int b = 0; b < n; b++, bp += 5) {
+        const float r0 = bp[0] - x.x, r1 = bp[1] - x.y, r2 = bp[2] - x.z;
+        if (type == 1) {
+            float rr = r0 * r0 + r1 * r1 + r2 * r2;
+            float eb = bp[3] * bias_k * expf(-rr / bp[4]);
+            fb0 += eb * 2.f * r0 / bp[4];
+            fb1 += eb * 2.f * r1 / bp[4];
+            fb2 += eb * 2.f * r2 / bp[4];
+            energy += eb;
+        } else {
+            float ka = hydrogen ? 0.1f : 30.f;
+            float rn = sqrtf(r0 * r0 + r1 * r1 + r2 * r2);
+            float ei = expf(3.f * (1.f - rn));
+            float eb = bp[3] * bias_k * ka / (1.f + ei);
+            float f = -eb * ei / (1.f + ei) * 3.f;
+            fb0 += f * r0 / rn; fb1 += f * r1 / rn; fb2 += f * r2 / rn;
+            energy += eb;
+        }
+    }
+    return make_float4(fb0, fb1, fb2, energy);
+}
+
 // Returns the warp-summed energy (bfgs.cuh:221-394) and leaves in F (per atom) and PB what
 // add_intra_forces needs to complete dE/dx per atom: a line-search trial that is rejected, and a
 // plain Metropolis move, need the energy alone (58 % of the search's evaluations are rejected
@@ -827,7 +870,7 @@ __device__ __forceinline__ float eval_e_f(const Topo& T, const Env& env, const f
     }
     __syncwarp();
     if (!FORCES || PB) energy += intra_energy<FORCES>(T, X, vcap, PB);
-    else energy += intra_atomic(T, X, F, vcap);
+    else energy += intra_atomic(reinterpret_cast<const int2*>(T.b + T.o_prec), T.nprec, X, F, vcap);
     // bias (bfgs.cuh:356-388; vina.h:353-400)
     if (env.bias_type != 0 && T.nbias > 0) {
         __syncwarp();
@@ -835,30 +878,10 @@ __device__ __forceinline__ float eval_e_f(const Topo& T, const Env& env, const f
         for (int i = lane; i < T.natom; i += WARP) {
             const int b0 = T.bias_off(i), b1 = T.bias_off(i + 1);
             if (b0 < b1) {
-                float fb0 = 0.f, fb1 = 0.f, fb2 = 0.f;
-                const float px = X[i].x, py = X[i].y, pz = X[i].z;
-#pragma unroll 1
-                for (int b = b0; b < b1; b++) {
-                    const float* bp = T.bias() + 5 * b;
-                    const float r0 = bp[0] - px, r1 = bp[1] - py, r2 = bp[2] - pz;
-                    if (env.bias_type == 1) {
-                        float rr = r0 * r0 + r1 * r1 + r2 * r2;
-                        float eb = bp[3] * env.bias_k * expf(-rr / bp[4]);
-                        fb0 += eb * 2.f * r0 / bp[4];
-                        fb1 += eb * 2.f * r1 / bp[4];
-                        fb2 += eb * 2.f * r2 / bp[4];
-                        energy += eb;
-                    } else {
-                        float ka = T.type(i) == VN_H ? 0.1f : 30.f;
-                        float rn = sqrtf(r0 * r0 + r1 * r1 + r2 * r2);
-                        float ei = expf(3.f * (1.f - rn));
-                        float eb = bp[3] * env.bias_k * ka / (1.f + ei);
-                        float f = -eb * ei / (1.f + ei) * 3.f;
-                        fb0 += f * r0 / rn; fb1 += f * r1 / rn; fb2 += f * r2 / rn;
-                        energy += eb;
-                    }
-                }
-                if constexpr (FORCES) { F[i].x += fb0; F[i].y += fb1; F[i].z += fb2; }
+                const float4 fb = bias_atom(T.bias() + 5 * b0, b1 - b0, X[i], env.bias_type, env.bias_k, T.type(i) == VN_H,
+                                            energy);
+                energy = fb.w;
+                if constexpr (FORCES) { F[i].x += fb.x; F[i].y += fb.y; F[i].z += fb.z; }
             }
         }
     }
@@ -1305,6 +1328,16 @@ __device__ __forceinline__ void mutate(const Topo& T, const Env& env, const Rng&
     }
 }
 
+// rotation vector of chain `chain`'s start (mc.cu:18-104)
+__device__ __noinline__ float4 start_rotation(int chain, int nchain) {
+    const float s = chain + 0.5f, n = (float)nchain;
+    const float r = sqrtf(s / n), R = sqrtf(1.f - s / n);
+    const float al = 2.f * PI_F * s / 1.4142136f, be = 2.f * PI_F * s / 1.5337512f;
+    float v[3];
+    quat_to_rotvec(r * sinf(al), r * cosf(al), R * sinf(be), R * cosf(be), v);
+    return make_float4(v[0], v[1], v[2], 0.f);
+}
+
 // initial randomisation (mc.cu:18-104); G is D floats of scratch, SC 2T floats
 __device__ __forceinline__ void randomize(const Topo& T, const Env& env, const Rng& rng, int chain, int nchain,
                                           Slot P, float* G, float* SC) {
@@ -1314,9 +1347,6 @@ __device__ __forceinline__ void randomize(const Topo& T, const Env& env, const R
         if (env.constraint) {
             G[0] = G[1] = G[2] = G[3] = G[4] = G[5] = 0.f;
         } else {
-            const float s = chain + 0.5f, n = (float)nchain;
-            const float r = sqrtf(s / n), R = sqrtf(1.f - s / n);
-            const float al = 2.f * PI_F * s / 1.4142136f, be = 2.f * PI_F * s / 1.5337512f;
             if (env.bias_type == 2) {
                 G[0] = G[1] = G[2] = 0.f;
             } else {
@@ -1324,7 +1354,8 @@ __device__ __forceinline__ void randomize(const Topo& T, const Env& env, const R
                 G[1] = (env.box_lo[1] + (env.box_hi[1] - env.box_lo[1]) * u01(u.y)) - P.h[2];
                 G[2] = (env.box_lo[2] + (env.box_hi[2] - env.box_lo[2]) * u01(u.z)) - P.h[3];
             }
-            quat_to_rotvec(r * sinf(al), r * cosf(al), R * sinf(be), R * cosf(be), G + 3);
+            const float4 v = start_rotation(chain, nchain);
+            G[3] = v.x; G[4] = v.y; G[5] = v.z;
         }
     }
 #pragma unroll 1

@@ -100,7 +100,9 @@ __device__ void load_initial(const int* blob, Slot P, int natom, int ntors) {
         P.h[1] = c0[0]; P.h[2] = c0[1]; P.h[3] = c0[2];
         P.h[4] = P.h[5] = P.h[6] = P.h[7] = 0.f;
     }
+#pragma unroll 1
     for (int i = lane; i < natom; i += WARP) P.x[i] = make_float4(x0[3 * i], x0[3 * i + 1], x0[3 * i + 2], 0.f);
+#pragma unroll 1
     for (int i = lane; i < ntors; i += WARP) P.d[i] = d0[i];
     __syncwarp();
 }
