@@ -521,7 +521,7 @@ __device__ __forceinline__ void rotvec_to_quat(float vx, float vy, float vz, flo
         const float h = th * 0.5f;
         if (h <= PI_F) __sincosf(h, &s, &c);     // hardware sine/cosine on [0, pi]
         else { const float2 sc = sincos_far(h); s = sc.x; c = sc.y; }
-        const float k = __fdividef(s, th);
+        const float k = div_ftz(s, th);
         q0 = c;
         q1 = k * vx;
         q2 = k * vy;
@@ -562,12 +562,12 @@ __device__ __forceinline__ RotGradBasis rot_grad_basis(float vx, float vy, float
     if (ang > EPS_F) {
         th = normalize_angle_2pi(ang);
         if (th > PI_F) { th = 2.f * PI_F - th; ang = -ang; }
-        B.vb0 = __fdividef(vx, ang); B.vb1 = __fdividef(vy, ang); B.vb2 = __fdividef(vz, ang);
+        B.vb0 = div_ftz(vx, ang); B.vb1 = div_ftz(vy, ang); B.vb2 = div_ftz(vz, ang);
     } else {
         th = 0.f; B.vb0 = B.vb1 = B.vb2 = 0.f;
     }
     __sincosf(th, &B.s, &B.c);                   // th in [0, pi]
-    if (th > EPS_F) { B.sdt = __fdividef(B.s, th); B.omc = __fdividef(1.f - B.c, th); }
+    if (th > EPS_F) { B.sdt = div_ftz(B.s, th); B.omc = div_ftz(1.f - B.c, th); }
     else { float t2 = th * th; B.sdt = 1.f - t2 / 6.f; B.omc = th / 2.f - th * t2 / 24.f; }
     return B;
 }
@@ -653,18 +653,13 @@ __device__ __forceinline__ void slot_load(Slot P, const float* rec, int natom, i
 // ---------------------------------------------------------------- grid sample
 __device__ __forceinline__ float grid_sample(const GridView& g, int map, float x, float y, float z,
                                              float& gx_, float& gy_, float& gz_) {
-    float u0 = (x - g.ox) * g.inv_s, u1 = (y - g.oy) * g.inv_s, u2 = (z - g.oz) * g.inv_s;
-    bool c0 = false, c1 = false, c2 = false;
-    if (!(u0 >= 0.f)) { u0 = 0.f; c0 = true; }      // also catches NaN
-    if (!(u1 >= 0.f)) { u1 = 0.f; c1 = true; }
-    if (!(u2 >= 0.f)) { u2 = 0.f; c2 = true; }
-    const float h0 = (float)(g.gx - 1), h1 = (float)(g.gy - 1), h2 = (float)(g.gz - 1);
-    if (u0 > h0) { u0 = h0; c0 = true; }
-    if (u1 > h1) { u1 = h1; c1 = true; }
-    if (u2 > h2) { u2 = h2; c2 = true; }
-    int i0 = min(max((int)floorf(u0), 0), g.gx - 2);
-    int i1 = min(max((int)floorf(u1), 0), g.gy - 2);
-    int i2 = min(max((int)floorf(u2), 0), g.gz - 2);
+    // outside the grid (and for NaN) the nearest point of its surface, with no gradient across it
+    const float r0 = (x - g.ox) * g.inv_s, r1 = (y - g.oy) * g.inv_s, r2 = (z - g.oz) * g.inv_s;
+    const float u0 = fminf(fmaxf(r0, 0.f), (float)(g.gx - 1));
+    const float u1 = fminf(fmaxf(r1, 0.f), (float)(g.gy - 1));
+    const float u2 = fminf(fmaxf(r2, 0.f), (float)(g.gz - 1));
+    const bool c0 = u0 != r0, c1 = u1 != r1, c2 = u2 != r2;
+    const int i0 = min((int)u0, g.gx - 2), i1 = min((int)u1, g.gy - 2), i2 = min((int)u2, g.gz - 2);
     const float fx = u0 - (float)i0, fy = u1 - (float)i1, fz = u2 - (float)i2;
     // 32-bit indices: the maps of one grid hold fewer than 2^31 values (20 x 81^3 at 30 A)
     const int sy = g.gx, sz = g.gx * g.gy;
@@ -976,7 +971,7 @@ __device__ __forceinline__ void refresh_center(const Topo& T, Slot P, float& cx,
     for (int i = lane; i < T.natom; i += WARP) { const float4 x = P.x[i]; s0 += x.x; s1 += x.y; s2 += x.z; }
     warp_sum3(s0, s1, s2);
     const float n = (float)T.natom;
-    cx = __fdividef(s0, n); cy = __fdividef(s1, n); cz = __fdividef(s2, n);
+    cx = div_ftz(s0, n); cy = div_ftz(s1, n); cz = div_ftz(s2, n);
     if (lane == 0) { P.h[1] = cx; P.h[2] = cy; P.h[3] = cz; }
     __syncwarp();
 }
