@@ -125,22 +125,27 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(GemmArgs g) {
 
 // ---------------------------------------------------------------------- tcgen05 GEMM, TMA-staged
 // Y[M x N] = act(X[M x K] W[K x N] + b) on the 5th-generation tensor cores: one CTA of 128
-// threads per 128-row tile, the FP32 accumulator (128 lanes x N columns) in tensor memory,
-// one thread issuing tcgen05.mma (kind::f16, BF16 operands, M = 128, K = 16 per instruction).
-// Operands arrive 32 K-values at a time by TMA (cp.async.bulk.tensor, each CTA its own), double
-// buffered: while the tensor cores work on one stage the next stage's tiles are loading.  The
-// canonical no-swizzle layouts come straight out of 3-D tensor maps:
+// threads per tile of 128 rows x 64 columns, the FP32 accumulator (128 lanes x 64 columns) in
+// tensor memory, one thread issuing tcgen05.mma (kind::f16, BF16 operands, M = 128, N = 64, K = 16 per
+// instruction).  Operands arrive 32 K-values at a time by TMA (cp.async.bulk.tensor, each CTA its
+// own) into a ring of six stages: at the network's sizes a GEMM is a few hundred nanoseconds of
+// tensor work behind 8 to 32 dependent copies and an epilogue, so copies run ahead and the columns
+// are spread over CTAs (1024 x 256 x 256: 10.5 us, and 16.5 at K = 672; with 256-wide tiles and two
+// stages 22 and 33).
+// The canonical no-swizzle layouts come straight out of 3-D tensor maps:
 //  * X (K-major): dims (8 k, rows, K/8 chunks), strides (ld*2 B, 16 B), box (8, 128, 4): four
 //    2 KB chunk blocks of 128 rows x 16 B; core matrices K-adjacent 2048 B apart, M-adjacent
 //    128 B apart;
-//  * W (N-major): dims (8 n, K rows, N/8 chunks), strides (N*2 B, 16 B), box (8, 32, N/8): N/8
+//  * W (N-major): dims (8 n, K rows, N/8 chunks), strides (N*2 B, 16 B), box (8, 32, 8): eight
 //    blocks of 32 k-rows x 16 B; core matrices K-adjacent 128 B, N-adjacent 512 B apart.
 // Rows beyond the map's extent arrive as zeros.  Split-K: grid.y CTAs share a tile's K range
 // (kchunk each) and write FP32 partials [split][M][N], summed by k_sum_splits in split order.
 // Every wait is bounded: on timeout the kernel records an error, waits (bounded) for its own
-// copies and MMAs in flight, and releases its tensor memory.  N is 64 or 256, kchunk a
-// multiple of 32.
-constexpr int TC_BM = 128, TC_BK = 32;
+// copies and MMAs in flight, and releases its tensor memory.  N is a multiple of 64, kchunk of
+// 32.
+constexpr int TC_BM = 128, TC_BK = 32, TC_BN = 64, TC_STAGES = 6;
+constexpr int TC_A_BYTES = TC_BM * TC_BK * 2, TC_B_BYTES = TC_BN * TC_BK * 2;      // 8 and 4 KB per stage
+constexpr int TC_SMEM = 1024 + TC_STAGES * (TC_A_BYTES + TC_B_BYTES);
 constexpr long long TC_SPIN = 1LL << 26;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -171,32 +176,28 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         : "memory");
 }
 
-template <int N>
 __global__ void __launch_bounds__(128) k_gemm_tc(const __grid_constant__ CUtensorMap tmX,
                                                  const __grid_constant__ CUtensorMap tmW,
-                                                 const float* __restrict__ bias, int M, int kchunk, int relu,
+                                                 const float* __restrict__ bias, int M, int N, int kchunk, int relu,
                                                  __nv_bfloat16* __restrict__ Y16, float* __restrict__ Y32, int* err) {
-    static_assert(N == 64 || N == 256, "N");
-    constexpr int A_BYTES = TC_BM * TC_BK * 2;              // 8 KB per stage
-    constexpr int B_BYTES = N * TC_BK * 2;                  // 4 or 16 KB per stage
     extern __shared__ __align__(16) unsigned char tc_smem_raw[];
     // operand stages from a 1024-byte boundary (the launch requests 1 KB of slack)
     unsigned char* tc_smem = tc_smem_raw + ((1024u - (smem_u32(tc_smem_raw) & 1023u)) & 1023u);
-    unsigned char* sA[2] = {tc_smem, tc_smem + A_BYTES};
-    unsigned char* sB[2] = {tc_smem + 2 * A_BYTES, tc_smem + 2 * A_BYTES + B_BYTES};
-    __shared__ __align__(8) uint64_t mma_bar[2], tma_bar[2];
+    auto sA = [&](int b) { return tc_smem + b * TC_A_BYTES; };
+    auto sB = [&](int b) { return tc_smem + TC_STAGES * TC_A_BYTES + b * TC_B_BYTES; };
+    __shared__ __align__(8) uint64_t mma_bar[TC_STAGES], tma_bar[TC_STAGES];
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail, s_issued;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.x * TC_BM;
-    const int kbase = blockIdx.y * kchunk;
+    const int kbase = blockIdx.y * kchunk, n0 = blockIdx.z * TC_BN;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     :: "r"(smem_u32(&s_tmem)), "r"(N) : "memory");
+                     :: "r"(smem_u32(&s_tmem)), "r"(TC_BN) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        for (int i = 0; i < 2; i++) {
+        for (int i = 0; i < TC_STAGES; i++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&mma_bar[i])) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&tma_bar[i])) : "memory");
         }
@@ -209,41 +210,42 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const __grid_constant__ CUtenso
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
     // instruction descriptor: F32 accumulate, BF16 A and B, A K-major, B N-major, N, M = 128
-    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(N >> 3) << 17) |
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(TC_BN >> 3) << 17) |
                            ((uint32_t)(TC_BM >> 4) << 24);
     const int nstage = kchunk / TC_BK;
     if (tid == 0) {
         int loaded = 0, consumed = 0, issued = -1;
         bool fail = false;
+        // stage s in buffer s % TC_STAGES, the buffer's use s / TC_STAGES (the barriers' phase)
         auto load = [&](int s) {
-            const int b = s & 1;
+            const int b = s % TC_STAGES;
             const int k0 = kbase + s * TC_BK;
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                         :: "r"(smem_u32(&tma_bar[b])), "r"((uint32_t)(A_BYTES + B_BYTES)) : "memory");
-            tma_load_3d(sA[b], &tmX, 0, m0, k0 >> 3, smem_u32(&tma_bar[b]));
-            tma_load_3d(sB[b], &tmW, 0, k0, 0, smem_u32(&tma_bar[b]));
+                         :: "r"(smem_u32(&tma_bar[b])), "r"((uint32_t)(TC_A_BYTES + TC_B_BYTES)) : "memory");
+            tma_load_3d(sA(b), &tmX, 0, m0, k0 >> 3, smem_u32(&tma_bar[b]));
+            tma_load_3d(sB(b), &tmW, 0, k0, n0 >> 3, smem_u32(&tma_bar[b]));
         };
-        if (nstage > 0) { load(0); loaded = 1; }
+        while (loaded < nstage && loaded < TC_STAGES) load(loaded++);
         for (int s = 0; s < nstage && !fail; s++) {
-            const int b = s & 1;
-            if (s + 1 < nstage) {
-                // the other buffer held stage s - 1: its MMAs finish before it is refilled
-                if (s >= 1 && !mbar_wait(smem_u32(&mma_bar[(s - 1) & 1]), (uint32_t)(((s - 1) >> 1) & 1))) {
+            const int b = s % TC_STAGES;
+            if (s >= 1 && loaded < nstage) {
+                // the buffer of stage s - 1: its MMAs finish before it is refilled
+                const int q = s - 1;
+                if (!mbar_wait(smem_u32(&mma_bar[q % TC_STAGES]), (uint32_t)((q / TC_STAGES) & 1))) {
                     fail = true;
                     break;
                 }
-                load(s + 1);
-                loaded = s + 2;
+                load(loaded++);
             }
-            if (!mbar_wait(smem_u32(&tma_bar[b]), (uint32_t)((s >> 1) & 1))) {
+            if (!mbar_wait(smem_u32(&tma_bar[b]), (uint32_t)((s / TC_STAGES) & 1))) {
                 fail = true;
                 break;
             }
             consumed = s + 1;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             for (int step = 0; step < TC_BK / 16; step++) {
-                const uint64_t da = umma_desc(smem_u32(sA[b] + step * 2 * 2048), 2048, 128);
-                const uint64_t db = umma_desc(smem_u32(sB[b] + step * 256), 128, 512);
+                const uint64_t da = umma_desc(smem_u32(sA(b) + step * 2 * 2048), 2048, 128);
+                const uint64_t db = umma_desc(smem_u32(sB(b) + step * 256), 128, 512);
                 const uint32_t acc = (s > 0 || step > 0) ? 1u : 0u;
                 asm volatile(
                     "{\n\t.reg .pred p;\n\t"
@@ -257,7 +259,8 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const __grid_constant__ CUtenso
         }
         if (fail) {
             // copies still in flight land before the buffers are released (bounded)
-            for (int t = consumed; t < loaded; t++) mbar_wait(smem_u32(&tma_bar[t & 1]), (uint32_t)((t >> 1) & 1));
+            for (int t = consumed; t < loaded; t++)
+                mbar_wait(smem_u32(&tma_bar[t % TC_STAGES]), (uint32_t)((t / TC_STAGES) & 1));
             s_fail = 1;
         }
         s_issued = issued;
@@ -268,7 +271,7 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const __grid_constant__ CUtenso
     // released under MMAs still in flight; if this bounded wait times out as well, what the
     // tensor cores still do with the released columns is undefined
     const int issued = s_issued;
-    if (issued >= 0 && !mbar_wait(smem_u32(&mma_bar[issued & 1]), (uint32_t)((issued >> 1) & 1))) {
+    if (issued >= 0 && !mbar_wait(smem_u32(&mma_bar[issued % TC_STAGES]), (uint32_t)((issued / TC_STAGES) & 1))) {
         if (tid == 0) s_fail = 1;
     }
     __syncthreads();
@@ -276,7 +279,7 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const __grid_constant__ CUtenso
     if (!s_fail && issued == nstage - 1) {
         const int m = m0 + warp * 32 + lane;                   // this thread's row (TMEM lane)
         float* Yp = Y32 ? Y32 + (size_t)blockIdx.y * M * N : nullptr;
-        for (int c = 0; c < N; c += 8) {
+        for (int c = 0; c < TC_BN; c += 8) {
             uint32_t r[8];
             asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
@@ -287,18 +290,20 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const __grid_constant__ CUtenso
                 float v[8];
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
-                    v[j] = __uint_as_float(r[j]) + (bias ? bias[c + j] : 0.f);
+                    v[j] = __uint_as_float(r[j]) + (bias ? bias[n0 + c + j] : 0.f);
                     if (relu) v[j] = fmaxf(v[j], 0.f);
                 }
                 if (Yp) {
 #pragma unroll
-                    for (int j = 0; j < 8; j++) Yp[(long long)m * N + c + j] = v[j];
+                    for (int j = 0; j < 8; j += 4)
+                        *reinterpret_cast<float4*>(Yp + (long long)m * N + n0 + c + j) =
+                            make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
                 }
                 if (Y16) {
                     __nv_bfloat162 h[4];
 #pragma unroll
                     for (int j = 0; j < 4; j++) h[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-                    *reinterpret_cast<uint4*>(Y16 + (long long)m * N + c) = *reinterpret_cast<uint4*>(h);
+                    *reinterpret_cast<uint4*>(Y16 + (long long)m * N + n0 + c) = *reinterpret_cast<uint4*>(h);
                 }
             }
         }
@@ -308,7 +313,7 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const __grid_constant__ CUtenso
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(N) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(TC_BN) : "memory");
 }
 
 // Y[i] = sum over splits s of P[s][i], in split order
@@ -385,13 +390,20 @@ __global__ void k_relu_bwd(long long n, const float* __restrict__ dh, const __nv
     }
 }
 
-// column sums of a rows x cols FP32 matrix
-__global__ void k_colsum(int rows, int cols, const float* __restrict__ s, float* __restrict__ d) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
+// column sums of a rows x cols FP32 matrix (cols a multiple of 8): a block per 8 columns, 128 rows at
+// a time, the 128 partial sums of a column folded in a fixed order.  (One thread per column, a chain
+// of dependent additions, took 62 us for 1024 rows, four times per training step: 40 % of it.)
+__global__ void __launch_bounds__(1024) k_colsum(int rows, int cols, const float* __restrict__ s, float* __restrict__ d) {
+    __shared__ float part[128][9];
+    const int c = threadIdx.x & 7, y = threadIdx.x >> 3, col = blockIdx.x * 8 + c;
     float acc = 0.f;
-    for (int r = 0; r < rows; r++) acc += s[(long long)r * cols + c];
-    d[c] = acc;
+    for (int r = y; r < rows; r += 128) acc += s[(long long)r * cols + col];
+    part[y][c] = acc;
+    for (int h = 64; h > 0; h >>= 1) {
+        __syncthreads();
+        if (y < h) part[y][c] += part[y + h][c];
+    }
+    if (y == 0) d[col] = part[0][c];
 }
 
 // Adam on the FP32 master parameters; refreshes their BF16 copy

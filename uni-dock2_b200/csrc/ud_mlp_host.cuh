@@ -75,8 +75,6 @@ struct MlpState {
         ck(cudaGetLastError(), "k_gemm_bf16");
     }
 
-    static constexpr int TC_SMEM = 96 * 1024;   // more than the 48 KB of stages: at most 2 CTAs
-                                                // per SM, so 2 x 256 tensor-memory columns fit
     DBuf<float> part;                            // split-K partial sums of the weight gradients
 
     // the driver's tensor-map encoder, looked up once through the runtime
@@ -108,11 +106,11 @@ struct MlpState {
         const cuuint32_t box[3] = {8, (cuuint32_t)TC_BM, TC_BK / 8};
         return encode(base, dim, str, box, "a K-major operand");
     }
-    // W operand: K rows x N values (row-major); N-major boxes of 32 rows
+    // W operand: K rows x N values (row-major); N-major boxes of 32 rows x 64 columns
     static CUtensorMap map_w(const __nv_bfloat16* base, int K, int N) {
         const cuuint64_t dim[3] = {8, (cuuint64_t)K, (cuuint64_t)(N / 8)};
         const cuuint64_t str[2] = {(cuuint64_t)N * 2, 16};
-        const cuuint32_t box[3] = {8, (cuuint32_t)TC_BK, (cuuint32_t)(N / 8)};
+        const cuuint32_t box[3] = {8, (cuuint32_t)TC_BK, (cuuint32_t)(TC_BN / 8)};
         return encode(base, dim, str, box, "an N-major operand");
     }
 
@@ -120,19 +118,16 @@ struct MlpState {
     // per row tile share the K range (FP32 partials summed in split order into Y32)
     void tc_run(cudaStream_t s, const __nv_bfloat16* X, int M, int K, int ldx, const __nv_bfloat16* W, int N,
                 const float* bias, int relu, __nv_bfloat16* Y16, float* Y32, int splits) {
-        if (K % 8 || ldx % 8 || (N != 64 && N != 256)) throw Fail(UD_EINVAL, "tensor-core GEMM shape");
+        if (K % 8 || ldx % 8 || N % TC_BN) throw Fail(UD_EINVAL, "tensor-core GEMM shape");
         const int kchunk = ((K + splits - 1) / splits + TC_BK - 1) / TC_BK * TC_BK;
         const CUtensorMap mx = map_x(X, M, K, ldx), mw = map_w(W, K, N);
-        const dim3 grid((unsigned)((M + TC_BM - 1) / TC_BM), (unsigned)splits);
+        const dim3 grid((unsigned)((M + TC_BM - 1) / TC_BM), (unsigned)splits, (unsigned)(N / TC_BN));
         float* y = Y32;
         if (splits > 1) {
             part.ensure((size_t)splits * M * N);
             y = part.p;
         }
-        if (N == 256)
-            k_gemm_tc<256><<<grid, 128, TC_SMEM, s>>>(mx, mw, bias, M, kchunk, relu, Y16, y, tc_err.p);
-        else
-            k_gemm_tc<64><<<grid, 128, TC_SMEM, s>>>(mx, mw, bias, M, kchunk, relu, Y16, y, tc_err.p);
+        k_gemm_tc<<<grid, 128, TC_SMEM, s>>>(mx, mw, bias, M, N, kchunk, relu, Y16, y, tc_err.p);
         ck(cudaGetLastError(), "k_gemm_tc");
         if (splits > 1) {
             const long long nmn = (long long)M * N;
@@ -162,8 +157,7 @@ struct MlpState {
     // a CUDA graph capture of the forward pass, which must not allocate
     void prepare(cudaStream_t s) {
         if (!use_tc || tc_attr) return;
-        ck(cudaFuncSetAttribute(k_gemm_tc<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM), "attr");
-        ck(cudaFuncSetAttribute(k_gemm_tc<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM), "attr");
+        ck(cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM), "attr");
         encoder();                                  // the encoder lookup, before any capture
         tc_err.ensure(1);
         ck(cudaMemsetAsync(tc_err.p, 0, sizeof(int), s), "memset");
@@ -202,7 +196,7 @@ struct MlpState {
     // contraction (the batch, for weight gradients) is split over CTAs to fill the GPU
     void tc_gemm(cudaStream_t s, const __nv_bfloat16* X, int M, int K, int ldx, const __nv_bfloat16* W, int N,
                  float* Y) {
-        const int tiles = (M + TC_BM - 1) / TC_BM;
+        const int tiles = (M + TC_BM - 1) / TC_BM * (N / TC_BN);
         int splits = 1;
         if (K >= 128) splits = std::max(1, std::min(K / 64, 296 / tiles));
         tc_run(s, X, M, K, ldx, W, N, nullptr, 0, nullptr, Y, splits);
@@ -225,7 +219,7 @@ struct MlpState {
         // output layer: dW4 = h3^T d [256 x 64], db4 = colsum(d), dh3 = d W4^T [n x 256]
         transpose(s, h16[2].p, n, mlp::HID, xt16.p, n32);
         tc_gemm(s, xt16.p, mlp::HID, n32, n32, d16.p, mlp::OUT, g.p + mlp::OFF_W4);
-        k_colsum<<<1, 64, 0, s>>>(n, mlp::OUT, dout.p, g.p + mlp::OFF_B4);
+        k_colsum<<<mlp::OUT / 8, 1024, 0, s>>>(n, mlp::OUT, dout.p, g.p + mlp::OFF_B4);
         transpose(s, w + mlp::OFF_W4, mlp::HID, mlp::OUT, wt16.p, mlp::HID);
         tc_gemm(s, d16.p, n, mlp::OUT, mlp::OUT, wt16.p, mlp::HID, dh.p);
         const long long off_w[3] = {mlp::OFF_W1, mlp::OFF_W2, mlp::OFF_W3};
@@ -238,7 +232,7 @@ struct MlpState {
             const int kin = l ? mlp::HID : mlp::IN;
             transpose(s, hin, n, kin, xt16.p, n32);
             tc_gemm(s, xt16.p, kin, n32, n32, d16.p, mlp::HID, g.p + off_w[l]);
-            k_colsum<<<1, 256, 0, s>>>(n, mlp::HID, dpre.p, g.p + off_b[l]);
+            k_colsum<<<mlp::HID / 8, 1024, 0, s>>>(n, mlp::HID, dpre.p, g.p + off_b[l]);
             if (l > 0) {
                 transpose(s, w + off_w[l], mlp::HID, mlp::HID, wt16.p, mlp::HID);
                 tc_gemm(s, d16.p, n, mlp::HID, mlp::HID, wt16.p, mlp::HID, dh.p);
@@ -264,7 +258,7 @@ struct MlpState {
         k_f32_to_bf16<<<blocks(no), 256, 0, s>>>(no, dout.p, d16.p);
         gemm(s, h16[2].p, 1, mlp::HID, d16.p, mlp::OUT, 1, mlp::HID, mlp::OUT, n, g.p + mlp::OFF_W4, mlp::OUT,
              nullptr, 0, nullptr, 0);
-        k_colsum<<<1, 64, 0, s>>>(n, mlp::OUT, dout.p, g.p + mlp::OFF_B4);
+        k_colsum<<<mlp::OUT / 8, 1024, 0, s>>>(n, mlp::OUT, dout.p, g.p + mlp::OFF_B4);
         gemm(s, d16.p, mlp::OUT, 1, w + mlp::OFF_W4, 1, mlp::OUT, n, mlp::HID, mlp::OUT, dh.p, mlp::HID, nullptr, 0,
              nullptr, 0);
         const long long off_w[3] = {mlp::OFF_W1, mlp::OFF_W2, mlp::OFF_W3};
@@ -277,7 +271,7 @@ struct MlpState {
             const int kin = l ? mlp::HID : mlp::IN;
             gemm(s, hin, 1, kin, d16.p, mlp::HID, 1, kin, mlp::HID, n, g.p + off_w[l], mlp::HID, nullptr, 0, nullptr,
                  0);
-            k_colsum<<<1, 256, 0, s>>>(n, mlp::HID, dpre.p, g.p + off_b[l]);
+            k_colsum<<<mlp::HID / 8, 1024, 0, s>>>(n, mlp::HID, dpre.p, g.p + off_b[l]);
             if (l > 0)
                 gemm(s, d16.p, mlp::HID, 1, w + off_w[l], 1, mlp::HID, n, mlp::HID, mlp::HID, dh.p, mlp::HID, nullptr,
                      0, nullptr, 0);
