@@ -136,6 +136,21 @@ def _p(a: Optional[np.ndarray]):
     return None if a is None else a.ctypes.data_as(C.c_void_p)
 
 
+def _flat(arrays) -> np.ndarray:
+    """All values of a sequence of arrays, one after another, as float32."""
+    try:
+        x = np.concatenate(arrays, axis=0)       # arrays of one trailing shape: one call for all
+    except (ValueError, TypeError):
+        x = np.concatenate([np.asarray(a, np.float32).reshape(-1) for a in arrays])
+    return np.ascontiguousarray(x, np.float32).reshape(-1)
+
+
+def _split(flat: np.ndarray, counts: np.ndarray) -> List[np.ndarray]:
+    """The views of flat that hold counts[0], counts[1], ... values."""
+    ends = np.cumsum(counts).tolist()
+    return [flat[a:b] for a, b in zip([0] + ends[:-1], ends)]
+
+
 def record_len(lig: Ligand) -> int:
     return 8 + 3 * lig.natom + lig.ntors
 
@@ -223,6 +238,8 @@ class Engine:
         self.h = h
         self.device = int(device)
         self.ligands: List[Ligand] = []
+        self._size_list: List[Tuple[int, int]] = []     # (atoms, torsions) of each ligand
+        self._size_array: Optional[np.ndarray] = None
         self.nchain = 0
         self.retain = 1
 
@@ -285,8 +302,11 @@ class Engine:
                                           _p(p["pairs"]), _p(p["bias_off"]), _p(p["bias"])))
         if bulk:
             self.ligands.extend(LigandRef(ligs, i) for i in range(len(ligs)))
+            self._size_list.extend(zip(ligs.natoms.tolist(), ligs.ntors.tolist()))
         else:
             self.ligands.extend(ligs)
+            self._size_list.extend((l.natom, l.ntors) for l in ligs)
+        self._size_array = None
 
     def device_memory(self):
         """(free, total) bytes of this context's device."""
@@ -297,31 +317,39 @@ class Engine:
     def clear_ligands(self):
         self._check(self.L.ud_clear_ligands(self.h))
         self.ligands = []
+        self._size_list = []
+        self._size_array = None
+
+    def _sizes(self, pose_lig: np.ndarray) -> Tuple[np.ndarray, np.ndarray]:
+        """(atoms, torsions) of the ligand of every pose."""
+        if self._size_array is None:
+            self._size_array = np.array(self._size_list, np.int64).reshape(-1, 2)
+        s = self._size_array[pose_lig]
+        return s[:, 0], s[:, 1]
 
     # ------------------------------------------------------------ compute
     def score_batch(self, pose_lig: Sequence[int], coords: Sequence[np.ndarray], centers, rotvecs,
                     mode: int = MODE_GRID, vcap: float = 1e30, slope: float = 1e6):
         pl = np.ascontiguousarray(pose_lig, np.int32)
-        x = np.ascontiguousarray(np.concatenate([np.asarray(c, np.float32).reshape(-1) for c in coords]))
+        x = _flat(coords)
         ce = np.ascontiguousarray(centers, np.float32).reshape(-1)
         rv = np.ascontiguousarray(rotvecs, np.float32).reshape(-1)
-        dims = [6 + self.ligands[l].ntors for l in pl]
+        dims = 6 + self._sizes(pl)[1]
         e = np.zeros(len(pl), np.float32)
-        g = np.zeros(int(sum(dims)), np.float32)
+        g = np.zeros(int(dims.sum()), np.float32)
         self._check(self.L.ud_score_batch(self.h, len(pl), _p(pl), _p(x), _p(ce), _p(rv), int(mode), float(vcap),
                                           float(slope), _p(e), _p(g)))
-        gs = np.split(g, np.cumsum(dims)[:-1]) if len(dims) > 1 else [g]
-        return e, gs
+        return e, _split(g, dims)
 
     def score_batch_timed(self, pose_lig: Sequence[int], coords: Sequence[np.ndarray], centers, rotvecs,
                           mode: int = MODE_GRID, vcap: float = 1e30, slope: float = 1e6, repeats: int = 5):
         """score_batch with the inputs resident on the device: (energies, gradients, mean
         kernel ms over `repeats` launches)."""
         pl = np.ascontiguousarray(pose_lig, np.int32)
-        x = np.ascontiguousarray(np.concatenate([np.asarray(c, np.float32).reshape(-1) for c in coords]))
+        x = _flat(coords)
         ce = np.ascontiguousarray(centers, np.float32).reshape(-1)
         rv = np.ascontiguousarray(rotvecs, np.float32).reshape(-1)
-        dims = np.array([6 + self.ligands[l].ntors for l in range(len(self.ligands))], np.int64)[pl]
+        dims = 6 + self._sizes(pl)[1]
         e = np.zeros(len(pl), np.float32)
         g = np.zeros(int(dims.sum()), np.float32)
         ms = C.c_float(0.0)
@@ -334,16 +362,15 @@ class Engine:
         """score_batch through ud_score_batch_noalloc: no device allocation inside the call;
         staging in the library's fixed per-device array (limits in include/udock_b200.h)."""
         pl = np.ascontiguousarray(pose_lig, np.int32)
-        x = np.ascontiguousarray(np.concatenate([np.asarray(c, np.float32).reshape(-1) for c in coords]))
+        x = _flat(coords)
         ce = np.ascontiguousarray(centers, np.float32).reshape(-1)
         rv = np.ascontiguousarray(rotvecs, np.float32).reshape(-1)
-        dims = [6 + self.ligands[l].ntors for l in pl]
+        dims = 6 + self._sizes(pl)[1]
         e = np.zeros(len(pl), np.float32)
-        g = np.zeros(int(sum(dims)), np.float32)
+        g = np.zeros(int(dims.sum()), np.float32)
         self._check(self.L.ud_score_batch_noalloc(self.h, len(pl), _p(pl), _p(x), _p(ce), _p(rv), int(mode),
                                                   float(vcap), float(slope), _p(e), _p(g)))
-        gs = np.split(g, np.cumsum(dims)[:-1]) if len(dims) > 1 else [g]
-        return e, gs
+        return e, _split(g, dims)
 
     def set_retain(self, retain: int):
         """Poses kept per chain (1..4); chain_poses/cluster then hold nchain * retain poses."""
@@ -446,23 +473,21 @@ class Engine:
 
     def score_terms(self, pose_lig, coords, mode: int = MODE_DIRECT, decomp: bool = False):
         pl = np.ascontiguousarray(pose_lig, np.int32)
-        x = np.ascontiguousarray(np.concatenate([np.asarray(c, np.float32).reshape(-1) for c in coords]))
+        x = _flat(coords)
         out = np.zeros((len(pl), 4), np.float32)
-        nd = int(sum(5 * self.ligands[l].natom for l in pl))
-        d = np.zeros(nd, np.float32) if decomp else None
+        d = np.zeros(int(5 * self._sizes(pl)[0].sum()), np.float32) if decomp else None
         self._check(self.L.ud_score_terms(self.h, len(pl), _p(pl), _p(x), int(mode), _p(out), _p(d)))
         return out, d
 
     def bfgs_batch(self, pose_lig, records: Sequence[np.ndarray], max_steps: int, rounds: int = 1,
                    vcap: float = 10.0, slope0: float = 1e6, ramp: bool = False, mode: int = MODE_GRID):
         pl = np.ascontiguousarray(pose_lig, np.int32)
-        recs = np.ascontiguousarray(np.concatenate([np.asarray(r, np.float32) for r in records]))
+        recs = _flat(records)
         ne = np.zeros(len(pl), np.int32)
         self._check(self.L.ud_bfgs_batch(self.h, len(pl), _p(pl), _p(recs), int(max_steps), int(rounds), float(vcap),
                                           float(slope0), int(ramp), int(mode), _p(ne)))
-        lens = [record_len(self.ligands[l]) for l in pl]
-        out = np.split(recs, np.cumsum(lens)[:-1]) if len(lens) > 1 else [recs]
-        return out, ne
+        nat, ntor = self._sizes(pl)
+        return _split(recs, 8 + 3 * nat + ntor), ne
 
     def search(self, seed: int, nchain: int, mc_steps: int, opt_steps: int, randomize: bool = True,
                mode: int = MODE_GRID) -> int:
