@@ -138,6 +138,8 @@ def _p(a: Optional[np.ndarray]):
 
 def _flat(arrays) -> np.ndarray:
     """All values of a sequence of arrays, one after another, as float32."""
+    if not isinstance(arrays, (list, tuple, np.ndarray)):
+        arrays = list(arrays)                    # a generator can be read once
     try:
         x = np.concatenate(arrays, axis=0)       # arrays of one trailing shape: one call for all
     except (ValueError, TypeError):
