@@ -171,6 +171,11 @@ constexpr unsigned ACC_MASK = (1u << 6) | (1u << 7) | (1u << 10) | (1u << 11);
 constexpr unsigned DON_MASK = (1u << 5) | (1u << 7) | (1u << 9) | (1u << 11) | (1u << 20);
 
 __device__ __forceinline__ float vdw(int t) { return c_vdw[t]; }
+// the same table in global memory, for lanes with different types: a constant load serves one
+// address at a time
+__device__ float g_vdw[NT] = {1.1f, 1.92f, 1.9f, 1.9f, 1.8f, 1.8f, 1.8f, 1.8f, 1.7f, 1.7f, 1.7f,
+                              1.7f, 1.5f, 2.2f, 2.1f, 2.0f, 1.8f, 2.0f, 2.2f, 2.3f, 1.2f};
+__device__ __forceinline__ float vdw_any(int t) { return __ldg(g_vdw + t); }
 
 __device__ __forceinline__ bool hyd_pair(int t1, int t2) {
     return ((1u << t1) & HYD_MASK) && ((1u << t2) & HYD_MASK);
@@ -838,7 +843,7 @@ __device__ __forceinline__ float eval_e_f(const Topo& T, const Env& env, const f
                     if (rr < 64.0) {
                         const int tj = (int)r.w;
                         float rn = sqrtf((float)rr), fdr;
-                        e_atom += eval_ef(rn - (r1 + vdw(tj)), ti, tj, fdr);
+                        e_atom += vina_ef(rn - (r1 + vdw_any(tj)), hyd_pair(ti, tj), hb_pair(ti, tj), fdr);
                         if (rn < EPS_F) rn = EPS_F;
                         fdr /= rn;
                         fx -= fdr * rv0; fy -= fdr * rv1; fz -= fdr * rv2;

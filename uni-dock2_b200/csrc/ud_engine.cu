@@ -333,10 +333,11 @@ __global__ void k_terms(const int* __restrict__ blobs, const LigDev* __restrict_
             if (j <= i) continue;
             float d0 = X[3 * j] - xi, d1 = X[3 * j + 1] - yi, d2 = X[3 * j + 2] - zi;
             float rr = d0 * d0 + d1 * d1 + d2 * d2;
-            if (rr < 64.f) e_intra += eval_e(sqrtf(rr) - (vdw(ti) + vdw(T.type(j))), ti, T.type(j));
+            if (rr < 64.f) e_intra += eval_e(sqrtf(rr) - (T.radius(i) + T.radius(j)), ti, T.type(j));
         }
         if (ti == VN_H) continue;
         float dec[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+        const float ri = T.radius(i);
         if (env.mode == 1) {
             int m = T.map_index(i);
             float gx, gy, gz;
@@ -346,7 +347,7 @@ __global__ void k_terms(const int* __restrict__ blobs, const LigDev* __restrict_
                 double rr = cutoff_r2(r.x, r.y, r.z, xi, yi, zi);
                 if (rr < 64.0) {
                     int tj = (int)r.w;
-                    float d = sqrtf((float)rr) - (vdw(ti) + vdw(tj));
+                    float d = sqrtf((float)rr) - (ri + vdw_any(tj));
                     e_inter += eval_e(d, ti, tj);
                     if (decomp) {
                         float x1 = d * 2.f, x2 = (d - 3.f) * 0.5f;
@@ -408,8 +409,9 @@ __global__ void k_terms(const int* __restrict__ blobs, const LigDev* __restrict_
 }
 
 // ====================================================================== BFGS batch
-template <int SUM>
-__global__ void k_bfgs(const int* __restrict__ blobs, const LigDev* __restrict__ ligs, int n, const int* item_lig,
+// MINB: CTAs per SM the register budget is sized for (see bfgs_kernel).
+template <int SUM, int MINB>
+__global__ void __launch_bounds__(256, MINB) k_bfgs(const int* __restrict__ blobs, const LigDev* __restrict__ ligs, int n, const int* item_lig,
                        const long long* item_off, float* recs, Env env, int max_steps, int rounds, float vcap,
                        float slope0, int ramp, int ws_max, int* nevals) {
     extern __shared__ __align__(16) float smem[];
@@ -1477,7 +1479,13 @@ void set_smem(K kernel, size_t bytes) {
 
 // The scoring and refinement kernels of a scoring mode: only direct sums walk the cell list.
 auto score_kernel(const Env& env) { return env.mode == UD_MODE_GRID ? k_score<SUM_GRID> : k_score<SUM_ROWS>; }
-auto bfgs_kernel(const Env& env) { return env.mode == UD_MODE_GRID ? k_bfgs<SUM_GRID> : k_bfgs<SUM_ROWS>; }
+// BFGS on n poses: with 80 registers three CTAs per SM, with 128 two that spill nothing.  The third pays
+// once there are poses for it (refinement of a 148-ligand screen batch 33.5 -> 30.1 ms), below that
+// the spills only cost (2048 poses 3.7 -> 4.2 ms).
+auto bfgs_kernel(ud_ctx* c, const Env& env, int n) {
+    if (n > c->nsm * 2 * 8) return env.mode == UD_MODE_GRID ? k_bfgs<SUM_GRID, 3> : k_bfgs<SUM_ROWS, 3>;
+    return env.mode == UD_MODE_GRID ? k_bfgs<SUM_GRID, 2> : k_bfgs<SUM_ROWS, 2>;
+}
 
 }  // namespace
 
@@ -2136,7 +2144,7 @@ int ud_bfgs_batch(ud_ctx* c, int n, const int* pose_lig, float* records, int max
         b.send(c->stream);
         int W = pick_warps(c, wsm, 0, 8);
         size_t smem = (size_t)W * wsm * 4;
-        const auto kb = bfgs_kernel(env);
+        const auto kb = bfgs_kernel(c, env, n);
         set_smem(kb, smem);
         kb<<<(n + W - 1) / W, 32 * W, smem, c->stream>>>(c->d_blobs.p, c->d_ligs.p, n, b.at<int>(ol),
                                                          b.at<long long>(oof), b.at<float>(orec), env, max_steps, rounds,
@@ -2191,12 +2199,14 @@ static SearchPlan plan_search(ud_ctx* c, int nchain, bool energy_only, K k3, K k
     int smem_sm = 0;
     ck(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, c->device), "attribute");
     const long long lim = smem_limit(c) / 4 - 64;       // floats of one CTA's shared memory
-    // CTA widths 8, 12 and 4 warps (want_w > 0: that one only): per width the instantiation
+    // CTA widths 4, 8 and 12 warps (want_w > 0: that one only): per width the instantiation
     // its shared memory allows (64 registers only where that reaches 32 warps per SM; 1 KB
-    // per CTA is reserved by the runtime), kept if it holds the most warps resident
+    // per CTA is reserved by the runtime), kept if it holds the most warps resident; of equals the
+    // narrowest, whose warps wait for fewer others at an item's end and which spreads few chains
+    // over more SMs (256 lead-sized ligands 102 -> 98 ms, 64 chains 53 -> 50 ms at 4 against 8)
     int per_sm = 0;
     K chosen = k3;
-    for (int w : {8, 12, 4}) {
+    for (int w : {4, 8, 12}) {
         if (want_w > 0 && w != want_w) continue;
         if ((long long)P.blob_max + (long long)w * P.wsm > lim) continue;
         const size_t smem = ((size_t)P.blob_max + (size_t)w * P.wsm) * 4;
@@ -2572,7 +2582,7 @@ static int dock_impl(ud_ctx* c, const ud_dock_params* p, float p_learned, long l
                 c->d_item_off.upload(io.data(), n, c->stream);
                 int W = pick_warps(c, wsm, 0, 8);
                 size_t smem = (size_t)W * wsm * 4;
-                const auto kb = bfgs_kernel(env);
+                const auto kb = bfgs_kernel(c, env, n);
                 set_smem(kb, smem);
                 kb<<<(n + W - 1) / W, 32 * W, smem, c->stream>>>(c->d_blobs.p, c->d_ligs.p, n, c->d_item_lig.p,
                                                                      c->d_item_off.p, c->d_best.p, env, 2,
