@@ -1103,16 +1103,25 @@ __global__ void k_cluster(const int* __restrict__ blobs, const LigDev* __restric
         int close = 0;
         for (int t = threadIdx.x; t < nl; t += blockDim.x) {
             const float* xl = base + (long long)lead[t] * L.stride + 8;
+            // the sum never falls: past the limit the pose is not close (tested every eight atoms, whose
+            // loads so overlap)
             float acc = 0.f;
-            for (int h = 0; h < T.nheavy; h++) {
-                int a = T.heavy(h);
-                float dx = __fsub_rn(xc[3 * a], xl[3 * a]);
-                float dy = __fsub_rn(xc[3 * a + 1], xl[3 * a + 1]);
-                float dz = __fsub_rn(xc[3 * a + 2], xl[3 * a + 2]);
+            const auto add = [&](int h) {
+                const int a = T.heavy(h);
+                const float dx = __fsub_rn(xc[3 * a], xl[3 * a]);
+                const float dy = __fsub_rn(xc[3 * a + 1], xl[3 * a + 1]);
+                const float dz = __fsub_rn(xc[3 * a + 2], xl[3 * a + 2]);
                 acc = __fmaf_rn(dx, dx, acc);
                 acc = __fmaf_rn(dy, dy, acc);
                 acc = __fmaf_rn(dz, dz, acc);
+            };
+            int h = 0;
+            for (; h + 8 <= T.nheavy && !(acc >= thr); h += 8) {
+#pragma unroll
+                for (int q = 0; q < 8; q++) add(h + q);
             }
+            if (!(acc >= thr))
+                for (; h < T.nheavy; h++) add(h);
             if (acc < thr) close = 1;
         }
         int any = __syncthreads_or(close);
