@@ -278,7 +278,9 @@ int ud_set_retain(ud_ctx* ctx, int retain);
  * shape, times short searches (3 MC steps) with 8, 12 or 4 warps per CTA and 1, 2 or 4
  * chains per warp per work item and keeps the fastest.  Results do not depend on the
  * packing.  Without it (and without ud_set_packing) the search takes the CTA width that
- * keeps the most warps resident.
+ * keeps the most warps resident, and where all chains fit the GPU four times over, a CTA of
+ * four warps on every chain, which evaluate a line search's trials at the same time (also
+ * with the autotuner on).
  * No reference counterpart (the reference launches one fixed shape, src/cuda/mc.cu:424-440). */
 int ud_set_autotune(ud_ctx* ctx, int on);
 
@@ -291,7 +293,8 @@ int ud_set_autotune(ud_ctx* ctx, int on);
 int ud_set_packing(ud_ctx* ctx, int warps_per_cta, int chains_per_warp);
 
 /* Launch shape of the last search (fused or learned): out4 = [warps per CTA, CTAs per SM,
- * register class (3, 4: 256-thread bound; 2: 384-thread bound), chains per warp per item].
+ * register class (3, 4: 256-thread bound; 2: 384-thread bound; 4 also where four warps share
+ * a chain), chains per warp per item].
  * No reference counterpart. */
 int ud_search_shape(const ud_ctx* ctx, int* out4);
 

@@ -1158,14 +1158,73 @@ __device__ UD_LS_ATTR float line_search(const Topo& T, const Env& env, Slot Px, 
     return e_new;
 }
 
+// A team is the warps of a CTA on one chain: every warp holds the chain's whole state and takes
+// every step of it, the same in all of them, but the trials of a line search, which its warps
+// evaluate at the same time; the warp of the first accepted trial completes the gradient and the others
+// copy its pose and gradient.  What is kept, counted and returned is what one warp's line search does.
+struct Team {
+    float* e;        // 2 x team size trial energies, by turns
+    int warp;        // this warp's number
+    int ws_max;      // floats from a warp's workspace to the next one's
+    int turn;
+};
+template <int SUM, int TEAM>
+__device__ UD_LS_ATTR float line_search_team(const Topo& T, const Env& env, Slot Px, Slot Pn, const Work& W, int dim,
+                                             float e0, float vcap, float slope, float& alpha_out, int& n_eval, Team& team) {
+    const float pg = gdot(W.p, W.g, dim);
+    float first = 1.f, e_new = 0.f;                       // the round's first step length
+#pragma unroll 1
+    for (int trial = 0; trial < LS_STEPS; trial += TEAM) {
+        float* e = team.e + TEAM * team.turn;
+        team.turn ^= 1;
+        if (trial + team.warp < LS_STEPS) {
+            apply_update(T, env, Px, Pn, W.p, first / (float)(1 << team.warp), W.sc);
+            e_new = eval_e_f<SUM>(T, env, Pn.x, W.F, vcap, slope, W.pb);
+            if (lane_id() == 0) e[team.warp] = e_new;
+        }
+        __syncthreads();
+        float alpha = first;
+        bool take = false;
+        int w = 0;
+#pragma unroll 1
+        for (; w < TEAM && trial + w < LS_STEPS; w++, alpha *= 0.5f) {
+            n_eval++;
+            e_new = e[w];
+            take = e_new - e0 < 1e-4f * alpha * pg;
+            if (take) break;
+        }
+        first = alpha;
+        if (!take && trial + w < LS_STEPS) continue;
+        const int win = take ? w : w - 1;                 // the last trial is kept even where it fails the test
+        if (win == team.warp) {
+            add_intra_forces(T, Pn.x, W.F, W.pb);
+            grad_from_forces(T, env, Pn, W.F, W.gn);
+        }
+        __syncthreads();
+        if (win != team.warp) {
+            const int to = (win - team.warp) * team.ws_max;
+            slot_words(reinterpret_cast<float4*>(Pn.h), reinterpret_cast<const float4*>(Pn.h + to),
+                       slot_floats(T.natom, T.ntors));
+#pragma unroll 1
+            for (int i = lane_id(); i < dim; i += WARP) W.gn[i] = W.gn[to + i];
+            __syncwarp();
+        }
+        __syncthreads();                                  // the winner's pose and gradient are read
+        break;
+    }
+    alpha_out = first;
+    return e_new;
+}
+
 // BFGS on the pose in slot ix (bfgs.cuh:729-829).  Uses slots ix and ialt, and keeps the start pose in
 // `ori` (a slot's words), to return to where the run has not improved on it: written once per run
 // and rarely read, so the search keeps it in global memory (L2), where it costs no residency.
 // Returns the slot index holding the result, whose header[0] is the final energy.
-template <int SUM>
+// TEAM > 1: by a team of warps.
+template <int SUM, int TEAM = 1>
 __device__ __forceinline__ int bfgs(const Topo& T, const Env& env, float* slots, int stride, int ix, int ialt,
                                     float4* ori, const Work& W, int max_steps, float vcap, float slope, int& n_eval,
-                                    int move_from = -1) {
+                                    int move_from = -1, Team* team = nullptr) {
     const int lane = lane_id();
     const int dim = 6 + T.ntors;
     float E_ori = 0.f, E = 0.f;
@@ -1178,9 +1237,14 @@ __device__ __forceinline__ int bfgs(const Topo& T, const Env& env, float* slots,
         if (step >= 0) minus_hv(W.H, W.g, W.p, dim);          // p = -H g
         float alpha;
         const bool mv = step < 0 && move_from >= 0;
-        const float E1 = line_search<SUM>(T, env, slot_at(slots, stride, mv ? move_from : cur, T.natom),
-                                     slot_at(slots, stride, mv ? cur : alt, T.natom), W, dim, E, vcap, slope, alpha,
-                                     n_eval, step < 0 ? (mv ? LS_MOVE : LS_INIT) : LS_TRIALS);
+        float E1;
+        if (TEAM > 1 && step >= 0)
+            E1 = line_search_team<SUM, TEAM>(T, env, slot_at(slots, stride, cur, T.natom), slot_at(slots, stride, alt, T.natom),
+                                             W, dim, E, vcap, slope, alpha, n_eval, *team);
+        else
+            E1 = line_search<SUM>(T, env, slot_at(slots, stride, mv ? move_from : cur, T.natom),
+                                  slot_at(slots, stride, mv ? cur : alt, T.natom), W, dim, E, vcap, slope, alpha, n_eval,
+                                  step < 0 ? (mv ? LS_MOVE : LS_INIT) : LS_TRIALS);
         if (step < 0) {
             E_ori = E = E1;
 #pragma unroll 1

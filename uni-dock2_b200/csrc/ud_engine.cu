@@ -409,15 +409,20 @@ __global__ void k_terms(const int* __restrict__ blobs, const LigDev* __restrict_
 }
 
 // ====================================================================== BFGS batch
-// MINB: CTAs per SM the register budget is sized for (see bfgs_kernel).
-template <int SUM, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_bfgs(const int* __restrict__ blobs, const LigDev* __restrict__ ligs, int n, const int* item_lig,
-                       const long long* item_off, float* recs, Env env, int max_steps, int rounds, float vcap,
-                       float slope0, int ramp, int ws_max, int* nevals) {
+// MINB: CTAs per SM the register budget is sized for; TEAM > 1: a CTA, a team of warps, per item (see
+// launch_bfgs).
+constexpr int TEAM_W = 4;
+template <int SUM, int MINB, int TEAM = 1>
+__global__ void __launch_bounds__(TEAM > 1 ? 32 * TEAM : 256, MINB)
+    k_bfgs(const int* __restrict__ blobs, const LigDev* __restrict__ ligs, int n, const int* item_lig,
+           const long long* item_off, float* recs, Env env, int max_steps, int rounds, float vcap, float slope0, int ramp,
+           int ws_max, int* nevals) {
     extern __shared__ __align__(16) float smem[];
     int warp = threadIdx.x >> 5, lane = lane_id();
-    int item = blockIdx.x * (blockDim.x >> 5) + warp;
+    __shared__ float s_trials[2 * TEAM];
+    const int item = TEAM > 1 ? (int)blockIdx.x : (int)(blockIdx.x * (blockDim.x >> 5)) + warp;
     if (item >= n) return;
+    Team team{s_trials, warp, ws_max, 0};
     float* ws = smem + (size_t)warp * ws_max;
     const LigDev L = ligs[item_lig[item]];
     Topo T = topo_view(blobs + L.blob_off);
@@ -429,9 +434,11 @@ __global__ void __launch_bounds__(256, MINB) k_bfgs(const int* __restrict__ blob
     float slope = slope0;
     for (int r = 0; r < rounds; r++) {
         const int alt = slot_next(cur);
-        cur = bfgs<SUM>(T, env, ws, stride, cur, alt, reinterpret_cast<float4*>(ws + slot_next(alt) * stride), W, max_steps, vcap, slope, ne);
+        cur = bfgs<SUM, TEAM>(T, env, ws, stride, cur, alt, reinterpret_cast<float4*>(ws + slot_next(alt) * stride), W,
+                              max_steps, vcap, slope, ne, -1, &team);
         if (ramp) slope = fminf(slope * 100.f, PENALTY_SLOPE);
     }
+    if (TEAM > 1 && warp != 0) return;
     slot_store(rec, slot_at(ws, stride, cur, T.natom), T.natom, T.ntors);
     if (nevals && lane == 0) nevals[item] = ne;
 }
@@ -468,6 +475,7 @@ __device__ __forceinline__ void init_best(float* out, Slot P, const Topo& T) {
 // RMAX: 1 (one pose, the common case, no extra registers) or 4 (R <= 4 at run time).
 template <int RMAX>
 struct Retained {
+    bool writes;             // false in all warps of a team but one
     float* out;
     int stride, R;
     float e0, e1, e2, e3;
@@ -491,13 +499,13 @@ struct Retained {
     }
     __device__ __forceinline__ void store(Slot P, const Topo& T, float energy) {
         if constexpr (RMAX == 1) {
-            slot_store(out, P, T.natom, T.ntors);
+            if (writes) slot_store(out, P, T.natom, T.ntors);
             e0 = energy;
         } else {
             const float t = worst();
             int r = 0;                               // the first record holding the highest energy
             if (!(e0 == t)) r = (R > 1 && e1 == t) ? 1 : ((R > 2 && e2 == t) ? 2 : 3);
-            slot_store(out + (long long)r * stride, P, T.natom, T.ntors);
+            if (writes) slot_store(out + (long long)r * stride, P, T.natom, T.ntors);
             if (r == 0) e0 = energy; else if (r == 1) e1 = energy; else if (r == 2) e2 = energy; else e3 = energy;
         }
     }
@@ -514,11 +522,11 @@ struct Proposal {
 // with one move applied (a random move, or a sample of the learned proposal), optimised by
 // BFGS with curl 10; Metropolis at T = 1.2 (step 0 always accepts); an accepted new best is
 // optimised again with curl 1000 and recorded.  Returns the accepted slot; sets *accepted.
-template <int SUM, class Keep>
+template <int SUM, int TEAM, class Keep>
 __device__ __forceinline__ int mc_step(const Topo& T, const Env& env, float* ws, int stride, int A, float4* ori,
                                        const Work& W,
                                        const Rng& rng, int step, int opt_steps, Keep& keep,
-                                       int& ne, const Proposal& prop, bool& accepted) {
+                                       int& ne, const Proposal& prop, bool& accepted, Team* team = nullptr) {
     const int lane = lane_id();
     const int C = slot_next(A);
     Slot SC = slot_at(ws, stride, C, T.natom);
@@ -580,8 +588,9 @@ __device__ __forceinline__ int mc_step(const Topo& T, const Env& env, float* ws,
     // curl 1000) go through one call site (phase 0 / 1).
     for (int phase = 0; phase < 2; phase++) {
         const int X = phase ? A : C;
-        const int R = bfgs<SUM>(T, env, ws, stride, X, slot_next(X), ori, W, opt_steps,
-                           phase ? VCAP_AUTH : VCAP_SEARCH, PENALTY_SLOPE, ne, (phase == 0 && learned) ? A : -1);
+        const int R = bfgs<SUM, TEAM>(T, env, ws, stride, X, slot_next(X), ori, W, opt_steps,
+                                      phase ? VCAP_AUTH : VCAP_SEARCH, PENALTY_SLOPE, ne, (phase == 0 && learned) ? A : -1,
+                                      team);
         const float e_new = ws[R * stride];
         if (phase == 0) {
             if (!(step == 0 || metropolis(e_acc, e_new, 1.2f, rx))) break;
@@ -604,7 +613,8 @@ __device__ __forceinline__ int mc_step(const Topo& T, const Env& env, float* ws,
 // threads: 4 CTAs = 64 registers, 3 = 80; 384 threads: 2 CTAs = 80 registers); the host
 // picks the width and instantiation that keep the most warps resident (shared memory
 // holds one topology blob per CTA, so wide CTAs pay when the blob is large).
-template <int MINB, int RMAX, int SUM, int NT = 256>
+// TEAM > 1: the warps of a CTA share every chain of its items (struct Team).
+template <int MINB, int RMAX, int SUM, int NT = 256, int TEAM = 1>
 __global__ void __launch_bounds__(NT, MINB) k_search(const int* __restrict__ blobs,
                                                 const LigDev* __restrict__ ligs, const int4* __restrict__ items,
                                                 int nitems, Env env, SearchP sp, float* best, int* work_counter,
@@ -616,6 +626,9 @@ __global__ void __launch_bounds__(NT, MINB) k_search(const int* __restrict__ blo
     const int warp = threadIdx.x >> 5, lane = lane_id();
     float* ws = wsbase + (size_t)warp * sp.ws_max;
     float4* const ori = sp.ori + (size_t)(blockIdx.x * (blockDim.x >> 5) + warp) * sp.ori_stride;
+    __shared__ float s_trials[2 * TEAM];
+    const bool leads = TEAM == 1 || warp == 0;
+    Team team{s_trials, warp, sp.ws_max, 0};
     unsigned long long my_evals = 0, my_heavy = 0;
     __shared__ __align__(8) uint64_t s_bar;
     __shared__ int s_flag;
@@ -637,10 +650,15 @@ __global__ void __launch_bounds__(NT, MINB) k_search(const int* __restrict__ blo
         const Topo T = topo_view(sblob);
         const int stride = slot_floats(T.natom, T.ntors);
         const Work W = work_at(ws, T);
+        int nth = 0;
         while (true) {
             int ci = 0;
-            if (lane == 0) ci = atomicAdd(&s_next, 1);
-            ci = __shfl_sync(FULL, ci, 0);
+            if constexpr (TEAM > 1) {
+                ci = nth++;
+            } else {
+                if (lane == 0) ci = atomicAdd(&s_next, 1);
+                ci = __shfl_sync(FULL, ci, 0);
+            }
             if (ci >= item.z) break;
             const int c = item.y + ci;
             float* out = best + L.best_off + (long long)c * sp.retain * L.stride;
@@ -649,8 +667,8 @@ __global__ void __launch_bounds__(NT, MINB) k_search(const int* __restrict__ blo
             Slot SA = slot_at(ws, stride, A, T.natom);
             load_initial(sblob, SA, T.natom, T.ntors);
             if (sp.randomize) randomize(T, env, rng, c, sp.nchain, SA, W.g, W.sc);
-            for (int r = 0; r < sp.retain; r++) init_best(out + (long long)r * L.stride, SA, T);
-            Retained<RMAX> keep{out, L.stride, sp.retain, 1e9f, 1e9f, 1e9f, 1e9f};
+            for (int r = 0; r < sp.retain && leads; r++) init_best(out + (long long)r * L.stride, SA, T);
+            Retained<RMAX> keep{leads, out, L.stride, sp.retain, 1e9f, 1e9f, 1e9f, 1e9f};
             int ne = 0;
             if (sp.mc_steps == 0) {
                 float e = eval_e_f<SUM, false>(T, env, SA.x, nullptr, VCAP_SEARCH, PENALTY_SLOPE, nullptr);
@@ -662,10 +680,10 @@ __global__ void __launch_bounds__(NT, MINB) k_search(const int* __restrict__ blo
                 const Proposal none{nullptr, 0.f};
                 bool acc;
                 for (int step = 0; step < sp.mc_steps; step++)
-                    A = mc_step<SUM>(T, env, ws, stride, A, ori, W, rng, step, sp.opt_steps, keep, ne, none, acc);
+                    A = mc_step<SUM, TEAM>(T, env, ws, stride, A, ori, W, rng, step, sp.opt_steps, keep, ne, none, acc, &team);
             }
-            my_evals += ne;
-            my_heavy += (unsigned long long)ne * T.nheavy;
+            my_evals += leads ? ne : 0;
+            my_heavy += leads ? (unsigned long long)ne * T.nheavy : 0;
         }
         __syncthreads();
     }
@@ -1027,7 +1045,7 @@ __global__ void __launch_bounds__(NT, MINB) k_learn_step(const int* __restrict__
             float* accp = acc + L.best_off + (long long)c * L.stride;
             const Rng rng{sp.k0, sp.k1, (uint32_t)c, (uint32_t)L.lig_uid};
             Slot SA = slot_at(ws, stride, 0, T.natom);
-            Retained<RMAX> keep{out, L.stride, sp.retain, 1e9f, 1e9f, 1e9f, 1e9f};
+            Retained<RMAX> keep{true, out, L.stride, sp.retain, 1e9f, 1e9f, 1e9f, 1e9f};
             if (step0 == 0) {
                 load_initial(sblob, SA, T.natom, T.ntors);
                 if (sp.randomize) randomize(T, env, rng, c, sp.nchain, SA, W.g, W.sc);
@@ -1046,7 +1064,7 @@ __global__ void __launch_bounds__(NT, MINB) k_learn_step(const int* __restrict__
                 const Proposal prop{(prop_out && step > 0 && s == 0) ? prop_out + g * mlp::OUT : nullptr,
                                     sp.p_learned};
                 bool accepted;
-                A = mc_step<SUM_GRID>(T, env, ws, stride, A, ori, W, rng, step, sp.opt_steps, keep, ne, prop, accepted);
+                A = mc_step<SUM_GRID, 1>(T, env, ws, stride, A, ori, W, rng, step, sp.opt_steps, keep, ne, prop, accepted);
                 // moves are recorded with blocks of one step (the features are the block's first pose)
                 if (rec_set.count && step > 0)
                     record_move(T, env, accp, slot_at(ws, stride, A, T.natom), accepted, rec_set, g);
@@ -1488,12 +1506,23 @@ void set_smem(K kernel, size_t bytes) {
 
 // The scoring and refinement kernels of a scoring mode: only direct sums walk the cell list.
 auto score_kernel(const Env& env) { return env.mode == UD_MODE_GRID ? k_score<SUM_GRID> : k_score<SUM_ROWS>; }
-// BFGS on n poses: with 80 registers three CTAs per SM, with 128 two that spill nothing.  The third pays
-// once there are poses for it (refinement of a 148-ligand screen batch 33.5 -> 30.1 ms), below that
-// the spills only cost (2048 poses 3.7 -> 4.2 ms).
-auto bfgs_kernel(ud_ctx* c, const Env& env, int n) {
-    if (n > c->nsm * 2 * 8) return env.mode == UD_MODE_GRID ? k_bfgs<SUM_GRID, 3> : k_bfgs<SUM_ROWS, 3>;
-    return env.mode == UD_MODE_GRID ? k_bfgs<SUM_GRID, 2> : k_bfgs<SUM_ROWS, 2>;
+// BFGS on n poses.  A few (up to four teams per SM) take a team of warps each.  Of more, with 128
+// registers two CTAs per SM spill nothing, with 80 three spill a little: the third pays once there are poses
+// for it (refinement of a 148-ligand screen batch 33.5 -> 30.1 ms), below that the spills only cost
+// (2048 poses 3.7 -> 4.2 ms).
+void launch_bfgs(ud_ctx* c, const Env& env, int n, int wsm, const int* lig, const long long* off, float* recs,
+                 int max_steps, int rounds, float vcap, float slope0, int ramp, int* nevals) {
+    const bool grid = env.mode == UD_MODE_GRID;
+    const bool team = n <= 4 * c->nsm && (long long)TEAM_W * wsm * 4 <= smem_limit(c) - 256;
+    const int W = team ? TEAM_W : pick_warps(c, wsm, 0, 8);
+    const size_t smem = (size_t)W * wsm * 4;
+    const auto k = team                    ? (grid ? k_bfgs<SUM_GRID, 4, TEAM_W> : k_bfgs<SUM_ROWS, 4, TEAM_W>)
+                   : n > 2 * W * c->nsm ? (grid ? k_bfgs<SUM_GRID, 3> : k_bfgs<SUM_ROWS, 3>)
+                                         : (grid ? k_bfgs<SUM_GRID, 2> : k_bfgs<SUM_ROWS, 2>);
+    set_smem(k, smem);
+    k<<<team ? n : (n + W - 1) / W, 32 * W, smem, c->stream>>>(c->d_blobs.p, c->d_ligs.p, n, lig, off, recs, env, max_steps,
+                                                            rounds, vcap, slope0, ramp, wsm, nevals);
+    ck(cudaGetLastError(), "k_bfgs launch");
 }
 
 }  // namespace
@@ -2151,14 +2180,8 @@ int ud_bfgs_batch(ud_ctx* c, int n, const int* pose_lig, float* records, int max
                      orec = b.add(packed.data(), packed.data(), tot * sizeof(float)),
                      on = b.add(nullptr, out_nevals, n * sizeof(int));
         b.send(c->stream);
-        int W = pick_warps(c, wsm, 0, 8);
-        size_t smem = (size_t)W * wsm * 4;
-        const auto kb = bfgs_kernel(c, env, n);
-        set_smem(kb, smem);
-        kb<<<(n + W - 1) / W, 32 * W, smem, c->stream>>>(c->d_blobs.p, c->d_ligs.p, n, b.at<int>(ol),
-                                                         b.at<long long>(oof), b.at<float>(orec), env, max_steps, rounds,
-                                                         vcap, slope0, ramp, wsm, b.at<int>(on));
-        ck(cudaGetLastError(), "k_bfgs launch");
+        launch_bfgs(c, env, n, wsm, b.at<int>(ol), b.at<long long>(oof), b.at<float>(orec), max_steps, rounds, vcap, slope0,
+                    ramp, b.at<int>(on));
         b.receive(c->stream, "k_bfgs");
         hs = 0;
         for (int i = 0; i < n; i++) {
@@ -2183,11 +2206,13 @@ struct SearchPlan {
     int minb = 3;          // instantiation: 3 or 4 (256-thread bound), 2 (384-thread bound)
     size_t smem = 0;
     long long tot = 0;
+    bool team = false;     // TEAM_W warps on every chain
 };
 
 extern "C++" {
 template <typename K>
-static SearchPlan plan_search(ud_ctx* c, int nchain, bool energy_only, K k3, K k4, K k12, int want_w = 0, int force_k = 0) {
+static SearchPlan plan_search(ud_ctx* c, int nchain, bool energy_only, K k3, K k4, K k12, int want_w = 0, int force_k = 0,
+                              K kteam = nullptr) {
     SearchPlan P;
     const int nlig = (int)c->h_ligs.size();
     std::vector<int> order(nlig);
@@ -2235,6 +2260,24 @@ static SearchPlan plan_search(ud_ctx* c, int nchain, bool energy_only, K k3, K k
         set_smem(k3, P.smem);
         ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k3, 32 * P.W, P.smem), "occupancy");
     }
+    // A launch with fewer chains than would fill the GPU takes a team of warps per chain, if all teams are
+    // resident at once: 64 chains of one ligand 53 -> 30 ms, 512 chains 22.9 -> 12.9 ms, and 512 chains
+    // on direct sums 104 -> 23 ms.
+    const long long total_chains = (long long)nlig * nchain;
+    if (kteam && !energy_only && want_w == 0 && force_k == 0 && (long long)P.blob_max + (long long)TEAM_W * P.wsm <= lim) {
+        const size_t smem = ((size_t)P.blob_max + (size_t)TEAM_W * P.wsm) * 4;
+        set_smem(kteam, smem);
+        int n = 0;
+        ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kteam, 32 * TEAM_W, smem), "occupancy");
+        if (total_chains <= (long long)c->nsm * n) {
+            P.team = true;
+            P.W = TEAM_W;
+            P.minb = 4;
+            P.smem = smem;
+            per_sm = n;
+            chosen = kteam;
+        }
+    }
     set_smem(chosen, P.smem);      // the candidates may have set a smaller size on the same kernel
     if (per_sm < 1) per_sm = 1;
     const long long resident = (long long)c->nsm * per_sm;
@@ -2243,9 +2286,8 @@ static SearchPlan plan_search(ud_ctx* c, int nchain, bool energy_only, K k3, K k
     // to its length but lengthen the launch's tail; on a 148-ligand screen batch (12-warp
     // CTAs, 400 MC steps) the search took 5.65 s at k = 1, 5.81 s at 2, 5.9-6.1 s at 3 and
     // 5.8-6.3 s at 4.  The autotuner and ud_set_packing can choose others.
-    const long long total_chains = (long long)nlig * nchain;
     const int k = force_k > 0 ? force_k : 1;
-    const int item_chains = P.W * k;
+    const int item_chains = P.team ? 1 : P.W * k;
     std::vector<int4> items;
     for (int l : order)
         for (int c0 = 0; c0 < nchain; c0 += item_chains)
@@ -2275,13 +2317,17 @@ static SearchKernel search_kernel_of(int minb, int rmax) {
     return minb == 4 ? k_search<4, 1, SUM> : (minb == 2 ? k_search<2, 1, SUM, 384> : k_search<3, 1, SUM>);
 }
 }  // extern "C++"
+static SearchKernel team_kernel(const Env& env, int rmax) {
+    if (env.mode == UD_MODE_GRID) return rmax > 1 ? k_search<4, 4, SUM_GRID, 128, TEAM_W> : k_search<4, 1, SUM_GRID, 128, TEAM_W>;
+    return rmax > 1 ? k_search<4, 4, SUM_LIST, 128, TEAM_W> : k_search<4, 1, SUM_LIST, 128, TEAM_W>;
+}
 static SearchKernel search_kernel(const Env& env, int minb, int rmax) {
     return env.mode == UD_MODE_GRID ? search_kernel_of<SUM_GRID>(minb, rmax) : search_kernel_of<SUM_LIST>(minb, rmax);
 }
 static SearchPlan plan_fused(ud_ctx* c, const Env& env, int nchain, bool energy_only, int want_w = 0, int force_k = 0) {
     const int r = c->retain;
     return plan_search(c, nchain, energy_only, search_kernel(env, 3, r), search_kernel(env, 4, r), search_kernel(env, 2, r),
-                       want_w, force_k);
+                       want_w, force_k, team_kernel(env, r));
 }
 
 static void run_search_plan(ud_ctx* c, const SearchPlan& P, const Env& env, uint64_t seed, int nchain, int mc_steps,
@@ -2299,7 +2345,7 @@ static void run_search_plan(ud_ctx* c, const SearchPlan& P, const Env& env, uint
     sp.ori = c->d_ori.p;
     sp.ori_stride = P.slot / 4;
     if (P.grid > 0) {
-        const SearchKernel kern = search_kernel(env, P.minb, c->retain);
+        const SearchKernel kern = P.team ? team_kernel(env, c->retain) : search_kernel(env, P.minb, c->retain);
         kern<<<P.grid, 32 * P.W, P.smem, c->stream>>>(c->d_blobs.p, c->d_ligs.p, c->d_items.p, P.nitems, env, sp,
                                                       c->d_best.p, c->d_counter.p, c->d_nevals.p);
         ck(cudaGetLastError(), "k_search launch");
@@ -2345,10 +2391,11 @@ static void launch_search(ud_ctx* c, uint64_t seed, int nchain, int mc_steps, in
     Env env = make_env(c, mode);
     c->nchain = nchain * c->retain;                  // records per ligand
     const bool energy_only = mc_steps == 0 || opt_steps == 0;
-    if (c->autotune && !(c->pack_w || c->pack_k)) autotune_search(c, env, seed, nchain, opt_steps, randomize);
-    const SearchPlan P = (c->pack_w || c->pack_k) ? plan_fused(c, env, nchain, energy_only, c->pack_w, c->pack_k)
-                         : c->autotune         ? plan_fused(c, env, nchain, energy_only, c->tune_w, c->tune_k)
-                                               : plan_fused(c, env, nchain, energy_only);
+    SearchPlan P = plan_fused(c, env, nchain, energy_only, c->pack_w, c->pack_k);
+    if (c->autotune && !(c->pack_w || c->pack_k) && !P.team) {
+        autotune_search(c, env, seed, nchain, opt_steps, randomize);
+        P = plan_fused(c, env, nchain, energy_only, c->tune_w, c->tune_k);
+    }
     c->best_floats = P.tot;
     c->d_best.ensure((size_t)P.tot);
     run_search_plan(c, P, env, seed, nchain, mc_steps, opt_steps, randomize);
@@ -2589,15 +2636,8 @@ static int dock_impl(ud_ctx* c, const ud_dock_params* p, float p_learned, long l
             if (n > 0) {
                 c->d_item_lig.upload(il.data(), n, c->stream);
                 c->d_item_off.upload(io.data(), n, c->stream);
-                int W = pick_warps(c, wsm, 0, 8);
-                size_t smem = (size_t)W * wsm * 4;
-                const auto kb = bfgs_kernel(c, env, n);
-                set_smem(kb, smem);
-                kb<<<(n + W - 1) / W, 32 * W, smem, c->stream>>>(c->d_blobs.p, c->d_ligs.p, n, c->d_item_lig.p,
-                                                                     c->d_item_off.p, c->d_best.p, env, 2,
-                                                                     p->refine_steps, VCAP_AUTH, 100.f, 1, wsm,
-                                                                     nullptr);
-                ck(cudaGetLastError(), "k_bfgs launch");
+                launch_bfgs(c, env, n, wsm, c->d_item_lig.p, c->d_item_off.p, c->d_best.p, 2, p->refine_steps, VCAP_AUTH,
+                            100.f, 1, nullptr);
                 c->counters[2]++;
             }
         }
