@@ -1,0 +1,30 @@
+"""Clustering, 32 poses of the ranking at a time, against the oracle around the batch's edges and from no
+two poses alike to all alike."""
+import numpy as np
+import pytest
+
+from gpu_helpers import engine_for
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nchain", [1, 31, 32, 33, 200, 300])
+@pytest.mark.parametrize("rmsd", [0.0, 1.0, 3.0, 99.0])
+def test_leaders_match_oracle(small_system, oracle64, nchain, rmsd):
+    """Torsion moves alone about a fixed root, so that the limits split the poses in every way."""
+    eng, _ = engine_for(small_system)
+    eng.set_flags(constraint=True)
+    eng.search(seed=3, nchain=nchain, mc_steps=0, opt_steps=0, randomize=True)
+    lead, cnt = eng.cluster(rmsd)
+    for l, lig in enumerate(small_system["ligs"]):
+        recs = eng.chain_poses(l)
+        x = recs[:, 8:8 + 3 * lig.natom].reshape(nchain, lig.natom, 3)[:, lig.types != 0].astype(np.float32)
+        e = np.where(np.isnan(recs[:, 0]), np.inf, recs[:, 0])
+        thr = np.float32(np.float32(rmsd) * np.float32(rmsd)) * np.float32(x.shape[1])
+        want = []
+        for c in np.argsort(e, kind="stable"):
+            d = [float(((x[c] - x[q]) ** 2).sum()) for q in want]
+            if not any(v < thr for v in d):
+                want.append(int(c))
+        assert list(lead[l, :cnt[l]]) == want and (lead[l, cnt[l]:] == -1).all()
+    eng.close()
