@@ -25,7 +25,7 @@ def test_leaders_match_a_plain_greedy_pass(small_system, nchain, rmsd):
         for c in np.argsort(e, kind="stable"):
             # squares summed in order with one rounding each, for all leaders at once
             d = np.zeros(len(want), np.float32)
-            diff = (x[c] - x[want]).reshape(len(want), -1).astype(np.float64)
+            diff = (x[c] - x[want]).reshape(len(want), 3 * x.shape[1]).astype(np.float64)
             for k in range(diff.shape[1]):
                 d = (diff[:, k] ** 2 + d).astype(np.float32)
             if not (d < thr).any():
