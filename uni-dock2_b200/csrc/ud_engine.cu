@@ -6,8 +6,9 @@
 //   k_score        E + generalised gradient of a pose batch   (src/cuda/bfgs_wrapper.cu:51-98)
 //   k_terms        final score terms, no curl                 (src/score/score.cpp:12-147)
 //   k_bfgs         BFGS / refinement rounds on pose records   (src/cuda/optimize.cu:14-77)
-//   k_search       persistent MC search: warp per chain; CTAs take (ligand, chain block)
-//                  work items in cost order from a global counter (src/cuda/mc.cu:109-448)
+//   k_search       persistent MC search: warp per chain, or four warps where the chains are few; CTAs
+//                  take (ligand, chain block) work items in cost order from a global counter
+//                  (src/cuda/mc.cu:109-448)
 //   k_cluster      CTA per ligand: energy ranking + greedy RMSD leaders (src/cuda/cluster.cu)
 //   k_filter       CTA per ligand: energy_range / num_pose filter (src/task/DockTask.cpp:188-220)
 //   k_gather       output records of the selected poses
