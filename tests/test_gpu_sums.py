@@ -86,3 +86,27 @@ def test_direct_search_follows_the_receptor(sums_sys, oracle64):
                                [r["rot_vec"] for r in recs], mode=MODE_DIRECT, vcap=10.0)
         assert rel_err([r["energy"] for r in recs], e) <= TOL
     eng.close()
+
+
+@pytest.mark.parametrize("mode", ["grid", "direct"])
+def test_scoring_workspace_of_the_largest_ligand(small_system, mode):
+    """Ligands at both ends of the sizes, alone (a workspace of their own) and beside the largest: the
+    same numbers."""
+    from conftest import random_poses
+    from ud2b200 import MODE_DIRECT, MODE_GRID, synth
+    from ud2b200.model import parse_ligands
+    ligs = parse_ligands({f"w{i}": synth.make_ligand(n, t, seed=720 + i, center=small_system["center"])
+                          for i, (n, t) in enumerate([(8, 0), (32, 1), (64, 14), (80, 20)])})
+    eng, _ = engine_for(dict(small_system, ligs=ligs))
+    m = MODE_DIRECT if mode == "direct" else MODE_GRID
+    rng = np.random.default_rng(3)
+    pl = np.arange(36) % 4
+    xs = [random_poses(ligs[l], small_system["box"], rng, 1)[0] for l in pl]
+    c, rv = np.array([x.mean(0) for x in xs]), rng.uniform(-1, 1, (36, 3)).astype(np.float32)
+    e, g = eng.score_batch(pl, xs, c, rv, mode=m, vcap=10.0)
+    for l in range(4):
+        at = np.flatnonzero(pl == l)
+        e1, g1 = eng.score_batch(pl[at], [xs[i] for i in at], c[at], rv[at], mode=m, vcap=10.0)
+        assert np.array_equal(e1, e[at]) and all(np.array_equal(a, g[i]) for a, i in zip(g1, at))
+        assert all(len(a) == 6 + ligs[l].ntors and np.isfinite(a).all() for a in g1)
+    eng.close()

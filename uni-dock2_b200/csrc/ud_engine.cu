@@ -59,6 +59,14 @@ __host__ __device__ inline int ws_floats(int n, int t, int npair, bool energy_on
     return energy_only ? w : w + r4(d * (d + 1)) + 4 * n + pb_floats(npair);
 }
 
+// and of the scoring kernel's: one slot, the forces, the pair buffer and the gradient.  Map lookups and
+// pair terms wait for memory, so warps in flight count, and the largest ligand of a call (80 atoms) sets
+// them.  With the BFGS workspace before, and with this one: 60,000 poses of uneven ligands 0.643 -> 0.461
+// ms on maps, 3.62 -> 3.32 ms direct; of screen ligands 0.361 -> 0.358 and 3.04 -> 2.74 ms.
+__host__ __device__ inline int score_floats(int n, int t, int npair) {
+    return slot_floats(n, t) + 4 * n + pb_floats(npair) + r4(6 + t);
+}
+
 struct LigDev {
     int blob_off;
     int blob_words;
@@ -230,15 +238,17 @@ __global__ void k_score(const int* __restrict__ blobs, const LigDev* __restrict_
     const int* blob = blobs + L.blob_off;
     Topo T = topo_view(blob);
     Slot P = slot_at(ws, 0, 0, T.natom);
-    Work W = work_at(ws, T);
+    float4* const F = reinterpret_cast<float4*>(ws + slot_floats(T.natom, T.ntors));
+    float* const pb = reinterpret_cast<float*>(F + T.natom);
+    float* const G = pb + pb_floats(T.nprec);
     const float* x = io.xyz + io.xoff[pose];
     for (int i = lane; i < 3 * T.natom; i += WARP) reinterpret_cast<float*>(P.x)[i + i / 3] = x[i];
     if (lane < 3) { P.h[1 + lane] = io.centers[3 * pose + lane]; P.h[4 + lane] = io.rotvecs[3 * pose + lane]; }
     __syncwarp();
-    float e = eval_e_grad<SUM>(T, env, P, W.F, W.g, vcap, slope, W.pb);
+    float e = eval_e_grad<SUM>(T, env, P, F, G, vcap, slope, pb_floats(T.nprec) ? pb : nullptr);
     if (lane == 0) out_e[pose] = e;
     float* g = out_g + io.goff[pose];
-    for (int i = lane; i < 6 + T.ntors; i += WARP) g[i] = W.g[i];
+    for (int i = lane; i < 6 + T.ntors; i += WARP) g[i] = G[i];
 }
 
 // ---------------------------------------------------------------------- bandwidth probe
@@ -1336,6 +1346,7 @@ struct LigHost {
     long long blob_off;
 };
 inline int lig_ws(const LigHost& h) { return ws_floats(h.natom, h.ntors, h.nprec); }
+inline int lig_score_ws(const LigHost& h) { return score_floats(h.natom, h.ntors, h.nprec); }
 }  // namespace
 
 #include "ud_mlp_host.cuh"
@@ -1520,6 +1531,13 @@ int pick_warps(ud_ctx* c, int ws, int extra, int want) {
     while (w > 1 && w * ws > lim) w--;
     if (w * ws > lim) throw Fail(UD_EINVAL, "ligand too large for shared memory");
     return w;
+}
+
+// The scoring kernel's, for a workspace of ws floats; a ligand whose BFGS workspace (full) fits in no
+// CTA is refused here as it is there.
+int score_warps(ud_ctx* c, int ws, int full) {
+    pick_warps(c, full, 0, 1);
+    return pick_warps(c, ws, 0, 8);
 }
 
 template <typename K>
@@ -1996,7 +2014,7 @@ int ud_score_batch(ud_ctx* c, int n, const int* pose_lig, const float* coords, c
         Env env = make_env(c, mode);
         std::vector<long long> xoff(n), goff(n);
         long long xs = 0, gs = 0;
-        int wsm = 0;
+        int wsm = 0, full = 0;
         for (int i = 0; i < n; i++) {
             int l = pose_lig[i];
             if (l < 0 || l >= (int)c->h_ligs.size()) throw Fail(UD_EINVAL, "pose ligand index out of range");
@@ -2004,7 +2022,8 @@ int ud_score_batch(ud_ctx* c, int n, const int* pose_lig, const float* coords, c
             goff[i] = gs;
             xs += 3LL * c->h_ligs[l].natom;
             gs += 6 + c->h_ligs[l].ntors;
-            wsm = std::max(wsm, lig_ws(c->h_ligs[l]));
+            wsm = std::max(wsm, lig_score_ws(c->h_ligs[l]));
+            full = std::max(full, lig_ws(c->h_ligs[l]));
         }
         BatchIO& b = c->io;
         b.begin();
@@ -2015,7 +2034,7 @@ int ud_score_batch(ud_ctx* c, int n, const int* pose_lig, const float* coords, c
                      orv = b.add(rotvecs, nullptr, 3 * (size_t)n * sizeof(float)),
                      oe = b.add(nullptr, out_e, n * sizeof(float)), og = b.add(nullptr, out_g, gs * sizeof(float));
         b.send(c->stream);
-        int W = pick_warps(c, wsm, 0, 8);
+        int W = score_warps(c, wsm, full);
         size_t smem = (size_t)W * wsm * 4;
         const auto ks = score_kernel(env);
         set_smem(ks, smem);
@@ -2081,7 +2100,7 @@ int ud_score_batch_timed(ud_ctx* c, int n, const int* pose_lig, const float* coo
         Env env = make_env(c, mode);
         std::vector<long long> xoff(n), goff(n);
         long long xs = 0, gs = 0;
-        int wsm = 0;
+        int wsm = 0, full = 0;
         for (int i = 0; i < n; i++) {
             int l = pose_lig[i];
             if (l < 0 || l >= (int)c->h_ligs.size()) throw Fail(UD_EINVAL, "pose ligand index out of range");
@@ -2089,7 +2108,8 @@ int ud_score_batch_timed(ud_ctx* c, int n, const int* pose_lig, const float* coo
             goff[i] = gs;
             xs += 3LL * c->h_ligs[l].natom;
             gs += 6 + c->h_ligs[l].ntors;
-            wsm = std::max(wsm, lig_ws(c->h_ligs[l]));
+            wsm = std::max(wsm, lig_score_ws(c->h_ligs[l]));
+            full = std::max(full, lig_ws(c->h_ligs[l]));
         }
         DBuf<int> dl; DBuf<long long> dxo, dgo; DBuf<float> dx, dc, dr, de, dg;
         dl.upload(pose_lig, n, c->stream);
@@ -2100,7 +2120,7 @@ int ud_score_batch_timed(ud_ctx* c, int n, const int* pose_lig, const float* coo
         dr.upload(rotvecs, 3 * (size_t)n, c->stream);
         de.ensure(n);
         dg.ensure(gs);
-        int W = pick_warps(c, wsm, 0, 8);
+        int W = score_warps(c, wsm, full);
         size_t smem = (size_t)W * wsm * 4;
         const auto ks = score_kernel(env);
         set_smem(ks, smem);
@@ -3122,13 +3142,14 @@ extern "C" int ud_score_batch_noalloc(ud_ctx* c, int n, const int* pose_lig, con
                                   "make one ud_score_batch, ud_search or ud_dock call first");
         Env env = make_env(c, mode);
         long long xs = 0, gs = 0;
-        int wsm = 0;
+        int wsm = 0, full = 0;
         for (int i = 0; i < n; i++) {
             const int l = pose_lig[i];
             if (l < 0 || l >= (int)c->h_ligs.size()) throw Fail(UD_EINVAL, "pose ligand index out of range");
             xs += 3LL * c->h_ligs[l].natom;
             gs += 6 + c->h_ligs[l].ntors;
-            wsm = std::max(wsm, lig_ws(c->h_ligs[l]));
+            wsm = std::max(wsm, lig_score_ws(c->h_ligs[l]));
+            full = std::max(full, lig_ws(c->h_ligs[l]));
         }
         const size_t o_lig = 0;
         const size_t o_xo = align256(o_lig + (size_t)n * sizeof(int));
@@ -3160,7 +3181,7 @@ extern "C" int ud_score_batch_noalloc(ud_ctx* c, int n, const int* pose_lig, con
         // every offset, energy and gradient word is written below: nothing has to start at zero
         k_pose_offsets<<<1, 1024, 0, st>>>(c->d_ligs.p, n, d_lig, d_xo, d_go);
         ck(cudaGetLastError(), "k_pose_offsets launch");
-        const int W = pick_warps(c, wsm, 0, 8);
+        const int W = score_warps(c, wsm, full);
         const size_t smem = (size_t)W * wsm * 4;
         const auto ks = score_kernel(env);
         set_smem(ks, smem);
