@@ -390,20 +390,28 @@ __global__ void k_relu_bwd(long long n, const float* __restrict__ dh, const __nv
     }
 }
 
-// column sums of a rows x cols FP32 matrix (cols a multiple of 8): a block per 8 columns, 128 rows at
-// a time, the 128 partial sums of a column folded in a fixed order.  (One thread per column, a chain
-// of dependent additions, took 62 us for 1024 rows, four times per training step: 40 % of it.)
+// column sums of a rows x cols FP32 matrix (cols a multiple of 8), every column's rows added in order: a
+// block per 8 columns; all threads load 128 rows ahead into shared memory while one thread per column
+// adds the 128 before them.  What bounds it is that chain of additions, 4 cycles a row.  (One thread per
+// column that also loads its rows took 62 us for 1024 rows, four times per training step: 40 % of it.
+// Sums of every 128th row folded pairwise were as fast, but rounded otherwise, which Adam's first steps
+// turn into other weights.)
 __global__ void __launch_bounds__(1024) k_colsum(int rows, int cols, const float* __restrict__ s, float* __restrict__ d) {
-    __shared__ float part[128][9];
+    __shared__ float tile[2][128][9];
     const int c = threadIdx.x & 7, y = threadIdx.x >> 3, col = blockIdx.x * 8 + c;
-    float acc = 0.f;
-    for (int r = y; r < rows; r += 128) acc += s[(long long)r * cols + col];
-    part[y][c] = acc;
-    for (int h = 64; h > 0; h >>= 1) {
-        __syncthreads();
-        if (y < h) part[y][c] += part[y + h][c];
+    float v = y < rows ? s[(long long)y * cols + col] : 0.f, acc = 0.f;
+    for (int r0 = 0, b = 0; r0 < rows; r0 += 128, b ^= 1) {
+        tile[b][y][c] = v;
+        __syncthreads();                     // also: the sums over this half of the tile two rounds ago are done
+        const int r = r0 + 128 + y;
+        if (r < rows) v = s[(long long)r * cols + col];
+        if (y == 0) {
+            const int n = min(128, rows - r0);
+#pragma unroll 16
+            for (int k = 0; k < n; k++) acc += tile[b][k][c];
+        }
     }
-    if (y == 0) d[col] = part[0][c];
+    if (y == 0) d[col] = acc;
 }
 
 // Adam on the FP32 master parameters; refreshes their BF16 copy

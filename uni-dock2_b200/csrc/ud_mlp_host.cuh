@@ -193,10 +193,11 @@ struct MlpState {
     }
 
     // Y[M x N] (FP32) = X[M x K] W[K x N] on the tensor cores, no bias or activation; a long
-    // contraction (the batch, for weight gradients) is split over CTAs to fill the GPU
+    // contraction (the batch, for weight gradients) is split over CTAs to fill the GPU: by rows of tiles
+    // alone, so that the partial sums, and with them the rounding, do not depend on the tiles' width
     void tc_gemm(cudaStream_t s, const __nv_bfloat16* X, int M, int K, int ldx, const __nv_bfloat16* W, int N,
                  float* Y) {
-        const int tiles = (M + TC_BM - 1) / TC_BM * (N / TC_BN);
+        const int tiles = (M + TC_BM - 1) / TC_BM;
         int splits = 1;
         if (K >= 128) splits = std::max(1, std::min(K / 64, 296 / tiles));
         tc_run(s, X, M, K, ldx, W, N, nullptr, 0, nullptr, Y, splits);
