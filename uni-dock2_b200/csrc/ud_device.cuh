@@ -1113,35 +1113,21 @@ __device__ __forceinline__ float gdot(const float* a, const float* b, int n) {
     return warp_sum(s);
 }
 
-// The lanes' part in the inverse Hessian's rows: a lane per row, and where two lanes per row fit the
-// warp (up to 16 rows: 10 torsions) one for each half of the columns, so that the chain of
-// dependent FP64 operations is half as long.  With one loop and no index search in the update:
-// 670 -> 624 ms on the 148-ligand screen batch at 100 MC steps.
-struct Rows {
-    int i, j0, j1;           // row, columns j0 .. j1 - 1
-    bool split;
-    __device__ __forceinline__ Rows(int dim) {
-        const int lane = lane_id(), h = (dim + 1) >> 1;
-        split = dim <= 16;
-        i = split ? lane & 15 : lane;
-        j0 = split && lane >= 16 ? h : 0;
-        j1 = split && lane < 16 ? h : dim;
-    }
-};
-// out = -H v for the packed symmetric H (bfgs.cuh:413-428)
+// out = -H v for the packed symmetric H (bfgs.cuh:413-428): a lane per row, its columns in order.
+// (Two lanes per row, one for each half of the columns, gave the same times, but sums in another order, which
+// part about one chain in 10^4 from the search as it was: 148-ligand screen batch at 100 MC steps 494.8 ms
+// either way.)  UNROLL: four columns ahead where a team's few warps wait for the chain of FP64 operations
+// (64 chains of one ligand 30.5 -> 29.4 ms); one where many warps share the instruction cache (the screen
+// batch 494.8 ms, with four 508).
+template <int UNROLL>
 __device__ __forceinline__ void minus_hv(const double* H, const float* v, float* out, int dim) {
-    const Rows R(dim);
 #pragma unroll 1
-    for (int i0 = 0; i0 < dim; i0 += WARP) {
-        const int i = R.i + i0, ri = i * (i + 1) / 2;
+    for (int i = lane_id(); i < dim; i += WARP) {
+        const int ri = i * (i + 1) / 2;
         double s = 0.0;
-        if (i < dim) {
-#pragma unroll 1
-            for (int j = R.j0, cj = j * (j + 1) / 2; j < R.j1; cj += ++j)
-                s += H[j < i ? ri + j : cj + i] * (double)v[j];            // H[j,i] or H[i,j]
-        }
-        if (R.split) s += __shfl_xor_sync(FULL, s, 16);
-        if (i < dim) out[i] = (float)(-s);
+#pragma unroll UNROLL
+        for (int j = 0, cj = 0; j < dim; cj += ++j) s += H[j < i ? ri + j : cj + i] * (double)v[j];   // H[j,i] or H[i,j]
+        out[i] = (float)(-s);
     }
     __syncwarp();
 }
@@ -1250,12 +1236,13 @@ __device__ __forceinline__ int bfgs(const Topo& T, const Env& env, float* slots,
     const int dim = 6 + T.ntors;
     float E_ori = 0.f, E = 0.f;
     const int ntri = dim * (dim + 1) / 2;
+    constexpr int HV_UNROLL = TEAM > 1 ? 4 : 1;
     int cur = ix, alt = ialt;
     // step -1 evaluates the start pose and sets H = I; move_from >= 0: the start pose is
     // that slot moved by W.p (line_search LS_MOVE)
 #pragma unroll 1
     for (int step = -1; step < max_steps; step++) {
-        if (step >= 0) minus_hv(W.H, W.g, W.p, dim);          // p = -H g
+        if (step >= 0) minus_hv<HV_UNROLL>(W.H, W.g, W.p, dim);          // p = -H g
         float alpha;
         const bool mv = step < 0 && move_from >= 0;
         float E1;
@@ -1301,18 +1288,22 @@ __device__ __forceinline__ int bfgs(const Topo& T, const Env& env, float* slots,
             __syncwarp();
         }
         if (alpha * yp < EPS_F) continue;
-        minus_hv(W.H, W.y, W.mhy, dim);
+        minus_hv<HV_UNROLL>(W.H, W.y, W.mhy, dim);
         const double yhy = -(double)gdot(W.y, W.mhy, dim);
         const double r = 1.0 / ((double)alpha * (double)yp);
         const double a = alpha;
         const double c1 = a * r, c2 = a * a * (r * r * yhy + r);
-        const Rows R(dim);
+        // Elements i + j(j+1)/2, i <= j: a lane per row i, and where two fit the warp (up to 16 rows: 10
+        // torsions) one for each half of the row's columns.  With the row loop of minus_hv, which has no index
+        // search either: 670 -> 624 ms on the 148-ligand screen batch at 100 MC steps.
+        const bool split = dim <= 16;
+        const int half = (dim + 1) >> 1, je = split && lane < 16 ? half : dim;
 #pragma unroll 1
-        for (int i = R.i; i < dim; i += WARP) {               // packed index i + j(j+1)/2, i <= j
+        for (int i = split ? lane & 15 : lane; i < dim; i += WARP) {
             const double pi = W.p[i], mi = W.mhy[i];
-            const int jb = max(R.j0, i);
+            const int jb = max(split && lane >= 16 ? half : 0, i);
 #pragma unroll 1
-            for (int j = jb, cj = jb * (jb + 1) / 2; j < R.j1; cj += ++j) {
+            for (int j = jb, cj = jb * (jb + 1) / 2; j < je; cj += ++j) {
                 const double pj = W.p[j];
                 W.H[cj + i] += c1 * (mi * pj + (double)W.mhy[j] * pi) + c2 * pi * pj;
             }
