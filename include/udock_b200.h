@@ -280,7 +280,7 @@ int ud_set_retain(ud_ctx* ctx, int retain);
  * packing.  Without it (and without ud_set_packing) the search takes the CTA width that
  * keeps the most warps resident, and where all chains fit the GPU four times over, a CTA of
  * four warps on every chain, which evaluate a line search's trials at the same time (also
- * with the autotuner on).
+ * with the autotuner on; not where a ligand has more than 4096 scored heavy pairs).
  * No reference counterpart (the reference launches one fixed shape, src/cuda/mc.cu:424-440). */
 int ud_set_autotune(ud_ctx* ctx, int on);
 

@@ -46,3 +46,50 @@ def test_team_refinement_is_that_of_one_warp(small_system, max_steps, rounds):
     eng.close()
     for i in range(1200):
         assert ne2[i] == ne[i % 10] and np.array_equal(many[i], few[i % 10], equal_nan=True)
+
+
+@pytest.fixture(scope="module")
+def large_sys(small_system):
+    """Ligands on both sides of the pair buffer's 4096 pairs (3813, 4215 and 4774), in a box that holds them."""
+    from ud2b200 import synth
+    from ud2b200.model import Box, parse_ligands
+    ligs = parse_ligands({f"p{i}": synth.make_ligand(n, t, seed=s, center=small_system["center"])
+                          for i, (n, t, s) in enumerate([(100, 10, 1), (100, 12, 2), (110, 10, 3)])})
+    return dict(small_system, ligs=ligs, box=Box.from_center_size(small_system["center"], [44.0] * 3))
+
+
+@pytest.mark.parametrize("which,team", [([0], True), ([1], False), ([2], False), ([0, 2], False)])
+def test_no_team_without_a_pair_buffer(large_sys, which, team):
+    """Atomic sums have no fixed order, a team needs equal bits: a launch that holds a ligand of more pairs
+    than the buffer takes one warp per chain.  Its recorded energies are those of its poses."""
+    from ud2b200 import MODE_GRID, split_record
+    ligs = [large_sys["ligs"][k] for k in which]
+    eng, _ = engine_for(dict(large_sys, ligs=ligs))
+    eng.search(seed=3, nchain=12, mc_steps=3, opt_steps=4, randomize=True)
+    assert (eng.search_shape()["register_class"] == 4) == team       # such a blob leaves one warp per chain no 64 registers
+    for l, lig in enumerate(ligs):
+        recs = [split_record(lig, r) for r in eng.chain_poses(l)]
+        recs = [r for r in recs if r["energy"] < 1e9]             # the others: no accepted pose
+        e, _ = eng.score_batch([l] * len(recs), [r["coords"] for r in recs], [r["center"] for r in recs],
+                               [r["rot_vec"] for r in recs], mode=MODE_GRID, vcap=1000.0)
+        assert len(recs) >= 4 and np.allclose([r["energy"] for r in recs], e, rtol=1e-4, atol=1e-4)
+    eng.close()
+
+
+def test_refinement_without_a_pair_buffer(large_sys):
+    """Few poses, those of ligands beyond the pair buffer among them: every pose's energy falls to that of
+    the pose returned."""
+    from ud2b200 import MODE_DIRECT, make_record, split_record
+    eng, _ = engine_for(large_sys)
+    ligs = large_sys["ligs"]
+    pl = [0, 1, 2, 0, 1, 2]
+    recs = [make_record(ligs[l], ligs[l].coords, ligs[l].center) for l in pl]
+    out, ne = eng.bfgs_batch(pl, recs, max_steps=5, rounds=2, vcap=1000.0, slope0=100.0, ramp=False, mode=MODE_DIRECT)
+    out = [split_record(ligs[l], r) for l, r in zip(pl, out)]
+    kw = dict(mode=MODE_DIRECT, vcap=1000.0, slope=100.0)
+    pose = lambda rs: ([r["coords"] for r in rs], [r["center"] for r in rs], [r["rot_vec"] for r in rs])  # noqa: E731
+    e, _ = eng.score_batch(pl, *pose(out), **kw)
+    e0, _ = eng.score_batch(pl, *pose([split_record(ligs[l], r) for l, r in zip(pl, recs)]), **kw)
+    eng.close()
+    assert (np.asarray(ne) > 2).all() and np.allclose([r["energy"] for r in out], e, rtol=1e-4, atol=1e-4)
+    assert (e <= e0).all() and (e < e0).any()

@@ -1169,6 +1169,8 @@ __device__ UD_LS_ATTR float line_search(const Topo& T, const Env& env, Slot Px, 
 // every step of it, the same in all of them, but the trials of a line search, which its warps
 // evaluate at the same time; the warp of the first accepted trial completes the gradient and the others
 // copy its pose and gradient.  What is kept, counted and returned is what one warp's line search does.
+// The warps meet at barriers by decisions that each of them takes for itself, so all that they compute must
+// be the same in every bit: no atomics (no team where the pair list does not fit the pair buffer).
 struct Team {
     float* e;        // 2 x team size trial energies, by turns
     int warp;        // this warp's number

@@ -1347,6 +1347,9 @@ struct LigHost {
 };
 inline int lig_ws(const LigHost& h) { return ws_floats(h.natom, h.ntors, h.nprec); }
 inline int lig_score_ws(const LigHost& h) { return score_floats(h.natom, h.ntors, h.nprec); }
+// Whether a team may take the ligand's chains: without a pair buffer the forces are summed by atomic adds, whose
+// order may differ between the team's warps, and with it the step at which each of them meets the others.
+inline bool lig_team(const LigHost& h) { return h.nprec <= PB_MAX; }
 }  // namespace
 
 #include "ud_mlp_host.cuh"
@@ -1547,14 +1550,15 @@ void set_smem(K kernel, size_t bytes) {
 
 // The scoring and refinement kernels of a scoring mode: only direct sums walk the cell list.
 auto score_kernel(const Env& env) { return env.mode == UD_MODE_GRID ? k_score<SUM_GRID> : k_score<SUM_ROWS>; }
-// BFGS on n poses.  A few (up to four teams per SM) take a team of warps each.  Of more, with 128
+// BFGS on n poses.  A few (up to four teams per SM) take a team of warps each, if `teams` (every ligand of
+// theirs passes lig_team).  Of more, with 128
 // registers two CTAs per SM spill nothing, with 80 three spill a little: the third pays once there are poses
 // for it (refinement of a 148-ligand screen batch 33.5 -> 30.1 ms), below that the spills only cost
 // (2048 poses 3.7 -> 4.2 ms).
-void launch_bfgs(ud_ctx* c, const Env& env, int n, int wsm, const int* lig, const long long* off, float* recs,
-                 int max_steps, int rounds, float vcap, float slope0, int ramp, int* nevals) {
+void launch_bfgs(ud_ctx* c, const Env& env, int n, int wsm, bool teams, const int* lig, const long long* off,
+                 float* recs, int max_steps, int rounds, float vcap, float slope0, int ramp, int* nevals) {
     const bool grid = env.mode == UD_MODE_GRID;
-    const bool team = n <= 4 * c->nsm && (long long)TEAM_W * wsm * 4 <= smem_limit(c) - 256;
+    const bool team = teams && n <= 4 * c->nsm && (long long)TEAM_W * wsm * 4 <= smem_limit(c) - 256;
     const int W = team ? TEAM_W : pick_warps(c, wsm, 0, 8);
     const size_t smem = (size_t)W * wsm * 4;
     const auto k = team                    ? (grid ? k_bfgs<SUM_GRID, 4, TEAM_W> : k_bfgs<SUM_ROWS, 4, TEAM_W>)
@@ -2201,12 +2205,14 @@ int ud_bfgs_batch(ud_ctx* c, int n, const int* pose_lig, float* records, int max
         std::vector<long long> off(n);
         long long tot = 0;
         int wsm = 0;
+        bool teams = true;
         for (int i = 0; i < n; i++) {
             int l = pose_lig[i];
             if (l < 0 || l >= (int)c->h_ligs.size()) throw Fail(UD_EINVAL, "pose ligand index out of range");
             off[i] = tot;
             tot += c->h_ligs[l].stride;
             wsm = std::max(wsm, lig_ws(c->h_ligs[l]));
+            teams &= lig_team(c->h_ligs[l]);
         }
         // records are packed at 8+3N+T floats each on the host side
         std::vector<float> packed(tot, 0.f);
@@ -2223,8 +2229,8 @@ int ud_bfgs_batch(ud_ctx* c, int n, const int* pose_lig, float* records, int max
                      orec = b.add(packed.data(), packed.data(), tot * sizeof(float)),
                      on = b.add(nullptr, out_nevals, n * sizeof(int));
         b.send(c->stream);
-        launch_bfgs(c, env, n, wsm, b.at<int>(ol), b.at<long long>(oof), b.at<float>(orec), max_steps, rounds, vcap, slope0,
-                    ramp, b.at<int>(on));
+        launch_bfgs(c, env, n, wsm, teams, b.at<int>(ol), b.at<long long>(oof), b.at<float>(orec), max_steps, rounds, vcap,
+                    slope0, ramp, b.at<int>(on));
         b.receive(c->stream, "k_bfgs");
         hs = 0;
         for (int i = 0; i < n; i++) {
@@ -2257,6 +2263,7 @@ template <typename K>
 static SearchPlan plan_search(ud_ctx* c, int nchain, bool energy_only, K k3, K k4, K k12, int want_w = 0, int force_k = 0,
                               K kteam = nullptr) {
     SearchPlan P;
+    bool teams = kteam != nullptr && !energy_only && want_w == 0 && force_k == 0;
     const int nlig = (int)c->h_ligs.size();
     std::vector<int> order(nlig);
     std::vector<double> cost(nlig);
@@ -2266,6 +2273,7 @@ static SearchPlan plan_search(ud_ctx* c, int nchain, bool energy_only, K k3, K k
         P.tot += (long long)nchain * c->retain * h.stride;
         P.wsm = std::max(P.wsm, ws_floats(h.natom, h.ntors, h.nprec, energy_only));
         P.slot = std::max(P.slot, slot_floats(h.natom, h.ntors));
+        teams &= lig_team(h);
         order[l] = l;
         // evaluation cost ~ intra pairs + grid atoms + kinematics, times BFGS length
         const double np = (double)(c->h_blobs[h.blob_off + H_NPAIR]);
@@ -2307,7 +2315,7 @@ static SearchPlan plan_search(ud_ctx* c, int nchain, bool energy_only, K k3, K k
     // resident at once: 64 chains of one ligand 53 -> 30 ms, 512 chains 22.9 -> 12.9 ms, and 512 chains
     // on direct sums 104 -> 23 ms.
     const long long total_chains = (long long)nlig * nchain;
-    if (kteam && !energy_only && want_w == 0 && force_k == 0 && (long long)P.blob_max + (long long)TEAM_W * P.wsm <= lim) {
+    if (teams && (long long)P.blob_max + (long long)TEAM_W * P.wsm <= lim) {
         const size_t smem = ((size_t)P.blob_max + (size_t)TEAM_W * P.wsm) * 4;
         set_smem(kteam, smem);
         int n = 0;
@@ -2667,9 +2675,11 @@ static int dock_impl(ud_ctx* c, const ud_dock_params* p, float p_learned, long l
             std::vector<int> il;
             std::vector<long long> io;
             int wsm = 0;
+            bool teams = true;
             for (int l = 0; l < nlig; l++) {
                 const LigHost& h = c->h_ligs[l];
                 wsm = std::max(wsm, lig_ws(h));
+                teams &= lig_team(h);
                 for (int k = 0; k < counts[l]; k++) {
                     il.push_back(l);
                     io.push_back(c->h_ligdev[l].best_off + (long long)leaders[(size_t)l * nrec_lig + k] * h.stride);
@@ -2679,8 +2689,8 @@ static int dock_impl(ud_ctx* c, const ud_dock_params* p, float p_learned, long l
             if (n > 0) {
                 c->d_item_lig.upload(il.data(), n, c->stream);
                 c->d_item_off.upload(io.data(), n, c->stream);
-                launch_bfgs(c, env, n, wsm, c->d_item_lig.p, c->d_item_off.p, c->d_best.p, 2, p->refine_steps, VCAP_AUTH,
-                            100.f, 1, nullptr);
+                launch_bfgs(c, env, n, wsm, teams, c->d_item_lig.p, c->d_item_off.p, c->d_best.p, 2, p->refine_steps,
+                            VCAP_AUTH, 100.f, 1, nullptr);
                 c->counters[2]++;
             }
         }
