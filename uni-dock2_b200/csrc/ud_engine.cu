@@ -59,6 +59,15 @@ __host__ __device__ inline int ws_floats(int n, int t, int npair, bool energy_on
     return energy_only ? w : w + r4(d * (d + 1)) + 4 * n + pb_floats(npair);
 }
 
+// The size of a ligand, by which one is refused as too large: the words that a workspace of four records and
+// plain vectors takes (and LigHost::size_stage, a topology of plain lists).  It follows the ligand alone, so that
+// a workspace or a topology laid out otherwise moves no limit: what does not fit in the layout in use takes the
+// kernels' far form (k_bfgs, k_search).
+__host__ __device__ inline int size_floats(int n, int t, int npair) {
+    const int d = 6 + t;
+    return 4 * rec_floats(n, t) + r4(3 * n) + 5 * r4(d) + r4(2 * t) + r4(d * (d + 1)) + pb_floats(npair);
+}
+
 // and of the scoring kernel's: one slot, the forces, the pair buffer and the gradient.  Map lookups and
 // pair terms wait for memory, so warps in flight count, and the largest ligand of a call (80 atoms) sets
 // them.  With the BFGS workspace before, and with this one: 60,000 poses of uneven ligands 0.643 -> 0.461
@@ -78,10 +87,10 @@ struct LigDev {
     long long out_off;   // float offset of the output records (num_pose capacity)
 };
 
-__device__ __forceinline__ Work work_at(float* ws, const Topo& T) {
+__device__ __forceinline__ Work work_at(float* ws, const Topo& T, int nslot = 3) {
     const int natom = T.natom, ntors = T.ntors, d = 6 + ntors;
     Work W;
-    W.g = ws + 3 * slot_floats(natom, ntors);
+    W.g = ws + nslot * slot_floats(natom, ntors);
     W.gn = W.g + r4(d);
     W.p = W.gn + r4(d);
     W.y = W.p + r4(d);
@@ -421,13 +430,14 @@ __global__ void k_terms(const int* __restrict__ blobs, const LigDev* __restrict_
 
 // ====================================================================== BFGS batch
 // MINB: CTAs per SM the register budget is sized for; TEAM > 1: a CTA, a team of warps, per item (see
-// launch_bfgs).
+// launch_bfgs).  FAR: the start pose in global memory (`far`, far_stride words per warp) instead of the workspace's
+// third slot, for ligands that do not fit otherwise (over about 3600 atoms).
 constexpr int TEAM_W = 4;
-template <int SUM, int MINB, int TEAM = 1>
+template <int SUM, int MINB, int TEAM = 1, bool FAR = false>
 __global__ void __launch_bounds__(TEAM > 1 ? 32 * TEAM : 256, MINB)
     k_bfgs(const int* __restrict__ blobs, const LigDev* __restrict__ ligs, int n, const int* item_lig,
            const long long* item_off, float* recs, Env env, int max_steps, int rounds, float vcap, float slope0, int ramp,
-           int ws_max, int* nevals) {
+           int ws_max, int* nevals, float4* far, int far_stride) {
     extern __shared__ __align__(16) float smem[];
     int warp = threadIdx.x >> 5, lane = lane_id();
     __shared__ float s_trials[2 * TEAM];
@@ -437,16 +447,15 @@ __global__ void __launch_bounds__(TEAM > 1 ? 32 * TEAM : 256, MINB)
     float* ws = smem + (size_t)warp * ws_max;
     const LigDev L = ligs[item_lig[item]];
     Topo T = topo_view(blobs + L.blob_off);
-    Work W = work_at(ws, T);
+    Work W = work_at(ws, T, FAR ? 2 : 3);
     float* rec = recs + item_off[item];
     const int stride = slot_floats(T.natom, T.ntors);
     slot_load(slot_at(ws, stride, 0, T.natom), rec, T.natom, T.ntors);
+    float4* const ori = FAR ? far + (size_t)item * far_stride : reinterpret_cast<float4*>(ws + 2 * stride);
     int cur = 0, ne = 0;
     float slope = slope0;
     for (int r = 0; r < rounds; r++) {
-        const int alt = slot_next(cur);
-        cur = bfgs<SUM, TEAM>(T, env, ws, stride, cur, alt, reinterpret_cast<float4*>(ws + slot_next(alt) * stride), W,
-                              max_steps, vcap, slope, ne, -1, &team);
+        cur = bfgs<SUM, TEAM>(T, env, ws, stride, cur, cur ^ 1, ori, W, max_steps, vcap, slope, ne, -1, &team);
         if (ramp) slope = fminf(slope * 100.f, PENALTY_SLOPE);
     }
     if (TEAM > 1 && warp != 0) return;
@@ -625,7 +634,8 @@ __device__ __forceinline__ int mc_step(const Topo& T, const Env& env, float* ws,
 // picks the width and instantiation that keep the most warps resident (shared memory
 // holds one topology blob per CTA, so wide CTAs pay when the blob is large).
 // TEAM > 1: the warps of a CTA share every chain of its items (struct Team).
-template <int MINB, int RMAX, int SUM, int NT = 256, int TEAM = 1>
+// FAR: the topology read from global memory, for ligands whose staged topology leaves no room for a warp.
+template <int MINB, int RMAX, int SUM, int NT = 256, int TEAM = 1, bool FAR = false>
 __global__ void __launch_bounds__(NT, MINB) k_search(const int* __restrict__ blobs,
                                                 const LigDev* __restrict__ ligs, const int4* __restrict__ items,
                                                 int nitems, Env env, SearchP sp, float* best, int* work_counter,
@@ -652,13 +662,14 @@ __global__ void __launch_bounds__(NT, MINB) k_search(const int* __restrict__ blo
         if (it >= nitems) break;
         const int4 item = items[it];          // (ligand, first chain, count, -)
         const LigDev L = ligs[item.x];
-        if (item.x != s_lig && !stage_blob(sblob, blobs + L.blob_off, L.stage_words, &s_bar, phase, &s_flag)) {
+        if (!FAR && item.x != s_lig && !stage_blob(sblob, blobs + L.blob_off, L.stage_words, &s_bar, phase, &s_flag)) {
             if (threadIdx.x == 0 && nevals) atomicAdd(nevals + 2, 1ull);
             break;
         }
         __syncthreads();
         if (threadIdx.x == 0) s_lig = item.x;
-        const Topo T = topo_view(sblob);
+        const int* const blob = FAR ? blobs + L.blob_off : sblob;
+        const Topo T = topo_view(blob);
         const int stride = slot_floats(T.natom, T.ntors);
         const Work W = work_at(ws, T);
         int nth = 0;
@@ -676,7 +687,7 @@ __global__ void __launch_bounds__(NT, MINB) k_search(const int* __restrict__ blo
             Rng rng{sp.k0, sp.k1, (uint32_t)c, (uint32_t)L.lig_uid};
             int A = 0;
             Slot SA = slot_at(ws, stride, A, T.natom);
-            load_initial(sblob, SA, T.natom, T.ntors);
+            load_initial(blob, SA, T.natom, T.ntors);
             if (sp.randomize) randomize(T, env, rng, c, sp.nchain, SA, W.g, W.sc);
             for (int r = 0; r < sp.retain && leads; r++) init_best(out + (long long)r * L.stride, SA, T);
             Retained<RMAX> keep{leads, out, L.stride, sp.retain, 1e9f, 1e9f, 1e9f, 1e9f};
@@ -1008,7 +1019,7 @@ __global__ void k_label_moves(const int* __restrict__ blobs, const LigDev* __res
     }
 }
 
-template <int MINB, int RMAX, int NT = 256>
+template <int MINB, int RMAX, int NT = 256, bool FAR = false>
 __global__ void __launch_bounds__(NT, MINB) k_learn_step(const int* __restrict__ blobs,
                                                         const LigDev* __restrict__ ligs, const int4* __restrict__ items,
                                                         int nitems, Env env, LearnP sp, const int* __restrict__ step_p,
@@ -1036,13 +1047,14 @@ __global__ void __launch_bounds__(NT, MINB) k_learn_step(const int* __restrict__
         if (it >= nitems) break;
         const int4 item = items[it];
         const LigDev L = ligs[item.x];
-        if (item.x != s_lig && !stage_blob(sblob, blobs + L.blob_off, L.stage_words, &s_bar, phase, &s_flag)) {
+        if (!FAR && item.x != s_lig && !stage_blob(sblob, blobs + L.blob_off, L.stage_words, &s_bar, phase, &s_flag)) {
             if (threadIdx.x == 0 && nevals) atomicAdd(nevals + 2, 1ull);
             break;
         }
         __syncthreads();
         if (threadIdx.x == 0) s_lig = item.x;
-        const Topo T = topo_view(sblob);
+        const int* const blob = FAR ? blobs + L.blob_off : sblob;
+        const Topo T = topo_view(blob);
         const int stride = slot_floats(T.natom, T.ntors);
         const Work W = work_at(ws, T);
         while (true) {
@@ -1058,7 +1070,7 @@ __global__ void __launch_bounds__(NT, MINB) k_learn_step(const int* __restrict__
             Slot SA = slot_at(ws, stride, 0, T.natom);
             Retained<RMAX> keep{true, out, L.stride, sp.retain, 1e9f, 1e9f, 1e9f, 1e9f};
             if (step0 == 0) {
-                load_initial(sblob, SA, T.natom, T.ntors);
+                load_initial(blob, SA, T.natom, T.ntors);
                 if (sp.randomize) randomize(T, env, rng, c, sp.nchain, SA, W.g, W.sc);
                 for (int r = 0; r < sp.retain; r++) init_best(out + (long long)r * L.stride, SA, T);
             } else {
@@ -1342,10 +1354,11 @@ struct BatchIO {
 };
 
 struct LigHost {
-    int natom, ntors, nheavy, blob_words, stride, nprec, stage_words;
+    int natom, ntors, nheavy, blob_words, stride, nprec, stage_words, size_stage;
     long long blob_off;
 };
 inline int lig_ws(const LigHost& h) { return ws_floats(h.natom, h.ntors, h.nprec); }
+inline int lig_size(const LigHost& h) { return size_floats(h.natom, h.ntors, h.nprec); }
 inline int lig_score_ws(const LigHost& h) { return score_floats(h.natom, h.ntors, h.nprec); }
 // Whether a team may take the ligand's chains: without a pair buffer the forces are summed by atomic adds, whose
 // order may differ between the team's warps, and with it the step at which each of them meets the others.
@@ -1384,7 +1397,7 @@ struct ud_ctx {
     DBuf<int> d_blobs;
     DBuf<LigDev> d_ligs;
     bool ligs_dirty = true;
-    int max_natom = 0, max_ntors = 0, max_blob = 0, max_stage = 0;
+    int max_natom = 0, max_ntors = 0, max_blob = 0, max_stage = 0, max_size_stage = 0;
     // search state
     int nchain = 0;
     long long best_floats = 0;
@@ -1536,10 +1549,10 @@ int pick_warps(ud_ctx* c, int ws, int extra, int want) {
     return w;
 }
 
-// The scoring kernel's, for a workspace of ws floats; a ligand whose BFGS workspace (full) fits in no
-// CTA is refused here as it is there.
-int score_warps(ud_ctx* c, int ws, int full) {
-    pick_warps(c, full, 0, 1);
+// The scoring kernel's, for a workspace of ws floats; a ligand of a size that fits in no CTA is refused, though
+// this workspace may.
+int score_warps(ud_ctx* c, int ws, int size) {
+    pick_warps(c, size, 0, 1);
     return pick_warps(c, ws, 0, 8);
 }
 
@@ -1550,23 +1563,42 @@ void set_smem(K kernel, size_t bytes) {
 
 // The scoring and refinement kernels of a scoring mode: only direct sums walk the cell list.
 auto score_kernel(const Env& env) { return env.mode == UD_MODE_GRID ? k_score<SUM_GRID> : k_score<SUM_ROWS>; }
-// BFGS on n poses.  A few (up to four teams per SM) take a team of warps each, if `teams` (every ligand of
-// theirs passes lig_team).  Of more, with 128
+// What the ligands of a refinement need: the largest size, workspace, slot and workspace of the far form, and whether
+// teams may take them all
+struct BfgsNeed {
+    int size = 0, ws = 0, slot = 0, far_ws = 0;
+    bool teams = true;
+    void add(const LigHost& h) {
+        ws = std::max(ws, lig_ws(h));
+        size = std::max(size, lig_size(h));
+        const int one = slot_floats(h.natom, h.ntors);
+        slot = std::max(slot, one);
+        far_ws = std::max(far_ws, lig_ws(h) - one);
+        teams &= lig_team(h);
+    }
+};
+// BFGS on n poses.  A few (up to four teams per SM) take a team of warps each.  Of more, with 128
 // registers two CTAs per SM spill nothing, with 80 three spill a little: the third pays once there are poses
 // for it (refinement of a 148-ligand screen batch 33.5 -> 30.1 ms), below that the spills only cost
 // (2048 poses 3.7 -> 4.2 ms).
-void launch_bfgs(ud_ctx* c, const Env& env, int n, int wsm, bool teams, const int* lig, const long long* off,
-                 float* recs, int max_steps, int rounds, float vcap, float slope0, int ramp, int* nevals) {
+void launch_bfgs(ud_ctx* c, const Env& env, int n, const BfgsNeed& need, const int* lig, const long long* off, float* recs,
+                 int max_steps, int rounds, float vcap, float slope0, int ramp, int* nevals) {
     const bool grid = env.mode == UD_MODE_GRID;
-    const bool team = teams && n <= 4 * c->nsm && (long long)TEAM_W * wsm * 4 <= smem_limit(c) - 256;
-    const int W = team ? TEAM_W : pick_warps(c, wsm, 0, 8);
+    pick_warps(c, need.size, 0, 1);                       // refuses what is too large
+    const bool team = need.teams && n <= 4 * c->nsm && (long long)TEAM_W * need.ws * 4 <= smem_limit(c) - 256;
+    const bool far = need.ws > smem_limit(c) / 4 - 64;
+    const int wsm = far ? need.far_ws : need.ws;
+    const int W = team ? TEAM_W : far ? 1 : pick_warps(c, wsm, 0, 8);
+    if (far) c->d_ori.ensure((size_t)n * (need.slot / 4));
     const size_t smem = (size_t)W * wsm * 4;
     const auto k = team                    ? (grid ? k_bfgs<SUM_GRID, 4, TEAM_W> : k_bfgs<SUM_ROWS, 4, TEAM_W>)
+                   : far                ? (grid ? k_bfgs<SUM_GRID, 2, 1, true> : k_bfgs<SUM_ROWS, 2, 1, true>)
                    : n > 2 * W * c->nsm ? (grid ? k_bfgs<SUM_GRID, 3> : k_bfgs<SUM_ROWS, 3>)
-                                         : (grid ? k_bfgs<SUM_GRID, 2> : k_bfgs<SUM_ROWS, 2>);
+                                        : (grid ? k_bfgs<SUM_GRID, 2> : k_bfgs<SUM_ROWS, 2>);
     set_smem(k, smem);
     k<<<team ? n : (n + W - 1) / W, 32 * W, smem, c->stream>>>(c->d_blobs.p, c->d_ligs.p, n, lig, off, recs, env, max_steps,
-                                                            rounds, vcap, slope0, ramp, wsm, nevals);
+                                                            rounds, vcap, slope0, ramp, wsm, nevals,
+                                                            far ? c->d_ori.p : nullptr, need.slot / 4);
     ck(cudaGetLastError(), "k_bfgs launch");
 }
 
@@ -1785,6 +1817,7 @@ int ud_add_ligands(ud_ctx* c, int nlig, const int* atom_off, const float* xyz, c
             int r0 = rot_off[t0], nrot = rot_off[t0 + T] - r0;
             int g0 = range_off[t0], nrange = range_off[t0 + T] - g0;
             int b0 = bias_off ? bias_off[a0] : 0, nb = bias_off ? bias_off[a0 + n] - b0 : 0;
+            int size_stage = 0;
             std::vector<int> blob(H_WORDS, 0);
             auto put = [&](int hdr, int count) {
                 blob[hdr] = (int)blob.size();
@@ -1923,6 +1956,9 @@ int ud_add_ligands(ud_ctx* c, int nlig, const int* atom_off, const float* xyz, c
                         }
                 }
                 blob[H_STAGE] = (int)blob.size();
+                // as plain lists: rotated atoms per torsion for the masks, gather lists without padding
+                size_stage = blob[H_STAGE] + r4(T + 1) + r4(nrot) - r4(n * ((T + 31) / 32)) + r4(n + 1) + r4(2 * np2) -
+                             r4(2 * nc) - r4(acc);
             }
             o = put(H_PAIR_OFF, n + 1);
             for (int i = 0; i <= n; i++) blob[o + i] = pair_off[a0 + i] - p0;
@@ -1970,6 +2006,7 @@ int ud_add_ligands(ud_ctx* c, int nlig, const int* atom_off, const float* xyz, c
             h.natom = n; h.ntors = T; h.nheavy = nheavy;
             h.blob_words = (int)blob.size();
             h.stage_words = blob[H_STAGE];
+            h.size_stage = size_stage;
             h.blob_off = (long long)c->h_blobs.size();
             h.stride = rec_floats(n, T);
             h.nprec = blob[H_NPREC];
@@ -1979,6 +2016,7 @@ int ud_add_ligands(ud_ctx* c, int nlig, const int* atom_off, const float* xyz, c
             c->max_ntors = std::max(c->max_ntors, T);
             c->max_blob = std::max(c->max_blob, h.blob_words);
             c->max_stage = std::max(c->max_stage, h.stage_words);
+            c->max_size_stage = std::max(c->max_size_stage, h.size_stage);
         }
         c->ligs_dirty = true;
         c->has_results = false;
@@ -1993,7 +2031,7 @@ int ud_clear_ligands(ud_ctx* c) {
     c->h_blobs.clear();
     c->h_ligs.clear();
     c->h_ligdev.clear();
-    c->max_natom = c->max_ntors = c->max_blob = c->max_stage = 0;
+    c->max_natom = c->max_ntors = c->max_blob = c->max_stage = c->max_size_stage = 0;
     c->ligs_dirty = true;
     c->has_results = false;
     c->nchain = 0;
@@ -2018,7 +2056,7 @@ int ud_score_batch(ud_ctx* c, int n, const int* pose_lig, const float* coords, c
         Env env = make_env(c, mode);
         std::vector<long long> xoff(n), goff(n);
         long long xs = 0, gs = 0;
-        int wsm = 0, full = 0;
+        int wsm = 0, size = 0;
         for (int i = 0; i < n; i++) {
             int l = pose_lig[i];
             if (l < 0 || l >= (int)c->h_ligs.size()) throw Fail(UD_EINVAL, "pose ligand index out of range");
@@ -2027,7 +2065,7 @@ int ud_score_batch(ud_ctx* c, int n, const int* pose_lig, const float* coords, c
             xs += 3LL * c->h_ligs[l].natom;
             gs += 6 + c->h_ligs[l].ntors;
             wsm = std::max(wsm, lig_score_ws(c->h_ligs[l]));
-            full = std::max(full, lig_ws(c->h_ligs[l]));
+            size = std::max(size, lig_size(c->h_ligs[l]));
         }
         BatchIO& b = c->io;
         b.begin();
@@ -2038,7 +2076,7 @@ int ud_score_batch(ud_ctx* c, int n, const int* pose_lig, const float* coords, c
                      orv = b.add(rotvecs, nullptr, 3 * (size_t)n * sizeof(float)),
                      oe = b.add(nullptr, out_e, n * sizeof(float)), og = b.add(nullptr, out_g, gs * sizeof(float));
         b.send(c->stream);
-        int W = score_warps(c, wsm, full);
+        int W = score_warps(c, wsm, size);
         size_t smem = (size_t)W * wsm * 4;
         const auto ks = score_kernel(env);
         set_smem(ks, smem);
@@ -2104,7 +2142,7 @@ int ud_score_batch_timed(ud_ctx* c, int n, const int* pose_lig, const float* coo
         Env env = make_env(c, mode);
         std::vector<long long> xoff(n), goff(n);
         long long xs = 0, gs = 0;
-        int wsm = 0, full = 0;
+        int wsm = 0, size = 0;
         for (int i = 0; i < n; i++) {
             int l = pose_lig[i];
             if (l < 0 || l >= (int)c->h_ligs.size()) throw Fail(UD_EINVAL, "pose ligand index out of range");
@@ -2113,7 +2151,7 @@ int ud_score_batch_timed(ud_ctx* c, int n, const int* pose_lig, const float* coo
             xs += 3LL * c->h_ligs[l].natom;
             gs += 6 + c->h_ligs[l].ntors;
             wsm = std::max(wsm, lig_score_ws(c->h_ligs[l]));
-            full = std::max(full, lig_ws(c->h_ligs[l]));
+            size = std::max(size, lig_size(c->h_ligs[l]));
         }
         DBuf<int> dl; DBuf<long long> dxo, dgo; DBuf<float> dx, dc, dr, de, dg;
         dl.upload(pose_lig, n, c->stream);
@@ -2124,7 +2162,7 @@ int ud_score_batch_timed(ud_ctx* c, int n, const int* pose_lig, const float* coo
         dr.upload(rotvecs, 3 * (size_t)n, c->stream);
         de.ensure(n);
         dg.ensure(gs);
-        int W = score_warps(c, wsm, full);
+        int W = score_warps(c, wsm, size);
         size_t smem = (size_t)W * wsm * 4;
         const auto ks = score_kernel(env);
         set_smem(ks, smem);
@@ -2204,15 +2242,13 @@ int ud_bfgs_batch(ud_ctx* c, int n, const int* pose_lig, float* records, int max
         Env env = make_env(c, mode);
         std::vector<long long> off(n);
         long long tot = 0;
-        int wsm = 0;
-        bool teams = true;
+        BfgsNeed need;
         for (int i = 0; i < n; i++) {
             int l = pose_lig[i];
             if (l < 0 || l >= (int)c->h_ligs.size()) throw Fail(UD_EINVAL, "pose ligand index out of range");
             off[i] = tot;
             tot += c->h_ligs[l].stride;
-            wsm = std::max(wsm, lig_ws(c->h_ligs[l]));
-            teams &= lig_team(c->h_ligs[l]);
+            need.add(c->h_ligs[l]);
         }
         // records are packed at 8+3N+T floats each on the host side
         std::vector<float> packed(tot, 0.f);
@@ -2229,8 +2265,8 @@ int ud_bfgs_batch(ud_ctx* c, int n, const int* pose_lig, float* records, int max
                      orec = b.add(packed.data(), packed.data(), tot * sizeof(float)),
                      on = b.add(nullptr, out_nevals, n * sizeof(int));
         b.send(c->stream);
-        launch_bfgs(c, env, n, wsm, teams, b.at<int>(ol), b.at<long long>(oof), b.at<float>(orec), max_steps, rounds, vcap,
-                    slope0, ramp, b.at<int>(on));
+        launch_bfgs(c, env, n, need, b.at<int>(ol), b.at<long long>(oof), b.at<float>(orec), max_steps, rounds, vcap, slope0,
+                    ramp, b.at<int>(on));
         b.receive(c->stream, "k_bfgs");
         hs = 0;
         for (int i = 0; i < n; i++) {
@@ -2256,13 +2292,15 @@ struct SearchPlan {
     size_t smem = 0;
     long long tot = 0;
     bool team = false;     // TEAM_W warps on every chain
+    bool far = false;      // topologies not staged
 };
 
 extern "C++" {
 template <typename K>
-static SearchPlan plan_search(ud_ctx* c, int nchain, bool energy_only, K k3, K k4, K k12, int want_w = 0, int force_k = 0,
-                              K kteam = nullptr) {
+static SearchPlan plan_search(ud_ctx* c, int nchain, bool energy_only, K k3, K k4, K k12, K kfar, int want_w = 0,
+                              int force_k = 0, K kteam = nullptr) {
     SearchPlan P;
+    int size = 0;
     bool teams = kteam != nullptr && !energy_only && want_w == 0 && force_k == 0;
     const int nlig = (int)c->h_ligs.size();
     std::vector<int> order(nlig);
@@ -2273,6 +2311,7 @@ static SearchPlan plan_search(ud_ctx* c, int nchain, bool energy_only, K k3, K k
         P.tot += (long long)nchain * c->retain * h.stride;
         P.wsm = std::max(P.wsm, ws_floats(h.natom, h.ntors, h.nprec, energy_only));
         P.slot = std::max(P.slot, slot_floats(h.natom, h.ntors));
+        size = std::max(size, lig_size(h));
         teams &= lig_team(h);
         order[l] = l;
         // evaluation cost ~ intra pairs + grid atoms + kinematics, times BFGS length
@@ -2284,6 +2323,7 @@ static SearchPlan plan_search(ud_ctx* c, int nchain, bool energy_only, K k3, K k
     int smem_sm = 0;
     ck(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, c->device), "attribute");
     const long long lim = smem_limit(c) / 4 - 64;       // floats of one CTA's shared memory
+    pick_warps(c, size, r4(c->max_size_stage), 1);      // refuses what is too large
     // CTA widths 4, 8 and 12 warps (want_w > 0: that one only): per width the instantiation
     // its shared memory allows (64 registers only where that reaches 32 warps per SM; 1 KB
     // per CTA is reserved by the runtime), kept if it holds the most warps resident; of equals the
@@ -2304,18 +2344,20 @@ static SearchPlan plan_search(ud_ctx* c, int nchain, bool energy_only, K k3, K k
         if (n * w > per_sm * P.W) { P.W = w; P.minb = minb; P.smem = smem; per_sm = n; chosen = kern; }
     }
     if (P.W == 0) {                                    // a ligand too large for 4 warps per CTA
+        P.far = (long long)P.blob_max + P.wsm > lim;
+        if (P.far) P.blob_max = 0;
         P.W = pick_warps(c, P.wsm, P.blob_max, 4);
         P.minb = 3;
         P.smem = ((size_t)P.blob_max + (size_t)P.W * P.wsm) * 4;
-        chosen = k3;
-        set_smem(k3, P.smem);
-        ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k3, 32 * P.W, P.smem), "occupancy");
+        chosen = P.far ? kfar : k3;
+        set_smem(chosen, P.smem);
+        ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, chosen, 32 * P.W, P.smem), "occupancy");
     }
     // A launch with fewer chains than would fill the GPU takes a team of warps per chain, if all teams are
     // resident at once: 64 chains of one ligand 53 -> 30 ms, 512 chains 22.9 -> 12.9 ms, and 512 chains
     // on direct sums 104 -> 23 ms.
     const long long total_chains = (long long)nlig * nchain;
-    if (teams && (long long)P.blob_max + (long long)TEAM_W * P.wsm <= lim) {
+    if (teams && !P.far && (long long)P.blob_max + (long long)TEAM_W * P.wsm <= lim) {
         const size_t smem = ((size_t)P.blob_max + (size_t)TEAM_W * P.wsm) * 4;
         set_smem(kteam, smem);
         int n = 0;
@@ -2375,10 +2417,13 @@ static SearchKernel team_kernel(const Env& env, int rmax) {
 static SearchKernel search_kernel(const Env& env, int minb, int rmax) {
     return env.mode == UD_MODE_GRID ? search_kernel_of<SUM_GRID>(minb, rmax) : search_kernel_of<SUM_LIST>(minb, rmax);
 }
+static SearchKernel far_kernel(const Env& env) {
+    return env.mode == UD_MODE_GRID ? k_search<3, 4, SUM_GRID, 256, 1, true> : k_search<3, 4, SUM_LIST, 256, 1, true>;
+}
 static SearchPlan plan_fused(ud_ctx* c, const Env& env, int nchain, bool energy_only, int want_w = 0, int force_k = 0) {
     const int r = c->retain;
     return plan_search(c, nchain, energy_only, search_kernel(env, 3, r), search_kernel(env, 4, r), search_kernel(env, 2, r),
-                       want_w, force_k, team_kernel(env, r));
+                       far_kernel(env), want_w, force_k, team_kernel(env, r));
 }
 
 static void run_search_plan(ud_ctx* c, const SearchPlan& P, const Env& env, uint64_t seed, int nchain, int mc_steps,
@@ -2396,7 +2441,9 @@ static void run_search_plan(ud_ctx* c, const SearchPlan& P, const Env& env, uint
     sp.ori = c->d_ori.p;
     sp.ori_stride = P.slot / 4;
     if (P.grid > 0) {
-        const SearchKernel kern = P.team ? team_kernel(env, c->retain) : search_kernel(env, P.minb, c->retain);
+        const SearchKernel kern = P.team  ? team_kernel(env, c->retain)
+                                  : P.far ? far_kernel(env)
+                                          : search_kernel(env, P.minb, c->retain);
         kern<<<P.grid, 32 * P.W, P.smem, c->stream>>>(c->d_blobs.p, c->d_ligs.p, c->d_items.p, P.nitems, env, sp,
                                                       c->d_best.p, c->d_counter.p, c->d_nevals.p);
         ck(cudaGetLastError(), "k_search launch");
@@ -2476,9 +2523,9 @@ static void launch_learned(ud_ctx* c, uint64_t seed, int nchain, int mc_steps, i
     const int lk = c->pack_k ? c->pack_k : 2;
     const SearchPlan P = c->retain > 1
                              ? plan_search(c, nchain, opt_steps == 0, k_learn_step<3, 4>, k_learn_step<4, 4>, k_learn_step<2, 4, 384>,
-                                           c->pack_w, lk)
+                                           k_learn_step<3, 4, 256, true>, c->pack_w, lk)
                              : plan_search(c, nchain, opt_steps == 0, k_learn_step<3, 1>, k_learn_step<4, 1>, k_learn_step<2, 1, 384>,
-                                           c->pack_w, lk);
+                                           k_learn_step<3, 4, 256, true>, c->pack_w, lk);
     c->best_floats = P.tot;
     c->d_best.ensure((size_t)P.tot);
     c->d_acc.ensure((size_t)P.tot);
@@ -2528,7 +2575,8 @@ static void launch_learned(ud_ctx* c, uint64_t seed, int nchain, int mc_steps, i
     sp.p_learned = std::min(1.f, p_learned * (float)sp.block);
     sp.mc_steps = mc_steps;
     const int nblocks = (mc_steps + sp.block - 1) / sp.block;
-    auto kern = c->retain > 1
+    auto kern = P.far ? k_learn_step<3, 4, 256, true>
+                : c->retain > 1
                     ? (P.minb == 4 ? k_learn_step<4, 4> : (P.minb == 2 ? k_learn_step<2, 4, 384> : k_learn_step<3, 4>))
                     : (P.minb == 4 ? k_learn_step<4, 1> : (P.minb == 2 ? k_learn_step<2, 1, 384> : k_learn_step<3, 1>));
     const int fblocks = (int)std::min<long long>((nch * 32 + 255) / 256, (long long)c->nsm * 16);
@@ -2674,12 +2722,10 @@ static int dock_impl(ud_ctx* c, const ud_dock_params* p, float p_learned, long l
         if (p->refine_steps > 0) {
             std::vector<int> il;
             std::vector<long long> io;
-            int wsm = 0;
-            bool teams = true;
+            BfgsNeed need;
             for (int l = 0; l < nlig; l++) {
                 const LigHost& h = c->h_ligs[l];
-                wsm = std::max(wsm, lig_ws(h));
-                teams &= lig_team(h);
+                need.add(h);
                 for (int k = 0; k < counts[l]; k++) {
                     il.push_back(l);
                     io.push_back(c->h_ligdev[l].best_off + (long long)leaders[(size_t)l * nrec_lig + k] * h.stride);
@@ -2689,8 +2735,8 @@ static int dock_impl(ud_ctx* c, const ud_dock_params* p, float p_learned, long l
             if (n > 0) {
                 c->d_item_lig.upload(il.data(), n, c->stream);
                 c->d_item_off.upload(io.data(), n, c->stream);
-                launch_bfgs(c, env, n, wsm, teams, c->d_item_lig.p, c->d_item_off.p, c->d_best.p, 2, p->refine_steps,
-                            VCAP_AUTH, 100.f, 1, nullptr);
+                launch_bfgs(c, env, n, need, c->d_item_lig.p, c->d_item_off.p, c->d_best.p, 2, p->refine_steps, VCAP_AUTH,
+                            100.f, 1, nullptr);
                 c->counters[2]++;
             }
         }
@@ -3152,14 +3198,14 @@ extern "C" int ud_score_batch_noalloc(ud_ctx* c, int n, const int* pose_lig, con
                                   "make one ud_score_batch, ud_search or ud_dock call first");
         Env env = make_env(c, mode);
         long long xs = 0, gs = 0;
-        int wsm = 0, full = 0;
+        int wsm = 0, size = 0;
         for (int i = 0; i < n; i++) {
             const int l = pose_lig[i];
             if (l < 0 || l >= (int)c->h_ligs.size()) throw Fail(UD_EINVAL, "pose ligand index out of range");
             xs += 3LL * c->h_ligs[l].natom;
             gs += 6 + c->h_ligs[l].ntors;
             wsm = std::max(wsm, lig_score_ws(c->h_ligs[l]));
-            full = std::max(full, lig_ws(c->h_ligs[l]));
+            size = std::max(size, lig_size(c->h_ligs[l]));
         }
         const size_t o_lig = 0;
         const size_t o_xo = align256(o_lig + (size_t)n * sizeof(int));
@@ -3191,7 +3237,7 @@ extern "C" int ud_score_batch_noalloc(ud_ctx* c, int n, const int* pose_lig, con
         // every offset, energy and gradient word is written below: nothing has to start at zero
         k_pose_offsets<<<1, 1024, 0, st>>>(c->d_ligs.p, n, d_lig, d_xo, d_go);
         ck(cudaGetLastError(), "k_pose_offsets launch");
-        const int W = score_warps(c, wsm, full);
+        const int W = score_warps(c, wsm, size);
         const size_t smem = (size_t)W * wsm * 4;
         const auto ks = score_kernel(env);
         set_smem(ks, smem);
