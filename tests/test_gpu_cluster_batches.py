@@ -32,3 +32,13 @@ def test_leaders_match_a_plain_greedy_pass(small_system, nchain, rmsd):
                 want.append(int(c))
         assert list(lead[l, :cnt[l]]) == want and (lead[l, cnt[l]:] == -1).all()
     eng.close()
+
+
+def test_as_many_chains_as_shared_memory_ranks(small_system):
+    """12 bytes per pose, and all but 32 bytes of the CTA's 227 KB for them."""
+    eng, _ = engine_for(dict(small_system, ligs=small_system["ligs"][:1]))
+    eng.search(seed=3, nchain=19368, mc_steps=0, opt_steps=0, randomize=True)
+    lead, cnt = eng.cluster(99.0)
+    e = eng.chain_poses(0)[:, 0]
+    eng.close()
+    assert cnt[0] == 1 and lead[0, 0] == np.argsort(np.where(np.isnan(e), np.inf, e), kind="stable")[0]

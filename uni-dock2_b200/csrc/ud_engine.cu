@@ -1138,10 +1138,12 @@ __global__ void k_cluster(const int* __restrict__ blobs, const LigDev* __restric
                           const float* __restrict__ best, float rmsd_limit, int* leaders, int* counts) {
     extern __shared__ __align__(16) float smem[];
     float* e = smem;
-    int* order = reinterpret_cast<int*>(e + nchain);
+    int* order = reinterpret_cast<int*>(e + max(nchain, 64));
     int* lead = order + nchain;
-    __shared__ int s_nl, s_close[32];
-    __shared__ unsigned s_near[32];
+    __shared__ int s_nl;
+    // the batch's marks take the energies' place after the ranking: as many chains fit as without them
+    int* const s_close = reinterpret_cast<int*>(e);
+    unsigned* const s_near = reinterpret_cast<unsigned*>(e) + 32;
     int lig = blockIdx.x;
     if (lig >= nlig) return;
     const LigDev L = ligs[lig];
@@ -2662,7 +2664,7 @@ static void launch_cluster(ud_ctx* c, float rmsd_limit) {
     int nchain = c->nchain;
     c->d_leaders.ensure((size_t)nlig * nchain);
     c->d_counts.ensure(nlig);
-    size_t smem = (size_t)nchain * 12;
+    size_t smem = ((size_t)std::max(nchain, 64) + 2 * (size_t)nchain) * 4;
     set_smem(k_cluster, smem);
     const int threads = nchain <= 32 ? 128 : (nchain <= 256 ? 512 : 1024);
     k_cluster<<<nlig, threads, smem, c->stream>>>(c->d_blobs.p, c->d_ligs.p, nlig, nchain, c->d_best.p, rmsd_limit,
