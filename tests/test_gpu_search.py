@@ -275,3 +275,25 @@ def test_constraint_docking_keeps_the_root_fragment(gpu_sys):
         assert np.all(gs[0][:6] == 0.0)
     finally:
         eng.set_flags(False, 0, 0.1)
+
+
+def test_autotuner_tunes_what_runs(gpu_sys):
+    """A tuned packing belongs to one kernel and workspace: maps or direct sums, with or without BFGS.  A new
+    one is timed first (nine short searches more), a known one is not, and the chains are the untuned ones
+    (enough of them that no team takes them)."""
+    from ud2b200 import MODE_DIRECT, MODE_GRID
+    eng, nl = gpu_sys["eng"], len(gpu_sys["ligs"])
+    kinds = [dict(mc_steps=2, opt_steps=2, mode=MODE_GRID), dict(mc_steps=2, opt_steps=0, mode=MODE_GRID),
+             dict(mc_steps=2, opt_steps=1, mode=MODE_DIRECT), dict(mc_steps=0, opt_steps=2, mode=MODE_GRID)]
+    plain = None
+    for on, want in ((False, [1, 1, 1, 1]), (True, [10, 10, 10, 1]), (None, [1, 1, 1, 1])):
+        if on is not None:
+            eng.set_autotune(on)
+        got, poses = [], []
+        for k in kinds:
+            eng.search(seed=9, nchain=200, randomize=True, **k)
+            got.append(eng.counters()["launches"])
+            poses += [eng.chain_poses(l).copy() for l in range(nl)]
+        plain = plain or poses
+        assert got == want and all(np.array_equal(a, b, equal_nan=True) for a, b in zip(poses, plain))
+    eng.set_autotune(False)

@@ -23,6 +23,8 @@
 #include <cstdio>
 #include <cstring>
 #include <cmath>
+#include <array>
+#include <map>
 #include <string>
 #include <vector>
 #include <algorithm>
@@ -1425,11 +1427,11 @@ struct ud_ctx {
     DBuf<float> d_sy, d_sm;
     int moves_max = 0, moves_n = 0;
     // chain packing autotuner (warps per CTA, chains per warp per work item)
-    int autotune = 0, tune_w = 8, tune_k = 0;
+    int autotune = 0;
     int pack_w = 0, pack_k = 0;               // ud_set_packing (0: chosen per batch)
     int shape[4] = {0, 0, 0, 0};              // last search: W, CTAs per SM, minb, k
     int retain = 1;                                   // poses kept per chain
-    long long tune_key = -1;
+    std::map<std::array<long long, 6>, std::pair<int, int>> tuned;      // by batch shape and kernel
     // measurement
     cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     float stage_ms[6] = {0, 0, 0, 0, 0, 0};
@@ -2448,12 +2450,15 @@ static void run_search_plan(ud_ctx* c, const SearchPlan& P, const Env& env, uint
 
 // Chain packing autotuner: warps per CTA (8, 12 or 4) and chains per warp per work item
 // (1, 2 or 4), each timed with CUDA events on a short search of the batch itself
-// (3 MC steps); the fastest is kept for batches of the same shape.  A chain's result does
+// (3 MC steps); the fastest is kept for batches of the same shape that run the same kernel in the same
+// workspace (maps or direct sums, with or without BFGS).  A chain's result does
 // not depend on the packing (its random stream is indexed by chain, ligand and step).
-static void autotune_search(ud_ctx* c, const Env& env, uint64_t seed, int nchain, int opt_steps, int randomize) {
-    const long long key = (long long)c->h_ligs.size() * 1000003LL + (long long)nchain * 131LL + c->max_stage * 7LL +
-                          c->retain;
-    if (c->tune_key == key) return;
+static std::pair<int, int> autotune_search(ud_ctx* c, const Env& env, uint64_t seed, int nchain, bool energy_only,
+                                           int opt_steps, int randomize) {
+    const std::array<long long, 6> key{(long long)c->h_ligs.size(), nchain, c->max_stage, c->retain,
+                                       env.mode == UD_MODE_GRID, energy_only};
+    const auto known = c->tuned.find(key);
+    if (known != c->tuned.end()) return known->second;
     cudaEvent_t e0, e1;
     ck(cudaEventCreate(&e0), "event");
     ck(cudaEventCreate(&e1), "event");
@@ -2461,10 +2466,10 @@ static void autotune_search(ud_ctx* c, const Env& env, uint64_t seed, int nchain
     int best_w = 8, best_k = 0;
     for (int w : {8, 12, 4})
         for (int k : {1, 2, 4}) {
-            const SearchPlan P = plan_fused(c, env, nchain, opt_steps == 0, w, k);
+            const SearchPlan P = plan_fused(c, env, nchain, energy_only, w, k);
             c->d_best.ensure((size_t)P.tot);
             ck(cudaEventRecord(e0, c->stream), "event");
-            run_search_plan(c, P, env, seed, nchain, 3, opt_steps, randomize);
+            run_search_plan(c, P, env, seed, nchain, 3, energy_only ? 0 : opt_steps, randomize);
             ck(cudaEventRecord(e1, c->stream), "event");
             ck(cudaEventSynchronize(e1), "autotune");
             float ms = 0.f;
@@ -2473,9 +2478,8 @@ static void autotune_search(ud_ctx* c, const Env& env, uint64_t seed, int nchain
         }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    c->tune_key = key;
-    c->tune_w = best_w;
-    c->tune_k = best_k;
+    if (c->tuned.size() >= 64) c->tuned.clear();
+    return c->tuned[key] = {best_w, best_k};
 }
 
 static void launch_search(ud_ctx* c, uint64_t seed, int nchain, int mc_steps, int opt_steps, int randomize, int mode) {
@@ -2486,8 +2490,8 @@ static void launch_search(ud_ctx* c, uint64_t seed, int nchain, int mc_steps, in
     const bool energy_only = mc_steps == 0 || opt_steps == 0;
     SearchPlan P = plan_fused(c, env, nchain, energy_only, c->pack_w, c->pack_k);
     if (c->autotune && !(c->pack_w || c->pack_k) && !P.team) {
-        autotune_search(c, env, seed, nchain, opt_steps, randomize);
-        P = plan_fused(c, env, nchain, energy_only, c->tune_w, c->tune_k);
+        const auto [w, k] = autotune_search(c, env, seed, nchain, energy_only, opt_steps, randomize);
+        P = plan_fused(c, env, nchain, energy_only, w, k);
     }
     c->best_floats = P.tot;
     c->d_best.ensure((size_t)P.tot);
@@ -2893,14 +2897,14 @@ int ud_mlp_set_gemm(ud_ctx* c, int kind) {
 int ud_set_retain(ud_ctx* c, int retain) {
     if (!c || retain < 1 || retain > 4) { g_err = "retain must be 1..4"; return UD_EINVAL; }
     c->retain = retain;
-    c->tune_key = -1;
+    c->tuned.clear();
     return UD_OK;
 }
 
 int ud_set_autotune(ud_ctx* c, int on) {
     if (!c) { g_err = "null context"; return UD_EINVAL; }
     c->autotune = on ? 1 : 0;
-    c->tune_key = -1;
+    c->tuned.clear();
     return UD_OK;
 }
 
