@@ -28,6 +28,33 @@ def test_team_search_is_the_search_of_one_warp(small_system, mode, constraint, r
     eng.close()
 
 
+@pytest.mark.parametrize("bias", ["pos", "align"])
+def test_team_search_with_bias_records(small_system, bias):
+    """The same with bias records on some of the atoms."""
+    import copy
+    rng = np.random.default_rng(6)
+    ligs = []
+    for lig in small_system["ligs"]:
+        lig = copy.copy(lig)
+        lig.bias_atoms = np.sort(rng.integers(0, lig.natom, 5)).astype(np.int32)
+        site = np.asarray(small_system["center"]) + rng.uniform(-3, 3, (5, 3))
+        lig.bias_params = np.column_stack([site, rng.uniform(-2, -0.5, 5), rng.uniform(0.5, 2, 5)]).astype(np.float32)
+        ligs.append(lig)
+    eng, _ = engine_for(dict(small_system, ligs=ligs))
+    got = {}
+    for kind in (0, 1 if bias == "pos" else 2):
+        eng.set_flags(bias_type=kind, bias_k=0.5)
+        for packing in ((0, 0), (8, 1)):
+            eng.set_packing(*packing)
+            ne = eng.search(seed=23, nchain=16, mc_steps=6, opt_steps=8, randomize=True)
+            got[bool(kind), packing] = (ne, [eng.chain_poses(l).copy() for l in range(len(ligs))])
+            assert eng.search_shape()["warps_per_cta"] == (8 if packing[0] else 4)
+    eng.close()
+    (na, a), (nb, b) = got[True, (0, 0)], got[True, (8, 1)]
+    assert na == nb and all(np.array_equal(x, y, equal_nan=True) for x, y in zip(a, b))
+    assert not any(np.array_equal(x, y, equal_nan=True) for x, y in zip(a, got[False, (0, 0)][1]))
+
+
 @pytest.mark.parametrize("max_steps,rounds", [(0, 1), (2, 5), (9, 1)])
 def test_team_refinement_is_that_of_one_warp(small_system, max_steps, rounds):
     """The same poses in a batch of ten (teams) and of 1200 (one warp each)."""
