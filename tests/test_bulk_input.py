@@ -166,3 +166,13 @@ def test_launch_plan_keeps_groups_budget_and_order():
     assert len(plan_launches(ref, per, int(per.sum()) * 2)) == len({g for g, _ in ref})
     with pytest.raises(MemoryError):
         plan_launches(ref, per, int(per.max()) - 1)
+
+
+def test_predicted_bytes_of_a_ligand():
+    """The launches that a memory budget gives, and with them the ligands' random streams, follow from this
+    count: it changes only on purpose."""
+    from ud2b200.batching import predict_dock_bytes
+    args = [np.array(v) for v in ((12, 29, 80), (2, 5, 20), (60, 520, 5200), (9, 70, 600), (2, 5, 20), (0, 0, 4))]
+    assert predict_dock_bytes(*args, nchain=128).tolist() == [31688, 67392, 223800]
+    assert predict_dock_bytes(*args, nchain=128, retain=4, num_pose=3, learned=True, decomp=True).tolist() == [
+        1064484, 1206248, 1705076]

@@ -43,9 +43,10 @@ def _centred(lig, system):
 
 @pytest.mark.parametrize("mode,retain", [("grid", 1), ("direct", 3)])
 @pytest.mark.parametrize("which", ["rigid", "hub"])
-def test_search_with_a_ligand_that_cannot_be_staged(wide, mode, retain, which):
-    """2408 atoms, and 13 atoms spread over the list that pair with 287 (whose gather lists are all as long):
-    the others of the batch keep their chains bit for bit, its own energies are those of its poses."""
+def test_search_with_a_very_large_or_uneven_ligand(wide, mode, retain, which):
+    """2408 atoms, whose topology cannot be staged, and 13 atoms spread over the list that pair with 287, whose
+    gather lists all have a tail: the others of the batch keep their chains bit for bit, its own energies are
+    those of its poses."""
     from ud2b200 import MODE_DIRECT, MODE_GRID, split_record
     m = MODE_GRID if mode == "grid" else MODE_DIRECT
     big = _centred(_ligand(2408) if which == "rigid" else _ligand(300, list(range(0, 299, 23))), wide)
@@ -94,6 +95,47 @@ def test_refinement_with_a_ligand_beyond_the_near_workspace(wide, mode):
                            mode=m, vcap=1000.0)
     eng.close()
     assert np.allclose([q["energy"] for q in r], e, rtol=1e-4, atol=1e-3)
+
+
+@pytest.mark.parametrize("natom,small", [(300, range(0, 299, 23)), (120, [7]), (33, [0, 32]), (64, range(0, 64, 3))])
+def test_gather_lists_of_uneven_lengths_match_oracle(wide, oracle64, natom, small):
+    """Atoms that pair with most others, one or more in a group of 32: rows of the lists and their tail."""
+    from ud2b200 import MODE_DIRECT
+    lig = _centred(_ligand(natom, list(small)), wide)
+    eng, _ = engine_for(dict(wide, ligs=[lig]))
+    rng = np.random.default_rng(natom)
+    x = lig.coords[None] * (1 + 0.02 * rng.normal(size=(3,) + lig.coords.shape)).astype(np.float32)
+    c, rv = x.mean(1), rng.uniform(-1, 1, (3, 3)).astype(np.float32)
+    e, g = eng.score_batch([0] * 3, x, c, rv, mode=MODE_DIRECT, vcap=10.0)
+    eng.close()
+    we, wg = oracle64.e_grad_batch(oracle64.ligand(lig), oracle64.make_env(wide["rec"], wide["box"], mode="direct"),
+                                   x.astype(np.float64), c.astype(np.float64), rv.astype(np.float64), 10.0, 1e6)
+    assert np.all(np.abs(e - we) <= 1e-4 * np.maximum(1.0, np.abs(we)))
+    for a, b in zip(g, wg):
+        assert np.abs(a - b).max() <= 1e-4 * max(1.0, np.abs(b).max())
+
+
+def test_topologies_stay_within_the_predicted_bytes(wide):
+    """What a launch's memory budget counts for a ligand's topology is an upper bound, also where padded
+    gather lists would take several times as much (2000 of each of four kinds, 4 MB for the rest)."""
+    from ud2b200 import MODE_DIRECT
+    from ud2b200.batching import predict_dock_bytes
+    kinds = [_centred(_ligand(*a), wide) for a in ((120, [7]), (40, [0, 39]), (200, [1, 60, 100, 150]))] + [wide["ligs"][4]]
+    ligs = kinds * 2000
+    count = lambda f: np.array([f(l) for l in kinds])  # noqa: E731
+    want = predict_dock_bytes(count(lambda l: l.natom), count(lambda l: l.ntors), count(lambda l: len(l.pairs)),
+                              count(lambda l: sum(map(len, l.rotated))), count(lambda l: sum(map(len, l.ranges))),
+                              np.zeros(4, int), nchain=0, retain=0, num_pose=0).sum() * 2000
+    eng, _ = engine_for(dict(wide, ligs=kinds))
+    x = [kinds[0].coords]
+    score = lambda: eng.score_batch([0], x, x[0].mean(0), np.zeros(3), mode=MODE_DIRECT)  # noqa: E731
+    score()
+    free = eng.device_memory()[0]
+    eng.add_ligands(ligs)
+    score()
+    used = free - eng.device_memory()[0]
+    eng.close()
+    assert 0.3 * want < used <= want + (4 << 20), (used, want)
 
 
 def test_too_large_is_refused_before_any_work(wide):

@@ -41,7 +41,7 @@ enum BlobHdr {
     H_RANGES,      // 2*nrange floats
     H_TMASK,       // natom rows of ceil(T / 32) words: bit k set where torsion k rotates the atom
     H_PAIR_OFF,    // natom+1 ints: per-atom intra adjacency (both directions)
-    H_PAIRS,       // packed entries: j | zero<<16 | hydrophobic pair<<17 | hbond pair<<18
+    H_PAIRS,       // its entries, 16 bits each
     H_BIAS_OFF,    // natom+1 ints (records)
     H_BIAS,        // 5 floats per record
     H_HEAVY,       // heavy atom indices
@@ -52,8 +52,9 @@ enum BlobHdr {
     H_MAPIDX,      // natom ints: grid map slot of each atom (-1: none), set at upload
     H_NPREC,       // number of heavy scored pairs (a count, not an offset)
     H_PREC,        // 2 words per pair: 16 i | hydrophobic | hbond<<1 | 16 j << 16, and R_i + R_j (float)
-    H_GOFF,        // per 32 atoms: first entry of their gather lists, longest of the 32 lists
+    H_GOFF,        // per 32 atoms: first entry of their gather lists, rows of the 32 lists | lists go on in the tail << 16
     H_GADJ,        // entry q of the lists of 32 atoms side by side: 4 * pair index | 16 * partner << 16
+    H_GTAIL,       // entries beyond the rows: natom+1 offsets from the section's start, then the entries (no section: 0)
     H_TOTAL,
     H_STAGE,       // words of the blob prefix the search stages into shared memory
     H_FRAME0,      // 3 words: non-collinear atoms no torsion moves (a rigid frame), or -1
@@ -75,7 +76,6 @@ enum BlobHdr {
 #define UD_LS_ATTR __forceinline__
 #endif
 constexpr int PREC_HYD = 1, PREC_HB = 2;
-constexpr int PAIR_ZERO = 1 << 16, PAIR_HYD = 1 << 17, PAIR_HB = 1 << 18;
 
 // Topology view: one base pointer and word offsets (keeps addressing 32-bit).
 struct Topo {
@@ -91,7 +91,7 @@ struct Topo {
         return (unsigned)b[o_tmask + a * ((ntors + 31) >> 5) + w];
     }
     __device__ __forceinline__ int pair_off(int i) const { return b[o_pair_off + i]; }
-    __device__ __forceinline__ int pair(int k) const { return b[o_pairs + k]; }
+    __device__ __forceinline__ int pair(int k) const { return reinterpret_cast<const unsigned short*>(b + o_pairs)[k]; }
     __device__ __forceinline__ int bias_off(int i) const { return b[o_bias_off + i]; }
     __device__ __forceinline__ const float* bias() const { return reinterpret_cast<const float*>(b + o_bias); }
     __device__ __forceinline__ int heavy(int h) const { return b[o_heavy + h]; }
@@ -749,27 +749,38 @@ __device__ __forceinline__ float intra_energy(const Topo& T, const float4* X, fl
     }
     return e;
 }
+__device__ __forceinline__ void gather_entry(unsigned v, const float4* X, const float* PB, const float4& xa, float& fx,
+                                             float& fy, float& fz) {
+    const float sc = *reinterpret_cast<const float*>(reinterpret_cast<const char*>(PB) + (v & 0xFFFFu));
+    const float4 xb = atom_at(X, v >> 16);
+    fx += sc * (xa.x - xb.x);
+    fy += sc * (xa.y - xb.y);
+    fz += sc * (xa.z - xb.z);
+}
 // The lists of 32 atoms lie side by side and are as long as their longest: every lane runs the
-// same loop over consecutive words.  A list's padding names the atom itself (difference zero).
+// same loop over consecutive words.  A list's padding names the atom itself (difference zero).  Where a few
+// atoms pair with most others, so that padding would take the topology over its bound (ud_add_ligands; one in
+// twelve of a screen batch), long lists go on in a tail.  (In line: 498 ms on the 148-ligand screen batch at 100
+// MC steps, 497 without tails; 512 with a function called for them.)
 __device__ __forceinline__ void intra_gather(const Topo& T, const float4* X, float4* F, const float* PB) {
     const int lane = lane_id();
 #pragma unroll 1
     for (int c = 0; 32 * c < T.natom; c++) {
         const int a = 32 * c + lane;
-        const int2 l = T.glist(c);                        // (first entry, entries per atom)
+        const int2 l = T.glist(c);                        // (first entry, rows)
         if (a >= T.natom) break;
         const int cnt = min(T.natom - 32 * c, WARP);
         const int* ent = T.b + T.o_gadj + l.x + lane;
         const float4 xa = X[a];
         float fx = 0.f, fy = 0.f, fz = 0.f;
+        const int rows = l.y & 0xFFFF;
 #pragma unroll 2
-        for (int q = 0; q < l.y; q++, ent += cnt) {
-            const unsigned v = (unsigned)*ent;
-            const float sc = *reinterpret_cast<const float*>(reinterpret_cast<const char*>(PB) + (v & 0xFFFFu));
-            const float4 xb = atom_at(X, v >> 16);
-            fx += sc * (xa.x - xb.x);
-            fy += sc * (xa.y - xb.y);
-            fz += sc * (xa.z - xb.z);
+        for (int q = 0; q < rows; q++, ent += cnt) gather_entry((unsigned)*ent, X, PB, xa, fx, fy, fz);
+        if (l.y != rows) {                                // the rest of the atom's list
+            const int* const tail = T.b + T.b[H_GTAIL];
+            const int k1 = tail[a + 1];
+#pragma unroll 1
+            for (int k = tail[a]; k < k1; k++) gather_entry((unsigned)tail[k], X, PB, xa, fx, fy, fz);
         }
         float4 f = F[a];
         f.x += fx; f.y += fy; f.z += fz;

@@ -385,7 +385,7 @@ __global__ void k_terms(const int* __restrict__ blobs, const LigDev* __restrict_
         int ti = T.type(i);
         float xi = X[3 * i], yi = X[3 * i + 1], zi = X[3 * i + 2];
         for (int k = T.pair_off(i); k < T.pair_off(i + 1); k++) {
-            int j = T.pair(k) & 0xFFFF;
+            int j = T.pair(k);
             if (j <= i) continue;
             float d0 = X[3 * j] - xi, d1 = X[3 * j + 1] - yi, d2 = X[3 * j + 2] - zi;
             float rr = d0 * d0 + d1 * d1 + d2 * d2;
@@ -1971,48 +1971,64 @@ int ud_add_ligands(ud_ctx* c, int nlig, const int* atom_off, const float* xyz, c
                     g[i].push_back(4 * p | (int)((unsigned)(16 * j) << 16));
                     g[j].push_back(4 * p | (int)((unsigned)(16 * i) << 16));
                 }
+                // The whole topology stays within the words that predict_dock_bytes (batching.py) counts for it:
+                // lists are cut to so many rows that it does, and go on in the tail.
                 const int nc = (n + 31) / 32;
+                const long long room = 160 + 13LL * n + 7LL * T + 2LL * nrange + 2LL * nrot + 5LL * nb + 3LL * np -
+                                       (long long)blob.size() - r4(2 * nc) - r4(n + 1) - r4((np + 1) / 2);
+                size_t longest = 0;
+                for (const auto& v : g) longest = std::max(longest, v.size());
+                int cut = (int)longest, acc = 0, over = 0;
+                for (;; cut--) {
+                    acc = over = 0;
+                    for (int c = 0; c < nc; c++) {
+                        size_t len = 0;
+                        for (int a = 32 * c; a < std::min(n, 32 * c + 32); a++) {
+                            len = std::max(len, std::min(g[a].size(), (size_t)cut));
+                            over += (int)(g[a].size() - std::min(g[a].size(), (size_t)cut));
+                        }
+                        acc += std::min(n - 32 * c, 32) * (int)len;
+                    }
+                    if (cut == 0 || r4(acc) + (over ? r4(n + 1 + over) : 0) <= room) break;
+                }
                 o = put(H_GOFF, 2 * nc);
-                int acc = 0;
-                for (int c = 0; c < nc; c++) {
+                for (int c = 0, first = 0; c < nc; c++) {
                     size_t len = 0;
                     for (int a = 32 * c; a < std::min(n, 32 * c + 32); a++) len = std::max(len, g[a].size());
-                    blob[o + 2 * c] = acc;
-                    blob[o + 2 * c + 1] = (int)len;
-                    acc += std::min(n - 32 * c, 32) * (int)len;
+                    const int rows = std::min((int)len, cut);
+                    blob[o + 2 * c] = first;
+                    blob[o + 2 * c + 1] = rows | ((int)len > rows ? 1 << 16 : 0);
+                    first += std::min(n - 32 * c, 32) * rows;
                 }
                 const int og = o;
                 o = put(H_GADJ, acc);
                 for (int c = 0; c < nc; c++) {
-                    const int cnt = std::min(n - 32 * c, 32);
-                    for (int q = 0; q < blob[og + 2 * c + 1]; q++)
+                    const int cnt = std::min(n - 32 * c, 32), rows = blob[og + 2 * c + 1] & 0xFFFF;
+                    for (int q = 0; q < rows; q++)
                         for (int l = 0; l < cnt; l++) {
                             const int a = 32 * c + l;
                             blob[o + blob[og + 2 * c] + cnt * q + l] =
                                 q < (int)g[a].size() ? g[a][q] : (int)((unsigned)(16 * a) << 16);
                         }
                 }
+                if (over) {
+                    o = put(H_GTAIL, n + 1 + over);
+                    int at = n + 1;
+                    for (int a = 0; a < n; a++) {
+                        blob[o + a] = at;
+                        for (size_t q = cut; q < g[a].size(); q++) blob[o + at++] = g[a][q];
+                    }
+                    blob[o + n] = at;
+                }
                 blob[H_STAGE] = (int)blob.size();
                 // as plain lists: rotated atoms per torsion for the masks, gather lists without padding
                 size_stage = blob[H_STAGE] + r4(T + 1) + r4(nrot) - r4(n * ((T + 31) / 32)) + r4(n + 1) + r4(2 * np2) -
-                             r4(2 * nc) - r4(acc);
+                             r4(2 * nc) - r4(acc) - (over ? r4(n + 1 + over) : 0);
             }
             o = put(H_PAIR_OFF, n + 1);
             for (int i = 0; i <= n; i++) blob[o + i] = pair_off[a0 + i] - p0;
-            o = put(H_PAIRS, np);
-            for (int i = 0; i < n; i++) {
-                const int ti = types[a0 + i];
-                for (int k = pair_off[a0 + i] - p0; k < pair_off[a0 + i + 1] - p0; k++) {
-                    const int v = pairs[p0 + k];
-                    const int tj = types[a0 + v];
-                    const unsigned b1 = 1u << ti, b2 = 1u << tj;
-                    int ent = v;
-                    if (ti == VN_H || tj == VN_H) ent |= PAIR_ZERO;
-                    if ((b1 & HYD_MASK) && (b2 & HYD_MASK)) ent |= PAIR_HYD;
-                    if (((b1 & ACC_MASK) && (b2 & DON_MASK)) || ((b1 & DON_MASK) && (b2 & ACC_MASK))) ent |= PAIR_HB;
-                    blob[o + k] = ent;
-                }
-            }
+            o = put(H_PAIRS, (np + 1) / 2);
+            for (int k = 0; k < np; k++) reinterpret_cast<unsigned short*>(&blob[o])[k] = (unsigned short)pairs[p0 + k];
             {   // rigid frame for recorded moves: three non-collinear atoms of the root fragment
                 std::vector<char> moved(n, 0);
                 for (int q = r0; q < r0 + nrot; q++) moved[rot_atoms[q]] = 1;

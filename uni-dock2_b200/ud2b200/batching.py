@@ -67,14 +67,14 @@ def record_floats(natom, ntors):
 def predict_dock_bytes(natom, ntors, npairs, nrot, nrange, nbias, nchain: int, retain: int = 1, num_pose: int = 10,
                        learned: bool = False, decomp: bool = False) -> np.ndarray:
     """Device bytes one ligand adds to a dock launch (an upper bound): its topology blob
-    (every section padded to 4 words), chain records (and the learned search's accepted
+    (which ud_add_ligands lays out to stay within this count), chain records (and the learned search's accepted
     poses, features and network activations), clustering and output buffers."""
     n = np.asarray(natom, np.int64)
     t = np.asarray(ntors, np.int64)
     p = np.asarray(npairs, np.int64)
     stride = record_floats(n, t)
-    blob = 4 * (64 + 96 + 13 * n + 7 * t + 2 * np.asarray(nrange, np.int64) + np.asarray(nrot, np.int64)
-                + n * ((t + 31) // 32) + 5 * np.asarray(nbias, np.int64) + 2 * p + n * np.minimum(n, p))
+    blob = 4 * (64 + 96 + 13 * n + 7 * t + 2 * np.asarray(nrange, np.int64) + 2 * np.asarray(nrot, np.int64)
+                + 5 * np.asarray(nbias, np.int64) + 3 * p)
     chains = nchain * retain
     rec = 4 * chains * stride
     b = blob + rec + 4 * chains + 64 + 16 * nchain                      # records, leaders, ligand entry, items
