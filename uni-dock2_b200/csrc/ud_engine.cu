@@ -1055,7 +1055,7 @@ __global__ void k_label_moves(const int* __restrict__ blobs, const LigDev* __res
     }
 }
 
-template <int MINB, int RMAX, int NT = 256, bool FAR = false>
+template <int MINB, int RMAX, int NT = 256>
 __global__ void __launch_bounds__(NT, MINB) k_learn_step(const int* __restrict__ blobs,
                                                         const LigDev* __restrict__ ligs, const int4* __restrict__ items,
                                                         int nitems, Env env, LearnP sp, const int* __restrict__ step_p,
@@ -1083,14 +1083,13 @@ __global__ void __launch_bounds__(NT, MINB) k_learn_step(const int* __restrict__
         if (it >= nitems) break;
         const int4 item = items[it];
         const LigDev L = ligs[item.x];
-        if (!FAR && item.x != s_lig && !stage_blob(sblob, blobs + L.blob_off, L.stage_words, &s_bar, phase, &s_flag)) {
+        if (item.x != s_lig && !stage_blob(sblob, blobs + L.blob_off, L.stage_words, &s_bar, phase, &s_flag)) {
             if (threadIdx.x == 0 && nevals) atomicAdd(nevals + 2, 1ull);
             break;
         }
         __syncthreads();
         if (threadIdx.x == 0) s_lig = item.x;
-        const int* const blob = FAR ? blobs + L.blob_off : sblob;
-        const Topo T = topo_view(blob);
+        const Topo T = topo_view(sblob);
         const int stride = slot_floats(T.natom, T.ntors);
         const Work W = work_at(ws, T);
         while (true) {
@@ -1106,7 +1105,7 @@ __global__ void __launch_bounds__(NT, MINB) k_learn_step(const int* __restrict__
             Slot SA = slot_at(ws, stride, 0, T.natom);
             Retained<RMAX> keep{true, out, L.stride, sp.retain, 1e9f, 1e9f, 1e9f, 1e9f};
             if (step0 == 0) {
-                load_initial(blob, SA, T.natom, T.ntors);
+                load_initial(sblob, SA, T.natom, T.ntors);
                 if (sp.randomize) randomize(T, env, rng, c, sp.nchain, SA, W.g, W.sc);
                 for (int r = 0; r < sp.retain; r++) init_best(out + (long long)r * L.stride, SA, T);
             } else {
@@ -2350,8 +2349,8 @@ struct SearchPlan {
 
 extern "C++" {
 template <typename K>
-static SearchPlan plan_search(ud_ctx* c, int nchain, bool energy_only, K k3, K k4, K k12, K kfar, int want_w = 0,
-                              int force_k = 0, K kteam = nullptr) {
+static SearchPlan plan_search(ud_ctx* c, int nchain, bool energy_only, K k3, K k4, K k12, int want_w = 0, int force_k = 0,
+                              K kteam = nullptr, K kfar = nullptr) {
     SearchPlan P;
     int size = 0;
     bool teams = kteam != nullptr && !energy_only && want_w == 0 && force_k == 0;
@@ -2397,7 +2396,7 @@ static SearchPlan plan_search(ud_ctx* c, int nchain, bool energy_only, K k3, K k
         if (n * w > per_sm * P.W) { P.W = w; P.minb = minb; P.smem = smem; per_sm = n; chosen = kern; }
     }
     if (P.W == 0) {                                    // a ligand too large for 4 warps per CTA
-        P.far = (long long)P.blob_max + P.wsm > lim;
+        P.far = kfar && (long long)P.blob_max + P.wsm > lim;
         if (P.far) P.blob_max = 0;
         P.W = pick_warps(c, P.wsm, P.blob_max, 4);
         P.minb = 3;
@@ -2476,7 +2475,7 @@ static SearchKernel far_kernel(const Env& env) {
 static SearchPlan plan_fused(ud_ctx* c, const Env& env, int nchain, bool energy_only, int want_w = 0, int force_k = 0) {
     const int r = c->retain;
     return plan_search(c, nchain, energy_only, search_kernel(env, 3, r), search_kernel(env, 4, r), search_kernel(env, 2, r),
-                       far_kernel(env), want_w, force_k, team_kernel(env, r));
+                       want_w, force_k, team_kernel(env, r), far_kernel(env));
 }
 
 static void run_search_plan(ud_ctx* c, const SearchPlan& P, const Env& env, uint64_t seed, int nchain, int mc_steps,
@@ -2578,9 +2577,9 @@ static void launch_learned(ud_ctx* c, uint64_t seed, int nchain, int mc_steps, i
     const int lk = c->pack_k ? c->pack_k : 2;
     const SearchPlan P = c->retain > 1
                              ? plan_search(c, nchain, opt_steps == 0, k_learn_step<3, 4>, k_learn_step<4, 4>, k_learn_step<2, 4, 384>,
-                                           k_learn_step<3, 4, 256, true>, c->pack_w, lk)
+                                           c->pack_w, lk)
                              : plan_search(c, nchain, opt_steps == 0, k_learn_step<3, 1>, k_learn_step<4, 1>, k_learn_step<2, 1, 384>,
-                                           k_learn_step<3, 4, 256, true>, c->pack_w, lk);
+                                           c->pack_w, lk);
     c->best_floats = P.tot;
     c->d_best.ensure((size_t)P.tot);
     c->d_acc.ensure((size_t)P.tot);
@@ -2630,8 +2629,7 @@ static void launch_learned(ud_ctx* c, uint64_t seed, int nchain, int mc_steps, i
     sp.p_learned = std::min(1.f, p_learned * (float)sp.block);
     sp.mc_steps = mc_steps;
     const int nblocks = (mc_steps + sp.block - 1) / sp.block;
-    auto kern = P.far ? k_learn_step<3, 4, 256, true>
-                : c->retain > 1
+    auto kern = c->retain > 1
                     ? (P.minb == 4 ? k_learn_step<4, 4> : (P.minb == 2 ? k_learn_step<2, 4, 384> : k_learn_step<3, 4>))
                     : (P.minb == 4 ? k_learn_step<4, 1> : (P.minb == 2 ? k_learn_step<2, 1, 384> : k_learn_step<3, 1>));
     const int fblocks = (int)std::min<long long>((nch * 32 + 255) / 256, (long long)c->nsm * 16);
