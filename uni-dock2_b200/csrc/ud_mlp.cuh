@@ -391,25 +391,45 @@ __global__ void k_relu_bwd(long long n, const float* __restrict__ dh, const __nv
 }
 
 // column sums of a rows x cols FP32 matrix (cols a multiple of 8), every column's rows added in order: a
-// block per 8 columns; all threads load 128 rows ahead into shared memory while one thread per column
-// adds the 128 before them.  What bounds it is that chain of additions, 4 cycles a row.  (One thread per
-// column that also loads its rows took 62 us for 1024 rows, four times per training step: 40 % of it.
-// Sums of every 128th row folded pairwise were as fast, but rounded otherwise, which Adam's first steps
-// turn into other weights.)
+// block per 8 columns; all threads load 1024 rows ahead while one thread per column adds the 1024 before
+// them from shared memory (a column's rows side by side, sixteen read ahead).  What bounds it is that chain of
+// additions, 4 cycles a row: 6.7 us for 1024 rows, four times per training step.  (One thread per column that
+// also loads its rows took 62 us.  Sums of every 128th row folded pairwise took 4.4, but round otherwise, which
+// Adam's first steps turn into other weights.)
+constexpr int CS_AHEAD = 8;
 __global__ void __launch_bounds__(1024) k_colsum(int rows, int cols, const float* __restrict__ s, float* __restrict__ d) {
-    __shared__ float tile[2][128][9];
+    constexpr int N = 128 * CS_AHEAD;
+    __shared__ __align__(16) float tile[8][N + 20];      // 16 more to read ahead, and a bank offset
     const int c = threadIdx.x & 7, y = threadIdx.x >> 3, col = blockIdx.x * 8 + c;
-    float v = y < rows ? s[(long long)y * cols + col] : 0.f, acc = 0.f;
-    for (int r0 = 0, b = 0; r0 < rows; r0 += 128, b ^= 1) {
-        tile[b][y][c] = v;
-        __syncthreads();                     // also: the sums over this half of the tile two rounds ago are done
-        const int r = r0 + 128 + y;
-        if (r < rows) v = s[(long long)r * cols + col];
-        if (y == 0) {
-            const int n = min(128, rows - r0);
-#pragma unroll 16
-            for (int k = 0; k < n; k++) acc += tile[b][k][c];
+    float v[CS_AHEAD], acc = 0.f;
+    const auto load = [&](int r0) {
+#pragma unroll
+        for (int i = 0; i < CS_AHEAD; i++) {
+            const int r = r0 + 128 * i + y;
+            v[i] = r < rows ? s[(long long)r * cols + col] : 0.f;
         }
+    };
+    load(0);
+    for (int r0 = 0; r0 < rows; r0 += N) {
+#pragma unroll
+        for (int i = 0; i < CS_AHEAD; i++) tile[c][128 * i + y] = v[i];
+        __syncthreads();
+        load(r0 + N);
+        if (y == 0) {
+            const float4* const t = reinterpret_cast<const float4*>(tile[c]);
+            const int n = (min(N, rows - r0) + 15) >> 4;   // rows beyond the last are zero
+            float4 q[4] = {t[0], t[1], t[2], t[3]};
+#pragma unroll 1
+            for (int k = 1; k <= n; k++) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const float4 u = q[i];
+                    q[i] = t[4 * k + i];
+                    acc += u.x; acc += u.y; acc += u.z; acc += u.w;
+                }
+            }
+        }
+        __syncthreads();
     }
     if (y == 0) d[col] = acc;
 }
