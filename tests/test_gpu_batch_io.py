@@ -62,3 +62,23 @@ def test_forms_of_the_coordinates(io_sys):
     assert np.array_equal(eng.score_batch([0, 0], same, c[[0, 5]], rv[:2])[0], want[[0, 5]])
     with pytest.raises(IndexError):
         eng.score_batch([99], xs[:1], c[:1], rv[:1])
+
+
+def test_batches_before_and_after_the_page_locked_block(small_system):
+    """Calls of several sizes again and again, until their copies go through page-locked memory: the same
+    numbers all along."""
+    eng, _ = engine_for(small_system)
+    sizes, first = (3, 700, 1600, 9000), {}
+    for rnd in range(60):
+        for n in sizes if rnd % 20 == 0 else sizes[1:3]:
+            if n not in first:
+                pl, xs = _poses(small_system, n)
+                first[n] = [pl, xs, np.array([x.mean(0) for x in xs]), np.full((n, 3), 0.2, np.float32), None]
+            pl, xs, c, rv, want = first[n]
+            e, g = eng.score_batch(pl, xs, c, rv, vcap=10.0)
+            got = np.concatenate([e, *g])
+            if want is None:
+                first[n][4] = got
+            else:
+                assert np.array_equal(got, want), (rnd, n)
+    eng.close()

@@ -1331,19 +1331,24 @@ struct DBuf {
 };
 
 // Inputs and outputs of one batch call (scoring, terms, refinement): laid out in one device
-// buffer, the inputs first, which stays with the context up to KEEP bytes.  Up to PACK bytes go each way as one
-// copy, through ordinary host memory; larger batches are copied array by array.  With eight
-// allocations and frees and six copies per call, a call of eight poses took 139 us, of which the kernel
-// was 12; now 73.  (Through a page-locked block of the context, 72, and 3 % less from 256 poses on, but a new
-// context's first call took 1.5 to 3.5 ms for the block where it now takes 0.15, and closing the context 0.5 more:
-// a program that makes a context per receptor would pay that each time.)
+// buffer, the inputs first, which stays with the context up to KEEP bytes.  Small batches go each way as one
+// copy through a staging buffer, larger ones are copied array by array.  With eight allocations and
+// frees and six copies per call, a call of eight poses took 139 us, of which the kernel was 12; now 73.
+// The staging buffer is ordinary memory (up to PACK bytes) until the context's calls have moved PIN_AFTER bytes,
+// and then page-locked (up to PINNED): that saves 1 us of a call of eight poses and 0.16 ms of 2048 refinements
+// (3.76 -> 3.60 ms), but the block takes 1.5 to 3.5 ms to allocate and 0.5 to free, about what it saves over so
+// many bytes.  (Allocated by the first call it made that 2.5 ms instead of 0.13, for every receptor of a program
+// that makes a context for each.)
 struct BatchIO {
-    static constexpr size_t PACK = 256 << 10, KEEP = (size_t)256 << 20;
+    static constexpr size_t PACK = 256 << 10, PINNED = 1 << 20, PIN_AFTER = 16 << 20, KEEP = (size_t)256 << 20;
     DBuf<unsigned char> dev;
     std::vector<unsigned char> host;
+    unsigned char* pin = nullptr;
+    size_t moved = 0;
     struct Part { const void* in; void* out; size_t bytes, at; };
     std::vector<Part> parts;
     size_t in_bytes = 0, bytes = 0;
+    unsigned char* stage = nullptr;        // this call's staging buffer, null if copied array by array
 
     void begin() { parts.clear(); in_bytes = bytes = 0; }
     size_t add(const void* in, void* out, size_t n) {
@@ -1356,10 +1361,23 @@ struct BatchIO {
     // allocate and send the inputs (all of them added before the outputs)
     void send(cudaStream_t s) {
         dev.ensure(bytes);
-        if (bytes <= PACK) {
+        if (bytes <= PINNED) moved += bytes;
+        if (!pin && moved > PIN_AFTER) {
+            moved = 0;
+            if (cudaMallocHost(reinterpret_cast<void**>(&pin), PINNED) != cudaSuccess) {
+                cudaGetLastError();                            // none to be had: as before, asked for again later
+                pin = nullptr;
+            }
+        }
+        stage = nullptr;
+        if (pin && bytes <= PINNED) stage = pin;
+        else if (bytes <= PACK) {
             if (host.size() < bytes) host.resize(bytes);
-            for (const Part& p : parts) if (p.in) memcpy(host.data() + p.at, p.in, p.bytes);
-            if (in_bytes) ck(cudaMemcpyAsync(dev.p, host.data(), in_bytes, cudaMemcpyHostToDevice, s), "H2D");
+            stage = host.data();
+        }
+        if (stage) {
+            for (const Part& p : parts) if (p.in) memcpy(stage + p.at, p.in, p.bytes);
+            if (in_bytes) ck(cudaMemcpyAsync(dev.p, stage, in_bytes, cudaMemcpyHostToDevice, s), "H2D");
         } else {
             for (const Part& p : parts)
                 if (p.in && p.bytes) ck(cudaMemcpyAsync(dev.p + p.at, p.in, p.bytes, cudaMemcpyHostToDevice, s), "H2D");
@@ -1370,10 +1388,10 @@ struct BatchIO {
         size_t o0 = bytes, o1 = 0;
         for (const Part& p : parts)
             if (p.out) { o0 = std::min(o0, p.at); o1 = std::max(o1, p.at + p.bytes); }
-        if (bytes <= PACK) {
-            if (o1 > o0) ck(cudaMemcpyAsync(host.data() + o0, dev.p + o0, o1 - o0, cudaMemcpyDeviceToHost, s), what);
-            else ck(cudaStreamSynchronize(s), what);      // a copy to pageable memory returns when it is done
-            for (const Part& p : parts) if (p.out) memcpy(p.out, host.data() + p.at, p.bytes);
+        if (stage) {
+            if (o1 > o0) ck(cudaMemcpyAsync(stage + o0, dev.p + o0, o1 - o0, cudaMemcpyDeviceToHost, s), what);
+            if (stage == pin || o1 <= o0) ck(cudaStreamSynchronize(s), what);      // to pageable memory it is done
+            for (const Part& p : parts) if (p.out) memcpy(p.out, stage + p.at, p.bytes);
         } else {
             for (const Part& p : parts)
                 if (p.out && p.bytes) ck(cudaMemcpyAsync(p.out, dev.p + p.at, p.bytes, cudaMemcpyDeviceToHost, s), "D2H");
@@ -1381,6 +1399,15 @@ struct BatchIO {
             if (bytes > KEEP) dev.release();
         }
     }
+    void release() {
+        dev.release();
+        if (pin) cudaFreeHost(pin);
+        pin = nullptr;
+    }
+    BatchIO() = default;
+    BatchIO(const BatchIO&) = delete;
+    BatchIO& operator=(const BatchIO&) = delete;
+    ~BatchIO() { release(); }
 };
 
 struct LigHost {
@@ -1697,7 +1724,7 @@ int ud_destroy(ud_ctx* c) {
     c->d_maps32.release(); c->d_maps16.release();
     c->d_blobs.release(); c->d_ligs.release(); c->d_best.release();
     c->d_order.release(); c->d_items.release(); c->d_counter.release(); c->d_leaders.release(); c->d_counts.release();
-    c->d_sel.release(); c->d_selcnt.release(); c->d_ori.release(); c->io.dev.release(); c->d_nevals.release();
+    c->d_sel.release(); c->d_selcnt.release(); c->d_ori.release(); c->io.release(); c->d_nevals.release();
     c->d_out.release(); c->d_terms.release(); c->d_decomp.release();
     c->d_item_lig.release(); c->d_item_off.release(); c->d_item_off2.release();
     for (auto& e : c->ev) if (e) cudaEventDestroy(e);
