@@ -275,7 +275,7 @@ int ud_counters(const ud_ctx* ctx, long long* out4);
 int ud_set_retain(ud_ctx* ctx, int retain);
 
 /* Chain packing autotuner for ud_search / ud_dock (on != 0): before a batch of a new
- * shape, times short searches (3 MC steps) with 8, 12 or 4 warps per CTA and 1, 2 or 4
+ * shape (or of another scoring mode, or without BFGS), times short searches (3 MC steps) with 8, 12 or 4 warps per CTA and 1, 2 or 4
  * chains per warp per work item and keeps the fastest.  Results do not depend on the
  * packing.  Without it (and without ud_set_packing) the search takes the CTA width that
  * keeps the most warps resident, and where all chains fit the GPU four times over, a CTA of
