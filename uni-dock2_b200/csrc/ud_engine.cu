@@ -1759,6 +1759,7 @@ int ud_set_receptor(ud_ctx* c, int n, const float* xyz, const int* types) {
             if (in) c->h_rec.push_back(make_float4(x, y, z, (float)t));
         }
         c->lists_built = false;
+        c->h_cell_start.clear();                       // empty lists until the cells below are there
         c->d_rec.upload(c->h_rec.data(), c->h_rec.size(), c->stream);
         // cell list over the kept region (box +- 8 A): counting sort, stable in receptor order
         int ncell = 1;
