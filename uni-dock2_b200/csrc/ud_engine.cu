@@ -2056,7 +2056,8 @@ int ud_add_ligands(ud_ctx* c, int nlig, const int* atom_off, const float* xyz, c
             o = put(H_PAIR_OFF, n + 1);
             for (int i = 0; i <= n; i++) blob[o + i] = pair_off[a0 + i] - p0;
             o = put(H_PAIRS, (np + 1) / 2);
-            for (int k = 0; k < np; k++) reinterpret_cast<unsigned short*>(&blob[o])[k] = (unsigned short)pairs[p0 + k];
+            const std::vector<unsigned short> adj(pairs + p0, pairs + p0 + np);
+            memcpy(blob.data() + o, adj.data(), adj.size() * sizeof(adj[0]));
             {   // rigid frame for recorded moves: three non-collinear atoms of the root fragment
                 std::vector<char> moved(n, 0);
                 for (int q = r0; q < r0 + nrot; q++) moved[rot_atoms[q]] = 1;
